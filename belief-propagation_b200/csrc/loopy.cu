@@ -831,8 +831,8 @@ __device__ __forceinline__ bool grid_barrier(LoopyCtl *c, uint32_t &gen, uint32_
 // the same intervals.  Scratch: 8 doubles per block after the partials.
 // false when a barrier gave up.
 template <int NT>
-__device__ bool grid_refine(const FloodArgs &a, LoopyCtl *ctl, uint32_t &gen, uint32_t *s_fail, SerialCheck &x,
-                            const LoopyCtl &sc, float *buf, uint32_t cap, double *red) {
+__device__ bool grid_refine(double *partials, const float *absdiff, LoopyCtl *ctl, uint32_t &gen, uint32_t *s_fail,
+                            SerialCheck &x, const LoopyCtl &sc, float *buf, uint32_t cap, double *red) {
     __shared__ double s_b[4];
     __shared__ double s_v[NT / 32][6];
     __shared__ double s_t[6];
@@ -842,10 +842,10 @@ __device__ bool grid_refine(const FloodArgs &a, LoopyCtl *ctl, uint32_t &gen, ui
     const bool do_p = !x.p_exact && !x.p_ref;
     ++x.refines;
     const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-    double *scr = a.partials + 2 * (size_t)G;
+    double *scr = partials + 2 * (size_t)G;
     const uint64_t L = ((n + G - 1) / G + 3) & ~3ull;
     const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
-    const float *xs = a.absdiff + (size_t)x.cb * stride, *xp = a.absdiff + (size_t)sc.prev_buf * stride;
+    const float *xs = absdiff + (size_t)x.cb * stride, *xp = absdiff + (size_t)sc.prev_buf * stride;
     double ls = 0.0, lp = 0.0;
     for (uint64_t k = lo + tid; k < hi; k += NT) {
         ls += (double)__ldcg(xs + k);
@@ -942,6 +942,73 @@ __device__ bool grid_refine(const FloodArgs &a, LoopyCtl *ctl, uint32_t &gen, ui
     return true;
 }
 
+// one serial-mode check of a one-launch loop: every block of the grid calls it
+// with the same f64 sum `tot` (in thread 0) and reaches the same decision; when
+// the bounds cannot decide, block 0 forms the serial sums and the blocks meet
+// once more to read them.  The terms are triple-buffered by check, so no
+// block overwrites them while block 0 reads.  sc: the block's copy of the
+// control block, updated.  false when a barrier gave up.
+template <int NT>
+__device__ __forceinline__ bool grid_serial_check(LoopyCtl *ctl, LoopyCtl &sc, double *partials, const float *absdiff,
+                                                  uint32_t &gen, uint32_t *s_fail, double tot, float *buf,
+                                                  uint32_t cap, double *red) {
+    SerialCheck x = serial_check(&sc, broadcast_sum(tot));
+    if (x.d < 0 && !grid_refine<NT>(partials, absdiff, ctl, gen, s_fail, x, sc, buf, cap, red)) return false;
+    if (x.d < 0) {
+        const bool s_ex0 = x.s_exact, p_ex0 = x.p_exact;
+        if (blockIdx.x == 0) {
+            serial_form<NT>(x, &sc, absdiff, buf, cap, false);
+            if (threadIdx.x == 0) {
+                ctl->fb_s = x.s;
+                ctl->fb_p = (float)x.plo;
+                ctl->fb_pform = x.p_exact && !p_ex0;
+            }
+        }
+        if (!grid_barrier(ctl, gen, s_fail)) return false;
+        if (blockIdx.x != 0) {
+            if (!s_ex0) {
+                x.s = *(volatile float *)&ctl->fb_s;
+                x.lo = x.hi = (double)x.s;
+                x.s_exact = true;
+            }
+            if (*(volatile uint32_t *)&ctl->fb_pform) {
+                x.plo = x.phi = (double)*(volatile float *)&ctl->fb_p;
+                x.p_exact = x.p_new = true;
+            }
+            x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, sc.tol);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) serial_commit(&sc, x);
+    return true;
+}
+
+// the run's outcome from a block's copy of the control block (one thread)
+__device__ __forceinline__ void publish_ctl(LoopyCtl *ctl, const LoopyCtl &sc) {
+    ctl->it = sc.it;
+    ctl->ret = sc.ret;
+    ctl->num_iter = sc.num_iter;
+    ctl->final_i = sc.final_i;
+    ctl->delta_f = sc.delta_f;
+    ctl->prev_f = sc.prev_f;
+    ctl->delta_d = sc.delta_d;
+    ctl->prev_d = sc.prev_d;
+    ctl->dlo = sc.dlo;
+    ctl->dhi = sc.dhi;
+    ctl->plo = sc.plo;
+    ctl->phi = sc.phi;
+    ctl->delta_exact = sc.delta_exact;
+    ctl->prev_exact = sc.prev_exact;
+    ctl->cur_buf = sc.cur_buf;
+    ctl->prev_buf = sc.prev_buf;
+    ctl->serial_sums = sc.serial_sums;
+    ctl->serial_refines = sc.serial_refines;
+    ctl->delta_ref = sc.delta_ref;
+    ctl->prev_ref = sc.prev_ref;
+    __threadfence();
+    ctl->done = sc.done;
+}
+
 template <int MS, bool UNI, int FU, bool SER = false, int MB = flood_min_blocks<MS, FU>()>
 __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood_fused(const FloodArgs a, uint32_t ntiles) {
     constexpr int NT = flood_nt<MS>();
@@ -981,67 +1048,14 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood_fused(const FloodA
         for (uint32_t k = threadIdx.x; k < gridDim.x; k += NT) acc += __ldcg(part + k);
         const double tot = block_sum<NT>(acc, red);
         if (SER && want) {
-            // every block reaches the same decision from the same sum; when
-            // the bound cannot decide, block 0 forms the serial sums and the
-            // blocks meet once more to read them.  The terms are
-            // triple-buffered by check, so no block overwrites them while
-            // block 0 reads.
-            SerialCheck x = serial_check(&s_ctl, broadcast_sum(tot));
-            if (x.d < 0 && !grid_refine<NT>(a, ctl, gen, &s_fail, x, s_ctl, sm, EMAX * MS, red)) break;
-            if (x.d < 0) {
-                const bool s_ex0 = x.s_exact, p_ex0 = x.p_exact;
-                if (blockIdx.x == 0) {
-                    serial_form<NT>(x, &s_ctl, a.absdiff, sm, EMAX * MS, false);
-                    if (threadIdx.x == 0) {
-                        ctl->fb_s = x.s;
-                        ctl->fb_p = (float)x.plo;
-                        ctl->fb_pform = x.p_exact && !p_ex0;
-                    }
-                }
-                if (!grid_barrier(ctl, gen, &s_fail)) break;
-                if (blockIdx.x != 0) {
-                    if (!s_ex0) {
-                        x.s = *(volatile float *)&ctl->fb_s;
-                        x.lo = x.hi = (double)x.s;
-                        x.s_exact = true;
-                    }
-                    if (*(volatile uint32_t *)&ctl->fb_pform) {
-                        x.plo = x.phi = (double)*(volatile float *)&ctl->fb_p;
-                        x.p_exact = x.p_new = true;
-                    }
-                    x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, s_ctl.tol);
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) serial_commit(&s_ctl, x);
+            if (!grid_serial_check<NT>(ctl, s_ctl, a.partials, a.absdiff, gen, &s_fail, tot, sm, EMAX * MS, red)) break;
         } else if (threadIdx.x == 0) {
             finalize(&s_ctl, want, (float)tot, tot);
         }
         __syncthreads();
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && !s_fail) {
-        ctl->it = s_ctl.it;
-        ctl->ret = s_ctl.ret;
-        ctl->num_iter = s_ctl.num_iter;
-        ctl->final_i = s_ctl.final_i;
-        ctl->delta_f = s_ctl.delta_f;
-        ctl->prev_f = s_ctl.prev_f;
-        ctl->delta_d = s_ctl.delta_d;
-        ctl->prev_d = s_ctl.prev_d;
-        ctl->dlo = s_ctl.dlo;
-        ctl->dhi = s_ctl.dhi;
-        ctl->plo = s_ctl.plo;
-        ctl->phi = s_ctl.phi;
-        ctl->delta_exact = s_ctl.delta_exact;
-        ctl->prev_exact = s_ctl.prev_exact;
-        ctl->cur_buf = s_ctl.cur_buf;
-        ctl->prev_buf = s_ctl.prev_buf;
-        ctl->serial_sums = s_ctl.serial_sums;
-        ctl->serial_refines = s_ctl.serial_refines;
-        ctl->delta_ref = s_ctl.delta_ref;
-        ctl->prev_ref = s_ctl.prev_ref;
-        __threadfence();
-        ctl->done = s_ctl.done;
+        publish_ctl(ctl, s_ctl);
     }
 }
 
@@ -1562,193 +1576,7 @@ __global__ void __launch_bounds__(1024) k_delta_final(LoopyCtl *ctl, const float
     }
 }
 
-// ------------------------------------------------------------------------
-// Edge-centric schedule (loopy_propagate_until_edge, graph.c:1186-1276, and
-// its _acc form, graph.c:1444-1547), reproduced with its quirks:
-//  * copy: num_edges * MAX_STATES BYTES of current into previous
-//    (graph.c:1211), i.e. the first 2.5E floats of the reference's padded
-//    array; the _acc form copies every float;
-//  * send from the beliefs themselves (no incoming product);
-//  * combine: belief(dest) *= message for each edge in edge order, no NaN
-//    check; the _acc form multiplies by the message of edge i, the batch's
-//    first iteration index (graph.c:1485);
-//  * normalise: node 0's belief, once per node with that node's state count
-//    (the base pointer is passed, graph.c:1225, :1505).
-struct EdgeArgs {
-    uint32_t V, E;
-    const uint32_t *in_ptr, *in_src, *pos_edge, *edge_pos;
-    const uint8_t *node_s, *pos_dims;
-    const float *joint;
-    float *belief;
-    float *msg0, *msg1;
-    double *partials;
-    float *absdiff;
-    LoopyCtl *ctl;
-    const uint32_t *run_len;
-    const uint8_t *run_s;
-    uint32_t nruns;
-};
-
-// previous/current roles: the _acc form swaps local pointers every iteration
-__device__ __forceinline__ void edge_roles(const EdgeArgs &a, uint32_t it, float *&prev, float *&curr) {
-    const LoopyCtl *c = a.ctl;
-    int p = (int)(c->msg_parity0 & 1u);
-    if (c->acc_edge && (it & 1u)) p ^= 1;
-    prev = p ? a.msg1 : a.msg0;
-    curr = p ? a.msg0 : a.msg1;
-}
-
-template <int MS>
-__global__ void k_edge_copy(const EdgeArgs a) {
-    if (*(volatile uint32_t *)&a.ctl->done) return;
-    float *prev, *curr;
-    edge_roles(a, a.ctl->it, prev, curr);
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t p = t / MS;
-    if (p >= a.E) return;
-    const uint32_t k = (uint32_t)(t % MS);
-    if (a.ctl->acc_edge) {
-        prev[t] = curr[t];
-        return;
-    }
-    const uint64_t f = (uint64_t)a.pos_edge[p] * 10u + k;   // float index in the padded layout
-    const uint64_t nbytes = (uint64_t)a.E * 10u;
-    const uint64_t nfull = nbytes / 4u;
-    if (f < nfull) {
-        prev[t] = curr[t];
-    } else if (f == nfull && (nbytes & 3u)) {
-        const uint32_t keep = 0xffffffffu << (8u * (uint32_t)(nbytes & 3u));
-        const uint32_t cb = __float_as_uint(curr[t]), pb = __float_as_uint(prev[t]);
-        prev[t] = __uint_as_float((pb & keep) | (cb & ~keep));
-    }
-}
-
-template <int MS, bool UNI>
-__global__ void k_edge_send(const EdgeArgs a) {
-    if (*(volatile uint32_t *)&a.ctl->done) return;
-    float *prev, *curr;
-    edge_roles(a, a.ctl->it, prev, curr);
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.E) return;
-    const uint32_t s = a.in_src[p];
-    int x = MS, y = MS;
-    if (!UNI) {
-        const uint8_t d = a.pos_dims[p];
-        x = d & 15;
-        y = d >> 4;
-    }
-    float buf[MS], m[MS];
-    ldv<MS>(a.belief + (size_t)s * MS, buf);
-    send_msg<MS, UNI>(a.joint + p * (MS * MS), buf, x, y, m);
-    stv<MS>(curr + p * MS, m);
-}
-
-template <int MS, bool UNI>
-__global__ void k_edge_combine(const EdgeArgs a) {
-    if (*(volatile uint32_t *)&a.ctl->done) return;
-    const uint32_t it = a.ctl->it;
-    float *prev, *curr;
-    edge_roles(a, it, prev, curr);
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= a.V) return;
-    const int S = UNI ? MS : a.node_s[v];
-    const uint32_t r0 = a.in_ptr[v], r1 = a.in_ptr[v + 1];
-    if (r0 == r1) return;
-    float b[MS];
-    ldv<MS>(a.belief + (size_t)v * MS, b);
-    if (a.ctl->acc_edge) {
-        const uint32_t i_batch = (it / 10u) * 10u;
-        if (i_batch >= a.E) return;
-        float mm[MS];
-        ldv<MS>(curr + (size_t)a.edge_pos[i_batch] * MS, mm);
-        for (uint32_t p = r0; p < r1; ++p) {
-#pragma unroll
-            for (int i = 0; i < MS; ++i)
-                if (UNI || i < S) b[i] = FMUL(b[i], mm[i]);
-        }
-    } else {
-        for (uint32_t p = r0; p < r1; ++p) {
-            float mm[MS];
-            ldv<MS>(curr + (size_t)p * MS, mm);
-#pragma unroll
-            for (int i = 0; i < MS; ++i)
-                if (UNI || i < S) b[i] = FMUL(b[i], mm[i]);
-        }
-    }
-    stv<MS>(a.belief + (size_t)v * MS, b);
-}
-
-// node 0 normalised once per node, in node order; within a run of equal
-// state counts the map is applied until it stops changing node 0 (it is then
-// the identity for the rest of the run)
-template <int MS>
-__global__ void k_edge_normalise_node0(const EdgeArgs a) {
-    if (*(volatile uint32_t *)&a.ctl->done) return;
-    if (threadIdx.x != 0 || blockIdx.x != 0 || a.V == 0) return;
-    float b[MS];
-    ldv<MS>(a.belief, b);
-    for (uint32_t r = 0; r < a.nruns; ++r) {
-        const int s = a.run_s[r];
-        const uint32_t len = a.run_len[r];
-        for (uint32_t k = 0; k < len; ++k) {
-            float sum = 0.0f;
-#pragma unroll
-            for (int i = 0; i < MS; ++i)
-                if (i < s) sum = FADD(sum, b[i]);
-            if (!(sum > 0.0f)) break;
-            bool changed = false;
-#pragma unroll
-            for (int i = 0; i < MS; ++i) {
-                if (i < s) {
-                    float nb = FDIV(b[i], sum);
-                    changed |= __float_as_uint(nb) != __float_as_uint(b[i]);
-                    b[i] = nb;
-                }
-            }
-            if (!changed) break;
-        }
-    }
-    stv<MS>(a.belief, b);
-}
-
-template <int MS, bool UNI>
-__global__ void __launch_bounds__(256) k_edge_delta(const EdgeArgs a) {
-    __shared__ double red[8];
-    __shared__ bool s_last;
-    __shared__ __align__(16) float buf[2 * 1024];
-    LoopyCtl *ctl = a.ctl;
-    if (*(volatile uint32_t *)&ctl->done) return;
-    const uint32_t it = ctl->it, ce = ctl->check_every;
-    const bool want = (ce <= 1) || ((it + 1) % ce == 0);
-    const bool serial = ctl->serial != 0;
-    float *absd = check_buffer(ctl, a.absdiff, it, want);
-    // the delta reads the local prev/curr AFTER this iteration's swap (_acc)
-    float *prev, *curr;
-    edge_roles(a, ctl->acc_edge ? it + 1 : it, prev, curr);
-    double dsum = 0.0;
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (want && p < a.E) {
-        int x = MS;
-        if (!UNI) x = a.pos_dims[p] & 15;
-        float o[MS], c[MS], ad[MS];
-        ldv<MS>(prev + p * MS, o);
-        ldv<MS>(curr + p * MS, c);
-#pragma unroll
-        for (int k = 0; k < MS; ++k) {
-            float d = 0.0f;
-            if (UNI || k < x) {
-                d = FSUB(o[k], c[k]);
-                if (d != d) d = 0.0f;
-                d = fabsf(d);
-            }
-            ad[k] = d;
-            dsum += (double)d;
-        }
-        if (absd) stv<MS>(absd + (size_t)a.pos_edge[p] * MS, ad);
-    }
-    if (serial) reduce_and_finalize<256, true>(ctl, a.partials, dsum, want, red, &s_last, a.absdiff, buf, 2 * 1024);
-    else reduce_and_finalize<256>(ctl, a.partials, dsum, want, red, &s_last);
-}
+#include "edge_loop.cuh"
 
 // ---------------------------------------------------------------- driver --
 
@@ -2210,27 +2038,44 @@ static int enqueue_node_iterations(bp_graph *g, uint32_t k, bool serial, int var
     return BP_OK;
 }
 
+// the edge schedule's one-launch loop: its resident grid (at most one thread
+// per edge or node)
 template <int MS, bool UNI>
-static int enqueue_edge_iterations(bp_graph *g, uint32_t k, bool, int) {
-    const EdgeArgs a = edge_args(g);
-    const uint64_t n = (uint64_t)g->E * MS;
-    for (uint32_t i = 0; i < k; ++i) {
-        k_edge_copy<MS><<<grid_for(n, 256), 256, 0, g->stream>>>(a);
-        k_edge_send<MS, UNI><<<grid_for(g->E, 256), 256, 0, g->stream>>>(a);
-        k_edge_combine<MS, UNI><<<grid_for(g->V, 256), 256, 0, g->stream>>>(a);
-        k_edge_normalise_node0<MS><<<1, 32, 0, g->stream>>>(a);
-        k_edge_delta<MS, UNI><<<grid_for(g->E, 256), 256, 0, g->stream>>>(a);
-        BP_CUDA(cudaGetLastError());
+static int edge_grid(const bp_graph *g, unsigned *grid, bool serial) {
+    static int bps_f64 = 0, bps_ser = 0;
+    static std::mutex mu;
+    int bps = 0;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        int &b = serial ? bps_ser : bps_f64;
+        if (b == 0) {
+            if (serial)
+                BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edge_loop<MS, UNI, true>, kEdgeThreads, 0));
+            else
+                BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edge_loop<MS, UNI, false>, kEdgeThreads, 0));
+            if (b < 1) return set_error(BP_ERR_CUDA, "edge-schedule kernel does not fit an SM");
+        }
+        bps = b;
     }
+    int dev = 0, sms = 0;
+    BP_CUDA(cudaGetDevice(&dev));
+    BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    *grid = (unsigned)std::min<uint64_t>((uint64_t)bps * sms, grid_for(std::max(g->E, g->V), kEdgeThreads));
     return BP_OK;
 }
 
-static int enqueue_iterations(bp_graph *g, int schedule, uint32_t k, bool serial, int variant) {
-    if (schedule == BP_SCHEDULE_NODE && variant == BP_KERNEL_SPLIT)
-        BP_DISPATCH_MS(g->ms, g->uniform != 0, enqueue_split_iterations, g, k, serial);
-    if (schedule == BP_SCHEDULE_NODE)
-        BP_DISPATCH_MS(g->ms, g->uniform != 0, enqueue_node_iterations, g, k, serial, variant);
-    BP_DISPATCH_MS(g->ms, g->uniform != 0, enqueue_edge_iterations, g, k, serial, variant);
+template <int MS, bool UNI>
+static int launch_edge_loop(bp_graph *g, unsigned grid, bool serial) {
+    EdgeArgs a = edge_args(g);
+    void *args[] = {(void *)&a};
+    const void *fn = serial ? (const void *)k_edge_loop<MS, UNI, true> : (const void *)k_edge_loop<MS, UNI, false>;
+    BP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kEdgeThreads), args, 0, g->stream));
+    return BP_OK;
+}
+
+static int enqueue_iterations(bp_graph *g, uint32_t k, bool serial, int variant) {
+    if (variant == BP_KERNEL_SPLIT) BP_DISPATCH_MS(g->ms, g->uniform != 0, enqueue_split_iterations, g, k, serial);
+    BP_DISPATCH_MS(g->ms, g->uniform != 0, enqueue_node_iterations, g, k, serial, variant);
 }
 
 static int flood_grid(bp_graph *g, int variant, uint32_t *grid, bool serial) {
@@ -2481,7 +2326,7 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
         return set_error(BP_ERR_INVALID, "unknown kernel variant %d", opt->kernel_variant);
     if (variant == BP_KERNEL_STAGED_TILE && opt->schedule == BP_SCHEDULE_NODE && !staged_applies(g, opt->schedule, serial))
         return set_error(BP_ERR_INVALID, "staged tiles need a uniform 2-state graph of mean in-degree <= 4.5 and the f64 delta");
-    uint32_t grid_blocks = grid_for(g->E, 256);
+    uint32_t grid_blocks = 1;
     if (opt->schedule == BP_SCHEDULE_NODE && (st = flood_grid(g, variant, &grid_blocks, serial))) return st;
     // small graphs (a co-resident block per tile), node schedule, f64 delta,
     // block tiles: every iteration in one cooperative launch
@@ -2496,8 +2341,14 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
             if ((st = fg())) return st;
         }
     }
+    unsigned egrid = 0;
+    if (opt->schedule == BP_SCHEDULE_EDGE) {
+        auto eg = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, edge_grid, g, &egrid, serial); };
+        if ((st = eg())) return st;
+    }
     // double-buffered partials, and in serial mode 8 more per block for the
     // grid-wide narrowing
+    if (egrid) grid_blocks = (serial ? 10u : 2u) * egrid;
     if (fgrid) grid_blocks = std::max(grid_blocks, (serial ? 10u : 2u) * fgrid);
     if ((st = ensure_partials(g, grid_blocks))) return st;
     if (serial && (st = ensure_absdiff(g))) return st;
@@ -2505,7 +2356,7 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
 
     const uint32_t n_launch = ce <= 1 ? max_it : ((max_it + ce - 1) / ce) * ce;
     uint32_t chunk = opt->graph_chunk;
-    if (chunk == 0) chunk = opt->schedule == BP_SCHEDULE_NODE ? 32 : 8;
+    if (chunk == 0) chunk = 32;
     if (chunk > n_launch) chunk = n_launch;
 
     LoopyCtl c = {};
@@ -2523,6 +2374,10 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
     c.plo = c.phi = -1.0;
     c.prev_exact = 1;
     c.delta_exact = 1;
+    // the edge loop's barriers also wait for one thread's work: node 0's
+    // normalisations over the runs of equal state counts, and the serial sum
+    // where it has to be formed
+    if (egrid) c.wait_ms = 2000u + g->nruns / 1000u + (serial ? (uint32_t)(c.n_terms / 50000u) : 0u);
     // test hook of the one-launch loop's bounded grid barrier: a shorter
     // wait limit, and a block that does not arrive at the first barrier
     if (const char *env = getenv("BP_DEBUG_WAIT_MS")) c.wait_ms = (uint32_t)strtoul(env, nullptr, 10);
@@ -2538,14 +2393,17 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
         if ((st = conv())) return st;
     }
 
-    if (fgrid) {
+    if (egrid) {
+        BP_CUDA(cudaEventRecord(g->ev0, g->stream));
+        auto le = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, launch_edge_loop, g, egrid, serial); };
+        if ((st = le())) return st;
+    } else if (fgrid) {
         BP_CUDA(cudaEventRecord(g->ev0, g->stream));
         auto lf = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, launch_fused, g, fgrid, fntiles, serial); };
         if ((st = lf())) return st;
     } else {
-        // CUDA graph of `chunk` iterations, cached per (schedule, delta, chunk)
-        const uint64_t key = 1ull | ((uint64_t)opt->schedule << 1) | ((uint64_t)serial << 2) |
-                             ((uint64_t)variant << 4) | ((uint64_t)chunk << 8);
+        // CUDA graph of `chunk` iterations, cached per (delta, kernel, chunk)
+        const uint64_t key = 1ull | ((uint64_t)serial << 2) | ((uint64_t)variant << 4) | ((uint64_t)chunk << 8);
         bp_graph::CachedGraph *slot = nullptr;
         for (auto &cg : g->loop_graph)
             if (cg.exec && cg.key == key) slot = &cg;
@@ -2562,7 +2420,7 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
             }
             cudaGraph_t graph = nullptr;
             BP_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-            st = enqueue_iterations(g, opt->schedule, chunk, serial, variant);
+            st = enqueue_iterations(g, chunk, serial, variant);
             cudaError_t ce2 = cudaStreamEndCapture(g->stream, &graph);
             if (st) {
                 if (graph) cudaGraphDestroy(graph);
