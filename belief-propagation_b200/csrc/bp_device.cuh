@@ -219,6 +219,28 @@ __device__ __forceinline__ void send_msg_regs(const float *j, const float *buf, 
     for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
 }
 
+// the same arithmetic on a table in shared memory, row after row
+template <int MS, bool UNI>
+__device__ __forceinline__ void send_msg_rows(const float *J, const float *buf, int x, int y, float *m) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MS; ++i) {
+        float partial = 0.0f;
+        if (UNI || i < x) {
+            float row[MS];
+            ldv<MS>(J + i * MS, row);
+#pragma unroll
+            for (int c = 0; c < MS; ++c)
+                if (UNI || c < y) partial = FADD(partial, FMUL(row[c], buf[c]));
+            sum = FADD(sum, partial);
+        }
+        m[i] = partial;
+    }
+    if (sum <= 0.0f) sum = 1.0f;
+#pragma unroll
+    for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
+}
+
 template <int MS, bool UNI>
 __device__ __forceinline__ void send_msg(const float *__restrict__ J, const float *buf, int x, int y,
                                          float *m) {

@@ -179,6 +179,15 @@ struct bp_graph {
 
     bpx::TreeData tree;
 
+    // the one-launch loop of small graphs, planned on first use: [serial delta]
+    struct LoopPlan {
+        int state = 0;                   // 0 not planned yet
+        uint32_t grid = 0, smem = 0;     // no grid: the graph has too many tiles
+        bool wide = false;
+    } loop_plan[2];
+    uint64_t *loop_flags = nullptr;      // [grid] its barrier's flags (device)
+    uint64_t loop_runs = 0;              // runs so far: every run's flags lie above the last one's
+
     // cached CUDA graphs of the iteration loop
     struct CachedGraph {
         cudaGraphExec_t exec = nullptr;

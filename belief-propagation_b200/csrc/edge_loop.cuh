@@ -29,8 +29,8 @@
 // 50,001 nodes x 3 states.  The orbit is now followed only until its period
 // is known (Brent's method), and the rest taken modulo the period.
 // 50,001 nodes, 200,003 edges, 3 states, serial delta, 50 iterations:
-// 105.9 -> 42.1 ms per solve (1.5 ms of it the iterations; the rest forms the
-// serial sum in the 34 checks that need it); f64 delta 0.72 ms.
+// 105.9 -> 4.0 ms per solve (0.9 ms of it the iterations; the rest forms the
+// serial sum in the 38 checks that need it, serial_grid.cuh); f64 delta 0.71 ms.
 #pragma once
 
 struct EdgeArgs {
@@ -49,7 +49,6 @@ struct EdgeArgs {
 };
 
 constexpr int kEdgeThreads = 256;
-constexpr uint32_t kEdgeStage = 2048;   // floats of staging for the serial delta
 
 // b = normalised once with its first s slots (a sum that is not positive
 // leaves it, graph.c:1046-1061); whether any bit changed
@@ -106,7 +105,6 @@ template <int MS, bool UNI, bool SER>
 __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
     constexpr int NT = kEdgeThreads;
     __shared__ double red[NT / 32];
-    __shared__ __align__(16) float buf[SER ? kEdgeStage : 4];
     __shared__ LoopyCtl s_ctl;
     __shared__ uint32_t s_fail;
 
@@ -221,8 +219,10 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
         for (uint32_t k = threadIdx.x; k < gridDim.x; k += NT) sum += __ldcg(part + k);
         const double tot = block_sum<NT>(sum, red);
         if (SER && want) {
-            if (!grid_serial_check<NT>(ctl, s_ctl, a.partials, a.absdiff, gen, &s_fail, tot, buf, kEdgeStage, red))
-                break;
+            SerialCheck x = serial_check(&s_ctl, broadcast_sum(tot));
+            if (x.d < 0 && !grid_serial_form<NT>(x, s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red)) break;
+            __syncthreads();   // every thread has read s_ctl
+            if (threadIdx.x == 0) serial_commit(&s_ctl, x);
         } else if (threadIdx.x == 0) {
             finalize(&s_ctl, want, (float)tot, tot);
         }
@@ -230,5 +230,6 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
         // the next iteration's sends read the beliefs combined here
         if (!s_ctl.done && !grid_barrier(ctl, gen, &s_fail)) break;
     }
+    if (SER && !s_fail && s_ctl.done) grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red);
     if (first == 0 && !s_fail) publish_ctl(ctl, s_ctl);
 }

@@ -437,19 +437,17 @@ __device__ __forceinline__ void serial_narrow(SerialCheck &x, int which, double 
 // iteration kernels' register allocation is not shaped by it)
 template <int NT>
 __device__ __noinline__ void serial_form(SerialCheck &x, const LoopyCtl *c, const float *absdiff, float *buf,
-                                         uint32_t cap, bool narrow) {
+                                         uint32_t cap) {
     const uint64_t n = c->n_terms, stride = c->ad_stride;
     const uint32_t pb = c->prev_buf;
     const float tol = c->tol;
     double lo, hi;
-    if (narrow) {
-        ++x.refines;
-        if (refine_block<NT>(absdiff + (size_t)x.cb * stride, n, buf, cap, lo, hi)) serial_narrow(x, 0, lo, hi);
+    ++x.refines;
+    if (refine_block<NT>(absdiff + (size_t)x.cb * stride, n, buf, cap, lo, hi)) serial_narrow(x, 0, lo, hi);
+    x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, tol);
+    if (x.d < 0 && !x.p_exact && !x.p_ref) {
+        if (refine_block<NT>(absdiff + (size_t)pb * stride, n, buf, cap, lo, hi)) serial_narrow(x, 1, lo, hi);
         x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, tol);
-        if (x.d < 0 && !x.p_exact && !x.p_ref) {
-            if (refine_block<NT>(absdiff + (size_t)pb * stride, n, buf, cap, lo, hi)) serial_narrow(x, 1, lo, hi);
-            x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, tol);
-        }
     }
     if (x.d < 0 && !x.s_exact) {
         x.s = exact_serial_sum<NT>(absdiff + (size_t)x.cb * stride, n, buf, cap);
@@ -509,7 +507,7 @@ __device__ __noinline__ void finalize_serial(LoopyCtl *c, bool want, double T, c
         return;
     }
     SerialCheck x = serial_check(c, broadcast_sum(T));
-    if (x.d < 0) serial_form<NT>(x, c, absdiff, buf, cap, true);
+    if (x.d < 0) serial_form<NT>(x, c, absdiff, buf, cap);
     __syncthreads();   // every thread has read c
     if (threadIdx.x == 0) serial_commit(c, x);
 }
@@ -776,18 +774,14 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood(const FloodArgs a,
     reduce_and_finalize<NT, SER>(ctl, a.partials, dsum, want, red, &s_last, a.absdiff, sm, EMAX * MS);
 }
 
-// Small graphs: every iteration in one cooperative launch.  When each tile
-// has a block of its own on the GPU at once (a cooperative launch guarantees
-// co-residency), the per-iteration launch costs more than the iteration, so
-// the blocks loop over the iterations themselves and meet at a grid barrier
-// after each one (its wait bounded by kWaitNs; a block that gives up sets
-// bar_fail, and the others then give up at the next barrier).  Each block
-// keeps a copy of the control block and, after the barrier, sums the
-// per-block delta partials in the same fixed order as k_flood's last block
-// does, so every block takes the same stopping decision and the results equal
-// the one-launch-per-iteration loop's.  Partials are double-buffered by
-// iteration parity: a block writes the next iteration's while others may
-// still read this one's.
+// ---- one cooperative launch for a whole run --------------------------------
+// Blocks that are all resident at once loop over the iterations themselves and
+// meet at a grid barrier (its wait bounded by kBarrierWaitNs; a block that
+// gives up sets bar_fail, and the others then give up at the next barrier).
+// Each block keeps a copy of the control block and sums the per-block delta
+// partials in the same fixed order, so every block takes the same stopping
+// decision.  Partials are double-buffered by iteration parity: a block writes
+// the next iteration's while others may still read this one's.
 constexpr uint64_t kBarrierWaitNs = 2000000000ull;   // 2 s
 
 // The wait is bounded by kBarrierWaitNs, or by c->wait_ms when the host set
@@ -823,166 +817,6 @@ __device__ __forceinline__ bool grid_barrier(LoopyCtl *c, uint32_t &gen, uint32_
     return *s_fail == 0;
 }
 
-// the narrowed intervals of an undecided check in the one-launch loop,
-// grid-wide: each block takes one slice of the terms (of s, and of the
-// previous delta when that is neither exact nor narrowed yet); slice sums,
-// a barrier, each slice's errors from its exact prefix, a barrier, and
-// every block sums the same slices in the same order, so all blocks end with
-// the same intervals.  Scratch: 8 doubles per block after the partials.
-// false when a barrier gave up.
-template <int NT>
-__device__ bool grid_refine(double *partials, const float *absdiff, LoopyCtl *ctl, uint32_t &gen, uint32_t *s_fail,
-                            SerialCheck &x, const LoopyCtl &sc, float *buf, uint32_t cap, double *red) {
-    __shared__ double s_b[4];
-    __shared__ double s_v[NT / 32][6];
-    __shared__ double s_t[6];
-    const uint64_t n = sc.n_terms, stride = sc.ad_stride;
-    const double c0 = refine_c0(n);
-    if (c0 == 0.0) return true;
-    const bool do_p = !x.p_exact && !x.p_ref;
-    ++x.refines;
-    const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-    double *scr = partials + 2 * (size_t)G;
-    const uint64_t L = ((n + G - 1) / G + 3) & ~3ull;
-    const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
-    const float *xs = absdiff + (size_t)x.cb * stride, *xp = absdiff + (size_t)sc.prev_buf * stride;
-    double ls = 0.0, lp = 0.0;
-    for (uint64_t k = lo + tid; k < hi; k += NT) {
-        ls += (double)__ldcg(xs + k);
-        if (do_p) lp += (double)__ldcg(xp + k);
-    }
-    ls = block_sum<NT>(ls, red);
-    lp = block_sum<NT>(lp, red);
-    if (tid == 0) {
-        scr[b] = ls;
-        scr[G + b] = lp;
-    }
-    if (!grid_barrier(ctl, gen, s_fail)) return false;
-    // prefixes before this slice, and the totals (the same in every block)
-    double ps = 0.0, ts = 0.0, pp = 0.0, tp = 0.0;
-    for (uint32_t k = tid; k < G; k += NT) {
-        const double vs = __ldcg(scr + k), vp = __ldcg(scr + G + k);
-        ts += vs;
-        tp += vp;
-        if (k < b) {
-            ps += vs;
-            pp += vp;
-        }
-    }
-    ps = block_sum<NT>(ps, red);
-    ts = block_sum<NT>(ts, red);
-    pp = block_sum<NT>(pp, red);
-    tp = block_sum<NT>(tp, red);
-    if (tid == 0) {
-        s_b[0] = ps;
-        s_b[1] = ts;
-        s_b[2] = pp;
-        s_b[3] = tp;
-    }
-    __syncthreads();
-    ps = s_b[0];
-    ts = s_b[1];
-    pp = s_b[2];
-    tp = s_b[3];
-    double pe;
-    const Refine rs = refine_segment<NT>(xs, lo, hi, ps, c0, buf, cap, pe);
-    Refine rp{0.0, 0.0, 0.0, false};
-    if (do_p) rp = refine_segment<NT>(xp, lo, hi, pp, c0, buf, cap, pe);
-    const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    if (tid == 0) {
-        scr[2 * (size_t)G + b] = rs.E;
-        scr[3 * (size_t)G + b] = rs.A;
-        scr[4 * (size_t)G + b] = rs.bad ? inf : rs.B;
-        scr[5 * (size_t)G + b] = rp.E;
-        scr[6 * (size_t)G + b] = rp.A;
-        scr[7 * (size_t)G + b] = rp.bad ? inf : rp.B;
-    }
-    if (!grid_barrier(ctl, gen, s_fail)) return false;
-    // the same totals in every block: fixed per-thread slices, then a fixed
-    // reduction order; the bounds (j = 2, 5) rounded up
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (uint32_t k = tid; k < G; k += NT) {
-#pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            const double y = __ldcg(scr + (size_t)(2 + j) * G + k);
-            v[j] = (j == 2 || j == 5) ? __dadd_ru(v[j], y) : v[j] + y;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 6; ++j)
-        for (int d = 16; d > 0; d >>= 1) {
-            const double y = __shfl_xor_sync(0xffffffffu, v[j], d);
-            v[j] = (j == 2 || j == 5) ? __dadd_ru(v[j], y) : v[j] + y;
-        }
-    if ((tid & 31u) == 0u)
-        for (int j = 0; j < 6; ++j) s_v[tid >> 5][j] = v[j];
-    __syncthreads();
-    if (tid == 0)
-        for (int j = 0; j < 6; ++j) {
-            double t = 0.0;
-            for (int w = 0; w < NT / 32; ++w) t = (j == 2 || j == 5) ? __dadd_ru(t, s_v[w][j]) : t + s_v[w][j];
-            s_t[j] = t;
-        }
-    __syncthreads();
-    double lo2, hi2;
-    const Refine Rs{s_t[0], s_t[1], s_t[2], !(s_t[2] < inf)};
-    if (!Rs.bad) {
-        refine_interval(ts, Rs, n, lo2, hi2);
-        serial_narrow(x, 0, lo2, hi2);
-    }
-    if (do_p) {
-        const Refine Rp{s_t[3], s_t[4], s_t[5], !(s_t[5] < inf)};
-        if (!Rp.bad) {
-            refine_interval(tp, Rp, n, lo2, hi2);
-            serial_narrow(x, 1, lo2, hi2);
-        }
-    }
-    x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, sc.tol);
-    __syncthreads();   // s_t and s_b are free
-    return true;
-}
-
-// one serial-mode check of a one-launch loop: every block of the grid calls it
-// with the same f64 sum `tot` (in thread 0) and reaches the same decision; when
-// the bounds cannot decide, block 0 forms the serial sums and the blocks meet
-// once more to read them.  The terms are triple-buffered by check, so no
-// block overwrites them while block 0 reads.  sc: the block's copy of the
-// control block, updated.  false when a barrier gave up.
-template <int NT>
-__device__ __forceinline__ bool grid_serial_check(LoopyCtl *ctl, LoopyCtl &sc, double *partials, const float *absdiff,
-                                                  uint32_t &gen, uint32_t *s_fail, double tot, float *buf,
-                                                  uint32_t cap, double *red) {
-    SerialCheck x = serial_check(&sc, broadcast_sum(tot));
-    if (x.d < 0 && !grid_refine<NT>(partials, absdiff, ctl, gen, s_fail, x, sc, buf, cap, red)) return false;
-    if (x.d < 0) {
-        const bool s_ex0 = x.s_exact, p_ex0 = x.p_exact;
-        if (blockIdx.x == 0) {
-            serial_form<NT>(x, &sc, absdiff, buf, cap, false);
-            if (threadIdx.x == 0) {
-                ctl->fb_s = x.s;
-                ctl->fb_p = (float)x.plo;
-                ctl->fb_pform = x.p_exact && !p_ex0;
-            }
-        }
-        if (!grid_barrier(ctl, gen, s_fail)) return false;
-        if (blockIdx.x != 0) {
-            if (!s_ex0) {
-                x.s = *(volatile float *)&ctl->fb_s;
-                x.lo = x.hi = (double)x.s;
-                x.s_exact = true;
-            }
-            if (*(volatile uint32_t *)&ctl->fb_pform) {
-                x.plo = x.phi = (double)*(volatile float *)&ctl->fb_p;
-                x.p_exact = x.p_new = true;
-            }
-            x.d = serial_decide(x.lo, x.hi, x.s_exact, x.plo, x.phi, x.p_exact, sc.tol);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) serial_commit(&sc, x);
-    return true;
-}
-
 // the run's outcome from a block's copy of the control block (one thread)
 __device__ __forceinline__ void publish_ctl(LoopyCtl *ctl, const LoopyCtl &sc) {
     ctl->it = sc.it;
@@ -1009,55 +843,8 @@ __device__ __forceinline__ void publish_ctl(LoopyCtl *ctl, const LoopyCtl &sc) {
     ctl->done = sc.done;
 }
 
-template <int MS, bool UNI, int FU, bool SER = false, int MB = flood_min_blocks<MS, FU>()>
-__global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood_fused(const FloodArgs a, uint32_t ntiles) {
-    constexpr int NT = flood_nt<MS>();
-    constexpr uint32_t EMAX = flood_smem_floats<MS>() / MS;
-    __shared__ __align__(16) float sm[EMAX * MS];
-    __shared__ double red[NT / 32];
-    __shared__ LoopyCtl s_ctl;
-    __shared__ uint32_t s_fail;
-
-    LoopyCtl *ctl = a.ctl;
-    if (threadIdx.x == 0) {
-        s_ctl = *ctl;
-        s_fail = 0;
-    }
-    __syncthreads();
-    const uint64_t keep = l2_evict_last_policy();
-    uint32_t gen = 0;
-    while (!s_ctl.done) {
-        const uint32_t it = s_ctl.it, ce = s_ctl.check_every;
-        const bool want = (ce <= 1) || ((it + 1) % ce == 0);
-        const int mp = (int)((s_ctl.msg_parity0 + it) & 1u), qp = (int)((s_ctl.q_parity0 + it) & 1u);
-        const float *__restrict__ m_old = mp ? a.msg1 : a.msg0;
-        float *__restrict__ m_new = mp ? a.msg0 : a.msg1;
-        const float *__restrict__ q_in = qp ? a.q1 : a.q0;
-        float *__restrict__ q_out = qp ? a.q0 : a.q1;
-        float *absd = SER ? check_buffer(&s_ctl, a.absdiff, it, want) : nullptr;
-        double dsum = 0.0;
-        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            flood_tile<MS, UNI, FU>(a, tile, want, absd, m_old, m_new, q_in, q_out, keep, sm, dsum);
-            __syncthreads();
-        }
-        const double t = block_sum<NT>(dsum, red);
-        double *part = a.partials + (size_t)(it & 1u) * gridDim.x;
-        if (threadIdx.x == 0) part[blockIdx.x] = t;
-        if (!grid_barrier(ctl, gen, &s_fail)) break;
-        double acc = 0.0;
-        for (uint32_t k = threadIdx.x; k < gridDim.x; k += NT) acc += __ldcg(part + k);
-        const double tot = block_sum<NT>(acc, red);
-        if (SER && want) {
-            if (!grid_serial_check<NT>(ctl, s_ctl, a.partials, a.absdiff, gen, &s_fail, tot, sm, EMAX * MS, red)) break;
-        } else if (threadIdx.x == 0) {
-            finalize(&s_ctl, want, (float)tot, tot);
-        }
-        __syncthreads();
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !s_fail) {
-        publish_ctl(ctl, s_ctl);
-    }
-}
+#include "serial_grid.cuh"
+#include "flood_loop.cuh"
 
 // Staged form of k_flood for uniform 2-state graphs (the layout is written
 // for 2 or 4 states; 4-state tables do not leave room for two stages of a
@@ -1616,6 +1403,15 @@ static int ensure_absdiff(bp_graph *g) {
     return BP_OK;
 }
 
+// the one-launch loop's barrier flags, one per block; zero below every run's tag
+static int ensure_loop_flags(bp_graph *g, uint32_t n) {
+    if (g->loop_flags) return BP_OK;
+    int st = dev_alloc(g, (void **)&g->loop_flags, sizeof(uint64_t) * n);
+    if (st) return st;
+    BP_CUDA(cudaMemsetAsync(g->loop_flags, 0, sizeof(uint64_t) * n, g->stream));
+    return BP_OK;
+}
+
 // runs of equal state count over node order, for the node-0 normalisation
 static int ensure_runs(bp_graph *g) {
     if (g->run_len || g->V == 0) return BP_OK;
@@ -2110,35 +1906,74 @@ static bool staged_applies(const bp_graph *g, int schedule, bool serial) {
     return (any & 15u) == 0;
 }
 
-// the fused loop: its grid (at most one co-resident block per tile), or 0
-// when the graph has more tiles than the GPU holds blocks at once
-template <int MS, bool UNI>
-static int fused_grid(const bp_graph *g, unsigned *grid, uint32_t *ntiles, bool serial) {
-    constexpr int FU = flood_unroll<MS>();
-    static int bps_f64 = -1, bps_ser = -1;
-    int &bps = serial ? bps_ser : bps_f64;
-    if (bps < 0) {
-        if (serial)
-            BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_flood_fused<MS, UNI, FU, true>,
-                                                                  flood_nt<MS>(), 0));
-        else
-            BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_flood_fused<MS, UNI, FU>, flood_nt<MS>(), 0));
-    }
-    int dev = 0, sms = 0;
+// the one-launch loop of small graphs: its grid (a co-resident block per
+// tile) and shared memory, or no grid when the graph has more tiles than the
+// GPU holds blocks at once.  Two tiles' worth of an average tile's data is
+// asked for where an SM has it: the messages, source ids and tables of a tile
+// up to twice the average size stay on chip.
+template <int MS, bool UNI, bool SER, bool WIDE>
+static int loop_plan_of(bp_graph *g, uint32_t tiles, uint32_t per_sm, bp_graph::LoopPlan *p) {
+    const void *fn = (const void *)k_flood_loop<MS, UNI, SER, WIDE>;
+    cudaFuncAttributes fa;
+    BP_CUDA(cudaFuncGetAttributes(&fa, fn));
+    int dev = 0, per_block = 0, per_mp = 0, reserved = 0;
     BP_CUDA(cudaGetDevice(&dev));
-    BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    *ntiles = grid_for(g->V, flood_nt<MS>());
-    *grid = (bps > 0 && (uint64_t)*ntiles <= (uint64_t)bps * sms) ? *ntiles : 0u;
+    BP_CUDA(cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    BP_CUDA(cudaDeviceGetAttribute(&per_mp, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    BP_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+    const int64_t most = std::min<int64_t>(per_block - (int64_t)fa.sharedSizeBytes,
+                                           per_mp / (int64_t)per_sm - reserved - (int64_t)fa.sharedSizeBytes - 128);
+    const int64_t least = sizeof(float) * flood_smem_floats<MS>();
+    if (most < least) return BP_OK;
+    const uint64_t avg = g->E / tiles + 1;
+    const uint64_t want = 4 * (2 * (uint64_t)flood_nt<MS>() * MS + 2 * avg * ((SER ? 3 : 2) * MS + 1 + loop_table_stride<MS>()) + 32);
+    const int64_t smem = std::min<int64_t>(most, (int64_t)std::max<uint64_t>(least, want)) & ~127ll;
+    BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int bps = 0;
+    BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, flood_nt<MS>(), (size_t)smem));
+    if (bps < (int)per_sm) return BP_OK;
+    p->grid = tiles;
+    p->smem = (uint32_t)smem;
+    p->wide = WIDE;
     return BP_OK;
 }
 
 template <int MS, bool UNI>
-static int launch_fused(bp_graph *g, unsigned grid, uint32_t ntiles, bool serial) {
-    constexpr int FU = flood_unroll<MS>();
-    FloodArgs a = flood_args(g);
-    void *args[] = {(void *)&a, (void *)&ntiles};
-    const void *fn = serial ? (const void *)k_flood_fused<MS, UNI, FU, true> : (const void *)k_flood_fused<MS, UNI, FU>;
-    BP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(flood_nt<MS>()), args, 0, g->stream));
+static int loop_plan(bp_graph *g, bool serial) {
+    bp_graph::LoopPlan &p = g->loop_plan[serial ? 1 : 0];
+    if (p.state) return BP_OK;
+    int dev = 0, sms = 0;
+    BP_CUDA(cudaGetDevice(&dev));
+    BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const uint32_t tiles = grid_for(g->V, flood_nt<MS>()), per_sm = (tiles + sms - 1) / sms;
+    int st = BP_OK;
+    if (per_sm <= (uint32_t)loop_min_blocks<MS, true>())
+        st = serial ? loop_plan_of<MS, UNI, true, true>(g, tiles, per_sm, &p)
+                    : loop_plan_of<MS, UNI, false, true>(g, tiles, per_sm, &p);
+    else if (per_sm <= (uint32_t)loop_min_blocks<MS, false>())
+        st = serial ? loop_plan_of<MS, UNI, true, false>(g, tiles, per_sm, &p)
+                    : loop_plan_of<MS, UNI, false, false>(g, tiles, per_sm, &p);
+    p.state = st ? 0 : 1;
+    return st;
+}
+
+template <int MS, bool UNI>
+static int launch_loop(bp_graph *g, bool serial) {
+    const bp_graph::LoopPlan &p = g->loop_plan[serial ? 1 : 0];
+    LoopArgs a;
+    a.f = flood_args(g);
+    a.flags = g->loop_flags;
+    a.run_tag = ++g->loop_runs << 32;
+    a.smem = p.smem;
+    const void *fn;
+    if (p.wide)
+        fn = serial ? (const void *)k_flood_loop<MS, UNI, true, true> : (const void *)k_flood_loop<MS, UNI, false, true>;
+    else
+        fn = serial ? (const void *)k_flood_loop<MS, UNI, true, false> : (const void *)k_flood_loop<MS, UNI, false, false>;
+    // the limit is the function's, shared by every graph: set for this launch
+    BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    void *args[] = {(void *)&a};
+    BP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.grid), dim3(flood_nt<MS>()), args, p.smem, g->stream));
     return BP_OK;
 }
 
@@ -2326,30 +2161,29 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
         return set_error(BP_ERR_INVALID, "unknown kernel variant %d", opt->kernel_variant);
     if (variant == BP_KERNEL_STAGED_TILE && opt->schedule == BP_SCHEDULE_NODE && !staged_applies(g, opt->schedule, serial))
         return set_error(BP_ERR_INVALID, "staged tiles need a uniform 2-state graph of mean in-degree <= 4.5 and the f64 delta");
+    // small graphs (a co-resident block per tile), node schedule, block tiles:
+    // every iteration in one cooperative launch (BP_FLOOD_FUSED=0 keeps the
+    // launch-per-iteration loop); the edge schedule always runs as one
     uint32_t grid_blocks = 1;
-    if (opt->schedule == BP_SCHEDULE_NODE && (st = flood_grid(g, variant, &grid_blocks, serial))) return st;
-    // small graphs (a co-resident block per tile), node schedule, f64 delta,
-    // block tiles: every iteration in one cooperative launch
-    // (BP_FLOOD_FUSED=0 keeps the launch-per-iteration loop)
-    unsigned fgrid = 0;
-    uint32_t fntiles = 0;
-    {
-        const char *env = getenv("BP_FLOOD_FUSED");
-        if (opt->schedule == BP_SCHEDULE_NODE && variant == BP_KERNEL_BLOCK_TILE &&
-            !(env && env[0] == '0')) {
-            auto fg = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, fused_grid, g, &fgrid, &fntiles, serial); };
-            if ((st = fg())) return st;
-        }
-    }
-    unsigned egrid = 0;
+    unsigned fgrid = 0, egrid = 0;
     if (opt->schedule == BP_SCHEDULE_EDGE) {
         auto eg = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, edge_grid, g, &egrid, serial); };
         if ((st = eg())) return st;
+    } else if (variant == BP_KERNEL_BLOCK_TILE) {
+        const char *env = getenv("BP_FLOOD_FUSED");
+        if (!(env && env[0] == '0')) {
+            auto lp = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, loop_plan, g, serial); };
+            if ((st = lp())) return st;
+            fgrid = g->loop_plan[serial ? 1 : 0].grid;
+        }
     }
-    // double-buffered partials, and in serial mode 8 more per block for the
-    // grid-wide narrowing
-    if (egrid) grid_blocks = (serial ? 10u : 2u) * egrid;
-    if (fgrid) grid_blocks = std::max(grid_blocks, (serial ? 10u : 2u) * fgrid);
+    if (const uint32_t one = std::max(fgrid, egrid)) {
+        // double-buffered partials, and in serial mode the serial sums' scratch
+        grid_blocks = (2u + (serial ? kSumScratch : 0u)) * one;
+        if (fgrid && (st = ensure_loop_flags(g, fgrid))) return st;
+    } else if ((st = flood_grid(g, variant, &grid_blocks, serial))) {
+        return st;
+    }
     if ((st = ensure_partials(g, grid_blocks))) return st;
     if (serial && (st = ensure_absdiff(g))) return st;
     if (opt->schedule == BP_SCHEDULE_EDGE && ((st = ensure_runs(g)) || (st = ensure_edge_pos(g)))) return st;
@@ -2399,7 +2233,7 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
         if ((st = le())) return st;
     } else if (fgrid) {
         BP_CUDA(cudaEventRecord(g->ev0, g->stream));
-        auto lf = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, launch_fused, g, fgrid, fntiles, serial); };
+        auto lf = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, launch_loop, g, serial); };
         if ((st = lf())) return st;
     } else {
         // CUDA graph of `chunk` iterations, cached per (delta, kernel, chunk)
@@ -2444,9 +2278,9 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
             }
         }
     }
-    if (serial) {
+    if (serial && !fgrid && !egrid) {
         // the returned delta and previous delta where the loop decided
-        // without forming them
+        // without forming them (the one-launch loops form them themselves)
         k_delta_final<<<2, 1024, 0, g->stream>>>(g->ctl, g->absdiff);
         BP_CUDA(cudaGetLastError());
     }

@@ -1,0 +1,299 @@
+// serial_grid.cuh -- the reference's serial fp32 delta formed by a whole
+// resident grid.  Included by loopy.cu (it uses the binade arithmetic of
+// block_serial_sum and the grid barrier there).
+//
+// Inside one binade of the running sum each add moves m (s = m U) by an
+// increment that depends on m only through its parity, so a run of terms is
+// a pair of increments (SumStep) and runs compose.  Every block takes one
+// slice of the terms and every warp a part of it; from the slice's f64 prefix
+// it guesses the binade(s) the running sum has there -- one, or the two on
+// either side of a crossing -- and composes its terms' steps for each guess.
+// One warp then walks the slices in order: the walk knows the exact running
+// sum, so a slice's pair counts only when it was made for the binade the sum
+// is in and the sum stays below the binade's top; otherwise that slice is
+// walked warp part by warp part, and a part that crosses (or was guessed
+// wrong) is added term by term.  The guesses decide the speed, never the
+// value: the result is the one-by-one sum bit for bit.
+//
+// Before, one block of the grid formed the sum while the others waited: 600k
+// terms 1.1 ms, now 75 us (592 blocks of 256 threads; bounded by three grid
+// barriers and the walk over a dozen crossings).  The interval narrowed from
+// the terms' own errors, which decided most checks before, took 29 us of
+// grid time each on 80k terms and still left the sum to be formed where the
+// delta creeps; the sum itself decides in one go.
+#pragma once
+
+// doubles of scratch per block behind the grid's 2 x G delta partials
+constexpr uint32_t kSumScratch = 42;
+constexpr int32_t kAnyUnit = 0x7fffffff;   // an empty slice: nothing to add in any binade
+
+struct SumRec {
+    int32_t ua, ub;   // unit exponents the two pairs were made for
+    SumStep a, b;
+    uint32_t pad[2];
+};
+static_assert(sizeof(SumRec) == 32, "two 16-byte loads");
+
+// the scratch arrays of sum j (0: the check's terms, 1: the previous check's)
+struct SumScr {
+    double *slice;   // [G]
+    SumRec *rec;     // [G]
+    uint4 *part;     // [G][8] the warps' pairs: a.e, a.o, b.e, b.o
+    __device__ SumScr(double *partials, uint32_t G, int j) {
+        double *base = partials + 2 * (size_t)G;
+        slice = base + (size_t)j * G;
+        rec = reinterpret_cast<SumRec *>(base + 2 * (size_t)G) + (size_t)j * G;
+        part = reinterpret_cast<uint4 *>(base + 10 * (size_t)G) + (size_t)j * G * 8;
+    }
+};
+
+// unit exponent of the binade of a positive double, within fp32's range
+__device__ __forceinline__ int32_t sum_unit(double s) {
+    if (!(s >= 0x1p-126)) return -149;
+    return min(ilogb(s), 127) - 23;
+}
+
+// terms x[lo, hi) in order, composed for unit exponents ua and ub; lane 0 of
+// the warp gets the pairs
+__device__ __forceinline__ void warp_sum_steps(const float *__restrict__ x, uint64_t lo, uint64_t hi, int32_t ua,
+                                               int32_t ub, SumStep &A, SumStep &B) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t k = (hi - lo + 31u) / 32u;
+    const uint64_t p0 = min(lo + lane * k, hi), p1 = min(p0 + k, hi);
+    A = B = SumStep{0u, 0u};
+    for (uint64_t p = p0; p < p1; ++p) {
+        const float t = __ldcg(x + p);
+        uint32_t fl;
+        bool special;
+        SumStep st = sum_term(t, ua, fl, special);
+        if (special) st.e = st.o = kSumSat;
+        A = sum_compose(A, st);
+        if (ub != ua) {
+            st = sum_term(t, ub, fl, special);
+            if (special) st.e = st.o = kSumSat;
+            B = sum_compose(B, st);
+        }
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        SumStep oa, ob;
+        oa.e = __shfl_down_sync(0xffffffffu, A.e, d);
+        oa.o = __shfl_down_sync(0xffffffffu, A.o, d);
+        ob.e = __shfl_down_sync(0xffffffffu, B.e, d);
+        ob.o = __shfl_down_sync(0xffffffffu, B.o, d);
+        if ((lane & (2u * d - 1u)) == 0u) {
+            A = sum_compose(A, oa);
+            B = sum_compose(B, ob);
+        }
+    }
+    if (ub == ua) B = A;
+}
+
+// a float's binade: unit exponent, m, and the m the binade ends at
+__device__ __forceinline__ void sum_split(float s, int32_t &eu, uint32_t &m, uint32_t &top, uint32_t &Es) {
+    const uint32_t sb = __float_as_uint(s);
+    Es = sb >> 23;
+    eu = Es ? (int32_t)Es - 150 : -149;
+    m = Es ? ((sb & 0x7fffffu) | 0x800000u) : sb;
+    top = Es ? 0x1000000u : 0x800000u;
+}
+
+__device__ __forceinline__ float sum_join(uint32_t Es, uint32_t m) {
+    return __uint_as_float((Es << 23) + m - (Es ? 0x800000u : 0u));
+}
+
+// s plus the terms x[lo, hi), one add after another; a whole warp, the same s
+// in every lane
+__device__ __forceinline__ float warp_serial_add(float s, const float *__restrict__ x, uint64_t lo, uint64_t hi) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float next = lo + lane < hi ? __ldcg(x + lo + lane) : 0.0f;
+    for (uint64_t p = lo; p < hi; p += 32) {
+        const float t = next;
+        next = p + 32 + lane < hi ? __ldcg(x + p + 32 + lane) : 0.0f;
+        // adding 0 past the end leaves s as it is
+#pragma unroll
+        for (int k = 0; k < 32; ++k) s = FADD(s, __shfl_sync(0xffffffffu, t, k));
+    }
+    return s;
+}
+
+// the walk over the slices (one warp; see the file header)
+__device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t L, uint64_t LW, uint32_t nw,
+                               const SumScr &scr, uint32_t G) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float s = 0.0f;
+    for (uint32_t base = 0; base < G; base += 32) {
+        const uint32_t cnt = min(32u, G - base);
+        SumRec r;
+        r.ua = r.ub = kAnyUnit;
+        r.a = r.b = SumStep{0u, 0u};
+        if (lane < cnt) {
+            const uint4 u0 = __ldcg(reinterpret_cast<const uint4 *>(scr.rec + base + lane));
+            const uint4 u1 = __ldcg(reinterpret_cast<const uint4 *>(scr.rec + base + lane) + 1);
+            r.ua = (int32_t)u0.x;
+            r.ub = (int32_t)u0.y;
+            r.a = SumStep{u0.z, u0.w};
+            r.b = SumStep{u1.x, u1.y};
+        }
+        for (uint32_t pos = 0; pos < cnt;) {
+            int32_t eu;
+            uint32_t m, top, Es;
+            sum_split(s, eu, m, top, Es);
+            if (Es >= 0xffu) return s;   // inf stays
+            SumStep inc{0u, 0u};
+            if (lane >= pos && r.ua != kAnyUnit)
+                inc = r.ua == eu ? r.a : (r.ub == eu ? r.b : SumStep{kSumSat, kSumSat});
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                SumStep o;
+                o.e = __shfl_up_sync(0xffffffffu, inc.e, d);
+                o.o = __shfl_up_sync(0xffffffffu, inc.o, d);
+                if ((int)lane >= d) inc = sum_compose(o, inc);
+            }
+            const uint32_t ma = sum_apply(m, inc);
+            const uint32_t fails = __ballot_sync(0xffffffffu, ma >= top);
+            const uint32_t f = fails ? min((uint32_t)__ffs(fails) - 1u, cnt) : cnt;
+            if (f > pos) s = sum_join(Es, __shfl_sync(0xffffffffu, ma, f - 1));
+            pos = f;
+            if (f == cnt) continue;
+            // slice base + f, one warp's part after another
+            const uint32_t b = base + f;
+            const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
+            const int32_t ua = __shfl_sync(0xffffffffu, r.ua, f), ub = __shfl_sync(0xffffffffu, r.ub, f);
+            const uint4 part = lane < nw ? __ldcg(scr.part + (size_t)b * 8 + lane) : make_uint4(0, 0, 0, 0);
+            for (uint32_t w = 0; w < nw; ++w) {
+                const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
+                if (p0 >= p1) break;
+                sum_split(s, eu, m, top, Es);
+                if (Es >= 0xffu) return s;
+                SumStep st;
+                st.e = __shfl_sync(0xffffffffu, ua == eu ? part.x : part.z, w);
+                st.o = __shfl_sync(0xffffffffu, ua == eu ? part.y : part.w, w);
+                const uint32_t mw = sum_apply(m, st);
+                if ((ua == eu || ub == eu) && mw < top) s = sum_join(Es, mw);
+                else s = warp_serial_add(s, x, p0, p1);
+            }
+            pos = f + 1;
+        }
+    }
+    return s;
+}
+
+// the serial sums of x0[0, n) and, when x1 is not null, of x1[0, n), by the
+// whole grid (at most 8 warps per block); every thread gets them.  false when
+// a barrier gave up.
+template <int NT>
+__device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0, const float *x1, uint64_t n,
+                                              LoopyCtl *ctl, uint32_t &gen, uint32_t *s_fail, double *red, float &sum0,
+                                              float &sum1) {
+    static_assert(NT <= 256, "eight warps' pairs per block");
+    constexpr uint32_t NW = NT / 32;
+    __shared__ uint4 s_part[2][NW];
+    const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    const uint64_t L = ((n + G - 1) / G + 3) & ~3ull, LW = (L + NW - 1) / NW;
+    const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
+    const int nsum = x1 ? 2 : 1;
+    double own[2] = {0.0, 0.0};
+    for (int j = 0; j < nsum; ++j) {
+        const float *x = j ? x1 : x0;
+        double v = 0.0;
+        for (uint64_t k = lo + tid; k < hi; k += NT) v += (double)__ldcg(x + k);
+        own[j] = broadcast_sum(block_sum<NT>(v, red));
+        if (tid == 0) SumScr(partials, G, j).slice[b] = own[j];
+    }
+    if (G > 1 && !grid_barrier(ctl, gen, s_fail)) return false;
+    const double wide = fmin(0.5, (double)n * 0x1p-24);
+    for (int j = 0; j < nsum; ++j) {
+        const SumScr scr(partials, G, j);
+        double v = 0.0;
+        for (uint32_t k = tid; k < b; k += NT) v += __ldcg(scr.slice + k);
+        const double P = broadcast_sum(block_sum<NT>(v, red));
+        const int32_t ua = sum_unit(P * (1.0 - wide)), ub = sum_unit((P + own[j]) * (1.0 + wide));
+        const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
+        SumStep A, B;
+        warp_sum_steps(j ? x1 : x0, p0, p1, ua, ub, A, B);
+        if (lane == 0) {
+            const uint4 r = make_uint4(A.e, A.o, B.e, B.o);
+            s_part[j][w] = r;
+            scr.part[(size_t)b * 8 + w] = r;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            SumRec r;
+            r.a = r.b = SumStep{0u, 0u};
+            for (uint32_t k = 0; k < NW; ++k) {
+                r.a = sum_compose(r.a, SumStep{s_part[j][k].x, s_part[j][k].y});
+                r.b = sum_compose(r.b, SumStep{s_part[j][k].z, s_part[j][k].w});
+            }
+            r.ua = lo < hi ? ua : kAnyUnit;
+            r.ub = ub;
+            r.pad[0] = r.pad[1] = 0;
+            scr.rec[b] = r;
+        }
+    }
+    if (G > 1) {
+        if (!grid_barrier(ctl, gen, s_fail)) return false;
+    } else {
+        __syncthreads();
+    }
+    if (b == 0 && w < (uint32_t)nsum) {
+        const float s = warp_sum_walk(w ? x1 : x0, n, L, LW, NW, SumScr(partials, G, (int)w), G);
+        if (lane == 0) {
+            if (w) ctl->fb_p = s;
+            else ctl->fb_s = s;
+        }
+    }
+    if (G > 1) {
+        if (!grid_barrier(ctl, gen, s_fail)) return false;
+    } else {
+        __syncthreads();
+    }
+    sum0 = *(volatile float *)&ctl->fb_s;
+    sum1 = x1 ? *(volatile float *)&ctl->fb_p : 0.0f;
+    return true;
+}
+
+// one serial-mode check of a one-launch loop, undecided by the bounds: the
+// serial sum of the check's terms and, where the previous delta is not exact
+// yet, of its terms decide.  Every block of the grid calls it with the same x.
+template <int NT>
+__device__ __forceinline__ bool grid_serial_form(SerialCheck &x, const LoopyCtl &sc, LoopyCtl *ctl, double *partials,
+                                                 const float *absdiff, uint32_t &gen, uint32_t *s_fail, double *red) {
+    const float *xs = absdiff + (size_t)x.cb * sc.ad_stride;
+    const float *xp = x.p_exact ? nullptr : absdiff + (size_t)sc.prev_buf * sc.ad_stride;
+    float s, p;
+    if (!grid_serial_sums<NT>(partials, xs, xp, sc.n_terms, ctl, gen, s_fail, red, s, p)) return false;
+    x.s = s;
+    x.lo = x.hi = (double)s;
+    x.s_exact = true;
+    ++x.sums;
+    if (xp) {
+        x.plo = x.phi = (double)p;
+        x.p_exact = x.p_new = true;
+        ++x.sums;
+    }
+    x.d = serial_decide(x.lo, x.hi, true, x.plo, x.phi, true, sc.tol);
+    return true;
+}
+
+// the returned delta and previous delta of a finished one-launch run, where
+// the loop decided without forming them
+template <int NT>
+__device__ __forceinline__ bool grid_serial_final(LoopyCtl &sc, LoopyCtl *ctl, double *partials, const float *absdiff,
+                                                  uint32_t &gen, uint32_t *s_fail, double *red) {
+    const bool cur = !sc.delta_exact, prev = !sc.prev_exact;
+    if (!cur && !prev) return true;
+    const float *xc = absdiff + (size_t)sc.cur_buf * sc.ad_stride, *xp = absdiff + (size_t)sc.prev_buf * sc.ad_stride;
+    float s, p;
+    if (!grid_serial_sums<NT>(partials, cur ? xc : xp, cur && prev ? xp : nullptr, sc.n_terms, ctl, gen, s_fail, red,
+                              s, p))
+        return false;
+    __syncthreads();   // every thread has read sc
+    if (threadIdx.x == 0) {
+        if (cur) sc.delta_f = s;
+        if (prev) sc.prev_f = cur ? p : s;
+        sc.delta_exact = sc.prev_exact = 1;
+    }
+    __syncthreads();
+    return true;
+}
