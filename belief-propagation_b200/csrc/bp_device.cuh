@@ -2,8 +2,9 @@
 //
 // Arithmetic parity: every product, sum and quotient that the reference
 // computes in fp32 is written with the round-to-nearest intrinsics
-// (__fmul_rn / __fadd_rn / __fsub_rn / __fdiv_rn), which nvcc never fuses
-// into FMA, in the reference's order.  Results are then bit-identical to the
+// (__fmul_rn / __fadd_rn / __fsub_rn), which nvcc never fuses into FMA, and
+// quotients are rounded as __fdiv_rn rounds them (divide_by_sum), in the
+// reference's order.  Results are then bit-identical to the
 // reference compiled with gcc on x86-64 (SSE, no contraction).
 #pragma once
 
@@ -17,7 +18,6 @@ namespace bpx {
 #define FMUL __fmul_rn
 #define FADD __fadd_rn
 #define FSUB __fsub_rn
-#define FDIV __fdiv_rn
 
 // ---- vector loads / stores of N consecutive floats ------------------------
 // N*4 bytes at an address that is a multiple of N*4 bytes (every array here is
@@ -193,6 +193,69 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return true;
 }
 
+// ---- quotients by one divisor ----------------------------------------------
+// m[i] / sum for i < n, each rounded as __fdiv_rn rounds it; sum <= 0 counts as
+// 1 (graph.c:901-904, :1015-1018) and slots at or beyond n come out 0.
+//
+// The update multiplies each belief into itself every iteration, so beliefs
+// and messages head to 0 through the subnormals (and evidence starts there),
+// where an fp32 divide leaves its fast path: 55 cycles a quotient become 350
+// for a zero and 485 for a subnormal numerator, and every lane of the warp
+// waits.  In f64 nothing is subnormal, and the quotients share one
+// reciprocal: an approximate one (rcp.approx.ftz.f64) after two Newton steps,
+// then per quotient q = a r and one residual correction q + (a - q b) r
+// (Markstein, IBM J. Res. Dev. 34(1), 1990).  That f64 quotient is within an
+// ulp of a / b, exact where a / b is a double, and two fp32 operands put a / b
+// either on a rounding boundary of fp32 (normal or subnormal) or at least
+// 2^-49 of itself away from it, so rounding it to fp32 gives __fdiv_rn's bits
+// (20 G operand pairs, subnormals and ties among them: no difference).
+// A warp's 2, 4 and 8 quotients, a full GPU (per SM): 5.1, 9.9, 19.4 ns with
+// fp32 divides of normal operands, 9.3, 13.1, 22.2 with a zero and 18.7, 22.2,
+// 29.9 with a subnormal among them; 6.1, 8.9, 14.8 ns here, whatever they are.
+// Messages of two states keep the fp32 divide (divide_message): their sums of
+// products are rarely 0 or subnormal, and on the 16.8M-node graph the f64
+// form of them cost 2 % of an iteration.
+template <int MS, bool UNI>
+__device__ __forceinline__ void divide_by_sum(float *m, float sum, int n) {
+    if (sum > 0.0f && sum <= 3.402823466e38f) {
+        const double b = (double)sum;
+        double r;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+        r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+        r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+#pragma unroll
+        for (int i = 0; i < MS; ++i) {
+            const double a = (double)m[i];
+            double q = __dmul_rn(a, r);
+            q = __fma_rn(__fma_rn(-q, b, a), r, q);
+            // a zero keeps its sign (sum is positive)
+            m[i] = __uint_as_float(__float_as_uint(__double2float_rn(q)) | (__float_as_uint(m[i]) & 0x80000000u));
+        }
+    } else if (!(sum <= 0.0f)) {
+        // inf: finite / inf = 0, inf / inf = NaN; NaN: NaN
+        const float f = sum == sum ? 0.0f : sum;
+#pragma unroll
+        for (int i = 0; i < MS; ++i) m[i] = FMUL(m[i], f);
+    }
+    if (!UNI) {
+#pragma unroll
+        for (int i = 0; i < MS; ++i)
+            if (i >= n) m[i] = 0.0f;
+    }
+}
+
+// a message's quotients
+template <int MS, bool UNI>
+__device__ __forceinline__ void divide_message(float *m, float sum, int n) {
+    if constexpr (MS <= 2) {
+        if (sum <= 0.0f) sum = 1.0f;
+#pragma unroll
+        for (int i = 0; i < MS; ++i) m[i] = (UNI || i < n) ? __fdiv_rn(m[i], sum) : 0.0f;
+    } else {
+        divide_by_sum<MS, UNI>(m, sum, n);
+    }
+}
+
 // ---- the send step ---------------------------------------------------------
 // m[i] = sum_j J[i][j] * buf[j] for i < x, j < y (partial sums from 0 in j
 // order), normalised by their sum over i (sum <= 0 replaced by 1):
@@ -214,9 +277,7 @@ __device__ __forceinline__ void send_msg_regs(const float *j, const float *buf, 
         }
         m[i] = partial;
     }
-    if (sum <= 0.0f) sum = 1.0f;
-#pragma unroll
-    for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
+    divide_message<MS, UNI>(m, sum, x);
 }
 
 // the same arithmetic on a table in shared memory, row after row
@@ -236,9 +297,7 @@ __device__ __forceinline__ void send_msg_rows(const float *J, const float *buf, 
         }
         m[i] = partial;
     }
-    if (sum <= 0.0f) sum = 1.0f;
-#pragma unroll
-    for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
+    divide_message<MS, UNI>(m, sum, x);
 }
 
 template <int MS, bool UNI>
@@ -274,9 +333,7 @@ __device__ __forceinline__ void send_msg(const float *__restrict__ J, const floa
             m[i] = partial;
         }
     }
-    if (sum <= 0.0f) sum = 1.0f;
-#pragma unroll
-    for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
+    divide_message<MS, UNI>(m, sum, x);
 }
 
 // the same send step on a dense x-by-y table (row stride y; for uniform
@@ -303,9 +360,7 @@ __device__ __forceinline__ void send_msg_dense(const float *__restrict__ J, cons
         }
         m[i] = partial;
     }
-    if (sum <= 0.0f) sum = 1.0f;
-#pragma unroll
-    for (int i = 0; i < MS; ++i) m[i] = (UNI || i < x) ? FDIV(m[i], sum) : 0.0f;
+    divide_message<MS, UNI>(m, sum, x);
 }
 
 // buf[i] *= m[i] for i < s unless m[i] is NaN: graph.c:450-459 (combine_message)
@@ -323,9 +378,7 @@ __device__ __forceinline__ void normalise(float *b, int s) {
 #pragma unroll
     for (int i = 0; i < MS; ++i)
         if (UNI || i < s) sum = FADD(sum, b[i]);
-    if (sum <= 0.0f) sum = 1.0f;
-#pragma unroll
-    for (int i = 0; i < MS; ++i) b[i] = (UNI || i < s) ? FDIV(b[i], sum) : 0.0f;
+    divide_by_sum<MS, UNI>(b, sum, s);
 }
 
 // ---- block reductions ------------------------------------------------------

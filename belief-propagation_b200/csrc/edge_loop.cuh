@@ -59,13 +59,16 @@ __device__ __forceinline__ bool edge_normalise_once(float *b, int s) {
     for (int i = 0; i < MS; ++i)
         if (i < s) sum = FADD(sum, b[i]);
     if (!(sum > 0.0f)) return false;
+    float nb[MS];
+#pragma unroll
+    for (int i = 0; i < MS; ++i) nb[i] = b[i];
+    divide_by_sum<MS, true>(nb, sum, s);
     bool changed = false;
 #pragma unroll
     for (int i = 0; i < MS; ++i)
         if (i < s) {
-            const float nb = FDIV(b[i], sum);
-            changed |= __float_as_uint(nb) != __float_as_uint(b[i]);
-            b[i] = nb;
+            changed |= __float_as_uint(nb[i]) != __float_as_uint(b[i]);
+            b[i] = nb[i];
         }
     return changed;
 }
