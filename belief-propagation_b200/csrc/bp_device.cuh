@@ -178,6 +178,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
+// release / acquire at GPU scope (a flag another block polls)
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void st_relaxed(uint64_t *p, uint64_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint64_t ld_relaxed(const uint64_t *p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -402,6 +413,16 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
     }
     __syncthreads();
     return t;  // valid in thread 0
+}
+
+// the block's total of the warps' sums red[0, NW) (as warp_sum left them), with
+// block_sum's order of additions -- its second shuffle tree over NW values and
+// zeros -- in any thread that has seen them
+template <int NW>
+__device__ __forceinline__ double warps_total(const double *red) {
+    static_assert(NW == 4 || NW == 8, "the trees written out");
+    if constexpr (NW == 4) return (red[0] + red[2]) + (red[1] + red[3]);
+    else return ((red[0] + red[4]) + (red[2] + red[6])) + ((red[1] + red[5]) + (red[3] + red[7]));
 }
 
 // programmatic dependent launch: a kernel launched with the programmatic

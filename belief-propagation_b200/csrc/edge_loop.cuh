@@ -29,8 +29,8 @@
 // 50,001 nodes x 3 states.  The orbit is now followed only until its period
 // is known (Brent's method), and the rest taken modulo the period.
 // 50,001 nodes, 200,003 edges, 3 states, serial delta, 50 iterations:
-// 105.9 -> 4.0 ms per solve (0.9 ms of it the iterations; the rest forms the
-// serial sum in the 38 checks that need it, serial_grid.cuh); f64 delta 0.71 ms.
+// 105.4 -> 3.8 ms per solve (0.9 ms of it the iterations; the rest forms the
+// serial sum in the 38 checks that need it, serial_grid.cuh); f64 delta 0.75 ms.
 #pragma once
 
 struct EdgeArgs {
@@ -223,7 +223,10 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
         const double tot = block_sum<NT>(sum, red);
         if (SER && want) {
             SerialCheck x = serial_check(&s_ctl, broadcast_sum(tot));
-            if (x.d < 0 && !grid_serial_form<NT>(x, s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red)) break;
+            if (x.d < 0 && !grid_serial_form<NT>(x, a.absdiff + (size_t)x.cb * s_ctl.ad_stride,
+                                                 a.absdiff + (size_t)s_ctl.prev_buf * s_ctl.ad_stride, s_ctl.n_terms,
+                                                 s_ctl.tol, ctl, a.partials, gen, &s_fail, red))
+                break;
             __syncthreads();   // every thread has read s_ctl
             if (threadIdx.x == 0) serial_commit(&s_ctl, x);
         } else if (threadIdx.x == 0) {

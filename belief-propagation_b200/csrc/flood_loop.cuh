@@ -29,9 +29,11 @@
 // summed in k_flood's order, so results and the f64 delta equal the
 // one-launch-per-iteration loop's bit for bit.
 //
-// 10,000 nodes, 40,000 edges, 2 states, per iteration: 8.2 -> 7.0 us with the
-// f64 delta, 11.7 -> 8.2 us with the serial one; 61 nodes of 2-4 states (one
-// tile): 5.7 -> 4.3 us.
+// What bounds it: the instruction stream of the few warps of a tile -- 1,400
+// instructions an iteration at 8 to 10 cycles each -- more than the memory:
+// 10,000 nodes, 40,000 edges, 2 states take 6.0 us an iteration with the f64
+// delta (8.2 before) and 7.5 with the serial one (11.7), 61 nodes of 2-4
+// states (one tile) 2.3 and 3.3 (5.7 and 6.8).
 #pragma once
 
 // blocks that meet by polling each other's flags: every block reads every
@@ -61,33 +63,82 @@ struct LoopArgs {
 // every block's flag at `tag` or above (this block's is set here); the wait is
 // bounded as grid_barrier's, and the same test hook holds a block back: it
 // never sets its flag and does not wait at its first barrier
-__device__ __forceinline__ bool flag_barrier(LoopyCtl *c, uint64_t *flags, uint64_t tag, bool first, uint32_t *s_fail) {
+__device__ __forceinline__ bool flag_barrier(LoopyCtl *c, uint64_t *flags, uint64_t tag, bool skip, bool first,
+                                             uint32_t wait_ms, uint32_t *s_fail) {
     __syncthreads();
-    const bool skip = c->bar_skip == blockIdx.x + 1u;
     if (threadIdx.x == 0 && !skip) {
-        __threadfence();
-        *(volatile uint64_t *)(flags + blockIdx.x) = tag;
+        fence_acq_rel();
+        st_relaxed(flags + blockIdx.x, tag);
     }
     if (!(skip && first)) {
-        const uint64_t limit = c->wait_ms ? (uint64_t)c->wait_ms * 1000000ull : kBarrierWaitNs;
+#pragma unroll 1
         for (uint32_t k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
             uint64_t t0 = 0;
-            for (uint32_t spin = 0; *(volatile uint64_t *)(flags + k) < tag; ++spin) {
+#pragma unroll 1
+            for (uint32_t spin = 0; ld_relaxed(flags + k) < tag; ++spin) {
                 if ((spin & 255u) != 255u) continue;
                 if (*(volatile uint32_t *)s_fail) break;
                 const uint64_t t = global_ns();
                 if (t0 == 0) t0 = t;
-                if (t - t0 > limit) {
+                if (t - t0 > (wait_ms ? (uint64_t)wait_ms * 1000000ull : kBarrierWaitNs)) {
                     *(volatile uint32_t *)s_fail = 1;
                     atomicExch(&c->bar_fail, 1u);
                     break;
                 }
             }
         }
+        fence_acq_rel();
     }
-    __threadfence();
     __syncthreads();
     return *(volatile uint32_t *)s_fail == 0;
+}
+
+// The steady loop is kept small -- runtime loops not unrolled, everything rare
+// out of line -- since a handful of warps per SM run straight through it every
+// iteration and wait for instructions otherwise.
+
+// |diff| terms of the tile's message buffers `from` and `to`, at their edge ids
+template <int MS, bool UNI>
+__device__ __noinline__ void loop_write_terms(float *dst, const float *from, const float *to, const uint32_t *srcs,
+                                              const uint32_t *pos_edge, uint32_t ne) {
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x; i < ne; i += flood_nt<MS>()) {
+        const int x = UNI ? MS : (int)(srcs[i] >> 24 & 15u);
+        float ad[MS];
+#pragma unroll
+        for (int k = 0; k < MS; ++k) {
+            float d = 0.0f;
+            if (UNI || k < x) {
+                d = FSUB(from[(size_t)i * MS + k], to[(size_t)i * MS + k]);
+                if (d != d) d = 0.0f;
+                d = fabsf(d);
+            }
+            ad[k] = d;
+        }
+        stv<MS>(dst + (size_t)pos_edge[i] * MS, ad);
+    }
+}
+
+// flood_tile on global memory, for a tile too large for its block
+template <int MS, bool UNI>
+__device__ __noinline__ double loop_flood_tile(const FloodArgs &a, bool want, float *absd, uint32_t t, uint32_t mp0,
+                                               uint32_t qp0, float *sm) {
+    const int mp = (int)((mp0 + t) & 1u), qp = (int)((qp0 + t) & 1u);
+    double dsum = 0.0;
+    flood_tile<MS, UNI, 1>(a, blockIdx.x, want, absd, mp ? a.msg1 : a.msg0, mp ? a.msg0 : a.msg1, qp ? a.q1 : a.q0,
+                           qp ? a.q0 : a.q1, 0, sm, dsum);
+    return dsum;
+}
+
+// acc *= the messages of positions [r0, r1) in order (combine)
+template <int MS, bool UNI>
+__device__ __forceinline__ void node_product(const float *m, uint32_t r0, uint32_t r1, int S, float *acc) {
+#pragma unroll 1
+    for (uint32_t p = r0; p < r1; ++p) {
+        float mm[MS];
+        ldv<MS>(m + (size_t)p * MS, mm);
+        combine<MS, UNI>(acc, mm, S);
+    }
 }
 
 template <int MS, bool UNI, bool SER, bool WIDE>
@@ -98,7 +149,8 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
     constexpr uint32_t NB = SER ? 3 : 2;   // message buffers
     constexpr uint32_t TS = loop_table_stride<MS>();
     extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ double red[NT / 32];
+    constexpr int NW = NT / 32;
+    __shared__ double red[NW], red_t[NW], red_b[NW];
     __shared__ LoopyCtl s_ctl;
     __shared__ uint32_t s_fail;
 
@@ -146,8 +198,13 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
     if (resident) {
         if (has) ldv<MS>(a.belief + (size_t)v * MS, b);
         const float *m0 = mp0 ? a.msg1 : a.msg0;
+#pragma unroll 1
         for (uint32_t i = tid; i < ne; i += NT) {
-            srcs[i] = a.in_src[e0 + i];
+            // the state counts beside the source (node ids of a graph this
+            // small are below 2^24)
+            uint32_t sv = a.in_src[e0 + i];
+            if (!UNI) sv |= (uint32_t)a.pos_dims[e0 + i] << 24;
+            srcs[i] = sv;
             float m[MS];
             ldv<MS>(m0 + (size_t)(e0 + i) * MS, m);
             stv<MS>(ms + (size_t)i * MS, m);
@@ -174,26 +231,24 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
     }
     __syncthreads();
 
-    // |diff| terms of messages buffers `from` and `to` at their edge ids
     auto write_terms = [&](float *dst, const float *from, const float *to) {
-        for (uint32_t i = tid; i < ne; i += NT) {
-            int x = MS;
-            if (!UNI) x = a.pos_dims[e0 + i] & 15;
-            float ad[MS];
-#pragma unroll
-            for (int k = 0; k < MS; ++k) {
-                float d = 0.0f;
-                if (UNI || k < x) {
-                    d = FSUB(from[(size_t)i * MS + k], to[(size_t)i * MS + k]);
-                    if (d != d) d = 0.0f;
-                    d = fabsf(d);
-                }
-                ad[k] = d;
-            }
-            stv<MS>(dst + (size_t)a.pos_edge[e0 + i] * MS, ad);
-        }
+        loop_write_terms<MS, UNI>(dst, from, to, srcs, a.pos_edge + e0, ne);
     };
 
+    // the decision's running state, the same in every thread of every block:
+    // each thread takes each decision itself, and the control block is
+    // written once at the end
+    const uint32_t max_it = s_ctl.max_it, wait_ms = s_ctl.wait_ms;
+    const float tol = s_ctl.tol;
+    const bool skip = s_ctl.bar_skip == blockIdx.x + 1u;
+    // f64 sum, interval of the serial sum, whether it is the sum itself and
+    // its check: of the last check (d) and of the one before (p), which stays
+    // where it is at the last allowed iteration, as the reference's does
+    double d_d = 0.0, dlo = 0.0, dhi = 0.0, p_d = s_ctl.prev_d, plo = s_ctl.plo, phi = s_ctl.phi;
+    float d_f = 0.0f, p_f = s_ctl.prev_f;
+    bool d_exact = true, p_exact = true, stop = false;
+    uint32_t d_buf = 0, p_buf = 0, sums = 0, it = 0;
+    double tot = 0.0;   // a lone tile's sum needs no exchange
     uint32_t gen = 0;
     uint32_t cur = 0;   // buffer of the latest messages
     bool ok = true;
@@ -204,7 +259,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
         // the first round's gathers, before the last iteration's decision
         float q[FU][MS];
         auto gather = [&](uint32_t i, float *o) {
-            const uint32_t s = srcs[i];
+            const uint32_t s = UNI ? srcs[i] : srcs[i] & 0xffffffu;
             if (solo) {
                 ldv<MS>(qs + (size_t)(qp * NT + s) * MS, o);
             } else {
@@ -235,45 +290,80 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
         if (t) {
             // the decision of iteration t - 1 (the reference's stopping rule)
             const bool want = (ce <= 1) || (t % ce == 0);
-            const double *part = a.partials + (size_t)((t - 1) & 1u) * G;
-            double acc = 0.0;
-            for (uint32_t k = tid; k < G; k += NT) acc += __ldcg(part + k);
-            const double tot = block_sum<NT>(acc, red);
-            if (SER && want) {
-                SerialCheck x = serial_check(&s_ctl, broadcast_sum(tot));
-                if (x.d < 0) {
-                    if (lazy) {
-                        const uint32_t p1 = (cur + 2u) % 3u, p2 = (cur + 1u) % 3u;
-                        write_terms(a.absdiff + (size_t)x.cb * s_ctl.ad_stride, ms + (size_t)p1 * ne * MS,
-                                    ms + (size_t)cur * ne * MS);
-                        if (!x.p_exact)
-                            write_terms(a.absdiff + (size_t)s_ctl.prev_buf * s_ctl.ad_stride,
-                                        ms + (size_t)p2 * ne * MS, ms + (size_t)p1 * ne * MS);
-                    }
-                    if (solo) __syncthreads();
-                    else if (lazy || ce <= 1) ok = grid_barrier(ctl, gen, &s_fail);
-                    ok = ok && grid_serial_form<NT>(x, s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red);
-                    if (!ok) break;
-                }
-                __syncthreads();   // every thread has read s_ctl
-                if (tid == 0) serial_commit(&s_ctl, x);
-            } else if (tid == 0) {
-                finalize(&s_ctl, want, (float)tot, tot);
+            if (!solo && want) {
+                const double *part = a.partials + (size_t)((t - 1) & 1u) * G;
+                double acc = 0.0;
+#pragma unroll 1
+                for (uint32_t k = tid; k < G; k += NT) acc += __ldcg(part + k);
+                acc = warp_sum(acc);
+                if ((tid & 31u) == 0) red_t[tid >> 5] = acc;
+                __syncthreads();
+                tot = warps_total<NW>(red_t);
             }
-            __syncthreads();
-            if (s_ctl.done) break;
+            it = t;
+            if (want) {
+                if (t > ce) {
+                    p_d = d_d;
+                    p_f = d_f;
+                    plo = dlo;
+                    phi = dhi;
+                    p_exact = d_exact;
+                    p_buf = d_buf;
+                }
+                d_d = tot;
+                d_f = (float)tot;
+                if constexpr (SER) {
+                    SerialCheck x;
+                    x.T = tot;
+                    x.plo = plo;
+                    x.phi = phi;
+                    x.p_exact = p_exact;
+                    x.p_ref = x.s_exact = x.s_ref = x.p_new = false;
+                    x.sums = x.refines = 0;
+                    x.cb = d_buf = check_index(t - 1, ce) % 3u;
+                    x.s = d_f;
+                    serial_interval(tot, s_ctl.n_terms, x.lo, x.hi);
+                    x.d = serial_decide(x.lo, x.hi, false, plo, phi, p_exact, tol);
+                    if (x.d < 0) {
+                        float *const tc = a.absdiff + (size_t)d_buf * s_ctl.ad_stride;
+                        float *const tp = a.absdiff + (size_t)p_buf * s_ctl.ad_stride;
+                        if (lazy) {
+                            const uint32_t p1 = (cur + 2u) % 3u, p2 = (cur + 1u) % 3u;
+                            write_terms(tc, ms + (size_t)p1 * ne * MS, ms + (size_t)cur * ne * MS);
+                            if (!p_exact) write_terms(tp, ms + (size_t)p2 * ne * MS, ms + (size_t)p1 * ne * MS);
+                        }
+                        if (solo) __syncthreads();
+                        else if (ce <= 1) ok = grid_barrier(ctl, gen, &s_fail);
+                        ok = ok && grid_serial_form<NT>(x, tc, tp, s_ctl.n_terms, tol, ctl, a.partials, gen, &s_fail, red_b);
+                        if (!ok) break;
+                        if (!p_exact) p_f = (float)x.plo;
+                        plo = x.plo;
+                        phi = x.phi;
+                        p_exact = x.p_exact;
+                        sums += x.sums;
+                    }
+                    d_f = x.s;
+                    dlo = x.lo;
+                    dhi = x.hi;
+                    d_exact = x.s_exact;
+                    stop = x.d == 1;
+                } else {
+                    stop = tot < (double)tol || fabs(tot - p_d) < (double)tol;
+                }
+                if (stop) break;
+            }
+            if ((ce <= 1 || want) && t >= max_it) break;
         }
         const bool want = (ce <= 1) || ((t + 1) % ce == 0);
-        float *absd = SER && !lazy ? check_buffer(&s_ctl, a.absdiff, t, want) : nullptr;
+        float *absd = SER && !lazy && want ? a.absdiff + (size_t)(check_index(t, ce) % 3u) * s_ctl.ad_stride : nullptr;
         double dsum = 0.0;
         if (!resident) {
-            const int mp = (int)((mp0 + t) & 1u);
-            flood_tile<MS, UNI, FU>(a, blockIdx.x, want, absd, mp ? a.msg1 : a.msg0, mp ? a.msg0 : a.msg1, q_in, q_out,
-                                    0, reinterpret_cast<float *>(dyn), dsum);
+            dsum = loop_flood_tile<MS, UNI>(a, want, absd, t, mp0, qp0, reinterpret_cast<float *>(dyn));
         } else {
             const float *mo = ms + (size_t)cur * ne * MS;
             cur = cur + 1u == NB ? 0u : cur + 1u;
             float *mn = ms + (size_t)cur * ne * MS;
+#pragma unroll 1
             for (uint32_t base = tid; base < ne; base += NT * FU) {
                 if (base != tid) {
 #pragma unroll
@@ -284,12 +374,8 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                 for (int u = 0; u < FU; ++u) {
                     const uint32_t i = base + u * NT;
                     if (i >= ne) break;
-                    int x = MS, y = MS;
-                    if (!UNI) {
-                        const uint8_t d = a.pos_dims[e0 + i];
-                        x = d & 15;
-                        y = d >> 4;
-                    }
+                    const uint32_t sv = UNI ? 0u : srcs[i];
+                    const int x = UNI ? MS : (int)(sv >> 24 & 15u), y = UNI ? MS : (int)(sv >> 28);
                     float m[MS], o[MS];
                     ldv<MS>(mo + (size_t)i * MS, o);
                     if (tables) {
@@ -321,18 +407,19 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                     }
                 }
             }
-            __syncthreads();
+        }
+        dsum = warp_sum(dsum);
+        if ((tid & 31u) == 0) red[tid >> 5] = dsum;
+        __syncthreads();
+        if (resident) {
             // the node: marginalise, then the next send buffer (flood_tile's
             // phase 2)
+            const float *mn = ms + (size_t)cur * ne * MS;
             if (has) {
                 float prod[MS];
 #pragma unroll
                 for (int i = 0; i < MS; ++i) prod[i] = 1.0f;
-                for (uint32_t p = r0; p < r1; ++p) {
-                    float mm[MS];
-                    ldv<MS>(mn + (size_t)p * MS, mm);
-                    combine<MS, UNI>(prod, mm, S);
-                }
+                node_product<MS, UNI>(mn, r0, r1, S, prod);
                 if (r1 > r0) {
 #pragma unroll
                     for (int i = 0; i < MS; ++i)
@@ -342,26 +429,54 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                 float qo[MS];
 #pragma unroll
                 for (int i = 0; i < MS; ++i) qo[i] = b[i];
-                for (uint32_t p = r0; p < r1; ++p) {
-                    float mm[MS];
-                    ldv<MS>(mn + (size_t)p * MS, mm);
-                    combine<MS, UNI>(qo, mm, S);
-                }
+                node_product<MS, UNI>(mn, r0, r1, S, qo);
                 if (solo) stv<MS>(qs + (size_t)((qp ^ 1u) * NT + tid) * MS, qo);
                 else stv<MS>(q_out + (size_t)v * MS, qo);
             }
         }
-        const double part = block_sum<NT>(dsum, red);
-        if (tid == 0) a.partials[(size_t)(t & 1u) * G + blockIdx.x] = part;
+        if (solo) tot = warps_total<NW>(red);
+        else if (tid == 0) a.partials[(size_t)(t & 1u) * G + blockIdx.x] = warps_total<NW>(red);
         if (solo) __syncthreads();
-        else if (G <= kFlagBlocks) ok = flag_barrier(ctl, la.flags, la.run_tag + t + 1u, t == 0, &s_fail);
+        else if (G <= kFlagBlocks) ok = flag_barrier(ctl, la.flags, la.run_tag + t + 1u, skip, t == 0, wait_ms, &s_fail);
         else ok = grid_barrier(ctl, gen, &s_fail);
         if (!ok) break;
     }
 
+    // the reference's loop variables at exit (graph.c:1313-1318; _acc:
+    // :1410-1414), which finalize_with keeps iteration by iteration
+    if (tid == 0 && ok) {
+        s_ctl.it = it;
+        s_ctl.done = stop ? 1u : 2u;
+        if (ce <= 1) {
+            s_ctl.ret = s_ctl.final_i = stop ? it - 1u : max_it;
+        } else {
+            s_ctl.num_iter = stop ? it - ce : it;
+            s_ctl.ret = s_ctl.num_iter;
+            s_ctl.final_i = stop ? it - ce : it;
+            if (!stop) {   // the _acc loop keeps the last check as the previous one too
+                p_d = d_d;
+                p_f = d_f;
+                plo = dlo;
+                phi = dhi;
+                p_buf = d_buf;
+            }
+        }
+        s_ctl.delta_f = d_f;
+        s_ctl.delta_d = d_d;
+        s_ctl.prev_f = p_f;
+        s_ctl.prev_d = p_d;
+        if (SER) {
+            s_ctl.delta_exact = d_exact;
+            s_ctl.prev_exact = ce > 1 && !stop ? d_exact : p_exact;
+            s_ctl.cur_buf = d_buf;
+            s_ctl.prev_buf = p_buf;
+            s_ctl.serial_sums = sums;
+        }
+    }
+    __syncthreads();
     if (ok && SER) {
         // the returned deltas where the loop decided without them
-        if (lazy && s_ctl.done) {
+        if (lazy) {
             const uint32_t p1 = (cur + 2u) % 3u, p2 = (cur + 1u) % 3u;
             if (!s_ctl.delta_exact)
                 write_terms(a.absdiff + (size_t)s_ctl.cur_buf * s_ctl.ad_stride, ms + (size_t)p1 * ne * MS,
@@ -373,13 +488,13 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
         if (!s_ctl.delta_exact || !s_ctl.prev_exact) {
             if (solo) __syncthreads();
             else ok = grid_barrier(ctl, gen, &s_fail);
-            ok = ok && grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red);
+            ok = ok && grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red_b);
         }
     }
     if (ok && resident) {
-        const uint32_t it = s_ctl.it;
         float *ml = ((mp0 + it) & 1u) ? a.msg1 : a.msg0, *mo = ((mp0 + it) & 1u) ? a.msg0 : a.msg1;
         const uint32_t old = cur ? cur - 1u : NB - 1u;
+#pragma unroll 1
         for (uint32_t i = tid; i < ne; i += NT) {
             float m[MS];
             ldv<MS>(ms + ((size_t)cur * ne + i) * MS, m);

@@ -11,20 +11,21 @@
 // One warp then walks the slices in order: the walk knows the exact running
 // sum, so a slice's pair counts only when it was made for the binade the sum
 // is in and the sum stays below the binade's top; otherwise that slice is
-// walked warp part by warp part, and a part that crosses (or was guessed
-// wrong) is added term by term.  The guesses decide the speed, never the
+// walked warp part by warp part, a part that crosses lane run by lane run, and
+// the run that crosses (or a part guessed wrong) is added term by term.  The guesses decide the speed, never the
 // value: the result is the one-by-one sum bit for bit.
 //
-// Before, one block of the grid formed the sum while the others waited: 600k
-// terms 1.1 ms, now 75 us (592 blocks of 256 threads; bounded by three grid
-// barriers and the walk over a dozen crossings).  The interval narrowed from
-// the terms' own errors, which decided most checks before, took 29 us of
-// grid time each on 80k terms and still left the sum to be formed where the
-// delta creeps; the sum itself decides in one go.
+// Before, one block of the grid formed the sum while the others waited (600k
+// terms 1.1 ms, 80k terms after an interval narrowed from the terms' errors
+// had not decided).  Now 80k terms (79 blocks) take 50 us and 600k terms (782
+// blocks) 70 us, two sums at once the same: half of it the walk, a few
+// thousand cycles for each of the half dozen slices that cross, the rest four
+// grid barriers.
 #pragma once
 
-// doubles of scratch per block behind the grid's 2 x G delta partials
-constexpr uint32_t kSumScratch = 42;
+// doubles of scratch per block behind the grid's 2 x G delta partials: two
+// sums' slice sum, record, warps' pairs and lanes' pairs
+constexpr uint32_t kSumScratch = 2 * (1 + 4 + 16 + 512);
 constexpr int32_t kAnyUnit = 0x7fffffff;   // an empty slice: nothing to add in any binade
 
 struct SumRec {
@@ -39,11 +40,13 @@ struct SumScr {
     double *slice;   // [G]
     SumRec *rec;     // [G]
     uint4 *part;     // [G][8] the warps' pairs: a.e, a.o, b.e, b.o
+    uint4 *lane;     // [G][8][32] the lanes' pairs
     __device__ SumScr(double *partials, uint32_t G, int j) {
         double *base = partials + 2 * (size_t)G;
         slice = base + (size_t)j * G;
         rec = reinterpret_cast<SumRec *>(base + 2 * (size_t)G) + (size_t)j * G;
         part = reinterpret_cast<uint4 *>(base + 10 * (size_t)G) + (size_t)j * G * 8;
+        lane = reinterpret_cast<uint4 *>(base + 42 * (size_t)G) + (size_t)j * G * 256;
     }
 };
 
@@ -53,27 +56,50 @@ __device__ __forceinline__ int32_t sum_unit(double s) {
     return min(ilogb(s), 127) - 23;
 }
 
+// sum_term's pair without its branches: term t added in the binade with unit
+// 2^eu; an inf saturates
+__device__ __forceinline__ SumStep sum_step(float t, int32_t eu) {
+    const uint32_t tb = __float_as_uint(t), Et = (tb >> 23) & 0xffu;
+    const uint32_t Mt = Et ? ((tb & 0x7fffffu) | 0x800000u) : (tb & 0x7fffffu);
+    const int32_t shift = (Et ? (int32_t)Et - 150 : -149) - eu;
+    const uint32_t sh = (uint32_t)min(max(-shift, 0), 31);
+    const uint32_t one = 1u << sh, half = one >> 1, rem = Mt & (one - 1u);
+    uint32_t fl = shift > 0 ? (shift >= 7 ? kSumSat : min(Mt << shift, kSumSat)) : Mt >> sh;
+    if (Mt == 0u) fl = 0u;
+    if (Et == 0xffu) fl = kSumSat;
+    const uint32_t tie = half != 0u && rem == half ? 1u : 0u, up = rem > half ? 1u : 0u;
+    SumStep st;
+    st.e = fl + (up | (tie & fl & 1u));
+    st.o = fl + (up | (tie & ~fl & 1u));
+    return st;
+}
+
 // terms x[lo, hi) in order, composed for unit exponents ua and ub; lane 0 of
-// the warp gets the pairs
+// the warp gets the pairs.  Each lane takes a run of them, four loads ahead,
+// and leaves its run's pairs in `lanes`.
 __device__ __forceinline__ void warp_sum_steps(const float *__restrict__ x, uint64_t lo, uint64_t hi, int32_t ua,
-                                               int32_t ub, SumStep &A, SumStep &B) {
+                                               int32_t ub, SumStep &A, SumStep &B, uint4 *lanes) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t k = (hi - lo + 31u) / 32u;
     const uint64_t p0 = min(lo + lane * k, hi), p1 = min(p0 + k, hi);
     A = B = SumStep{0u, 0u};
-    for (uint64_t p = p0; p < p1; ++p) {
-        const float t = __ldcg(x + p);
-        uint32_t fl;
-        bool special;
-        SumStep st = sum_term(t, ua, fl, special);
-        if (special) st.e = st.o = kSumSat;
-        A = sum_compose(A, st);
-        if (ub != ua) {
-            st = sum_term(t, ub, fl, special);
-            if (special) st.e = st.o = kSumSat;
-            B = sum_compose(B, st);
+    float t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = p0 + i < p1 ? __ldcg(x + p0 + i) : 0.0f;
+#pragma unroll 1
+    for (uint64_t p = p0; p < p1; p += 4) {
+        float n[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) n[i] = p + 4 + i < p1 ? __ldcg(x + p + 4 + i) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            A = sum_compose(A, sum_step(t[i], ua));   // a 0 past the end adds nothing
+            if (ub != ua) B = sum_compose(B, sum_step(t[i], ub));
+            t[i] = n[i];
         }
     }
+    if (ub == ua) B = A;
+    lanes[lane] = make_uint4(A.e, A.o, B.e, B.o);
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         SumStep oa, ob;
@@ -86,7 +112,6 @@ __device__ __forceinline__ void warp_sum_steps(const float *__restrict__ x, uint
             B = sum_compose(B, ob);
         }
     }
-    if (ub == ua) B = A;
 }
 
 // a float's binade: unit exponent, m, and the m the binade ends at
@@ -103,23 +128,66 @@ __device__ __forceinline__ float sum_join(uint32_t Es, uint32_t m) {
 }
 
 // s plus the terms x[lo, hi), one add after another; a whole warp, the same s
-// in every lane
-__device__ __forceinline__ float warp_serial_add(float s, const float *__restrict__ x, uint64_t lo, uint64_t hi) {
+// in every lane.  The terms go through 128 floats of shared memory, so that
+// the chain is the adds alone (out of shuffles it took 32 cycles a term).
+__device__ __forceinline__ float warp_serial_add(float s, const float *__restrict__ x, uint64_t lo, uint64_t hi,
+                                                 float *buf) {
     const uint32_t lane = threadIdx.x & 31u;
-    float next = lo + lane < hi ? __ldcg(x + lo + lane) : 0.0f;
-    for (uint64_t p = lo; p < hi; p += 32) {
-        const float t = next;
-        next = p + 32 + lane < hi ? __ldcg(x + p + 32 + lane) : 0.0f;
-        // adding 0 past the end leaves s as it is
+#pragma unroll 1
+    for (uint64_t p = lo; p < hi; p += 128) {
+        float t[4];
 #pragma unroll
-        for (int k = 0; k < 32; ++k) s = FADD(s, __shfl_sync(0xffffffffu, t, k));
+        for (int i = 0; i < 4; ++i) {
+            const uint64_t k = p + 32u * i + lane;
+            t[i] = k < hi ? __ldcg(x + k) : 0.0f;   // adding 0 past the end leaves s as it is
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) buf[32u * i + lane] = t[i];
+        __syncwarp();
+        const uint32_t n = (uint32_t)min(hi - p, (uint64_t)128);
+#pragma unroll 1
+        for (uint32_t k = 0; k < n; k += 32) {
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const float4 *>(buf + k + 4 * i);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s = FADD(FADD(FADD(FADD(s, v[i].x), v[i].y), v[i].z), v[i].w);
+        }
     }
     return s;
 }
 
+// the pairs of 32 consecutive runs (lane l: its run's, for the binade the sum
+// s is in) from run `pos` on, applied up to the first that leaves the binade
+// or has no pair for it; returns that run (32: none)
+__device__ __forceinline__ uint32_t warp_sum_apply(float &s, uint32_t pos, bool any, int32_t ua, int32_t ub, SumStep a,
+                                                   SumStep b) {
+    const uint32_t lane = threadIdx.x & 31u;
+    int32_t eu;
+    uint32_t m, top, Es;
+    sum_split(s, eu, m, top, Es);
+    SumStep inc{0u, 0u};
+    if (lane >= pos && !any) inc = ua == eu ? a : (ub == eu ? b : SumStep{kSumSat, kSumSat});
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        SumStep o;
+        o.e = __shfl_up_sync(0xffffffffu, inc.e, d);
+        o.o = __shfl_up_sync(0xffffffffu, inc.o, d);
+        if ((int)lane >= d) inc = sum_compose(o, inc);
+    }
+    const uint32_t ma = sum_apply(m, inc);
+    const uint32_t fails = __ballot_sync(0xffffffffu, ma >= top);
+    const uint32_t f = fails ? (uint32_t)__ffs(fails) - 1u : 32u;
+    if (f > pos) s = sum_join(Es, __shfl_sync(0xffffffffu, ma, f - 1));
+    return f;
+}
+
+__device__ __forceinline__ bool sum_is_inf(float s) { return __float_as_uint(s) >> 23 >= 0xffu; }
+
 // the walk over the slices (one warp; see the file header)
 __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t L, uint64_t LW, uint32_t nw,
-                               const SumScr &scr, uint32_t G) {
+                               const SumScr &scr, uint32_t G, float *buf) {
     const uint32_t lane = threadIdx.x & 31u;
     float s = 0.0f;
     for (uint32_t base = 0; base < G; base += 32) {
@@ -136,26 +204,10 @@ __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t
             r.b = SumStep{u1.x, u1.y};
         }
         for (uint32_t pos = 0; pos < cnt;) {
-            int32_t eu;
-            uint32_t m, top, Es;
-            sum_split(s, eu, m, top, Es);
-            if (Es >= 0xffu) return s;   // inf stays
-            SumStep inc{0u, 0u};
-            if (lane >= pos && r.ua != kAnyUnit)
-                inc = r.ua == eu ? r.a : (r.ub == eu ? r.b : SumStep{kSumSat, kSumSat});
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                SumStep o;
-                o.e = __shfl_up_sync(0xffffffffu, inc.e, d);
-                o.o = __shfl_up_sync(0xffffffffu, inc.o, d);
-                if ((int)lane >= d) inc = sum_compose(o, inc);
-            }
-            const uint32_t ma = sum_apply(m, inc);
-            const uint32_t fails = __ballot_sync(0xffffffffu, ma >= top);
-            const uint32_t f = fails ? min((uint32_t)__ffs(fails) - 1u, cnt) : cnt;
-            if (f > pos) s = sum_join(Es, __shfl_sync(0xffffffffu, ma, f - 1));
-            pos = f;
-            if (f == cnt) continue;
+            if (sum_is_inf(s)) return s;   // inf stays
+            const uint32_t f = warp_sum_apply(s, pos, r.ua == kAnyUnit, r.ua, r.ub, r.a, r.b);
+            if (f >= cnt) break;
+            pos = f + 1;
             // slice base + f, one warp's part after another
             const uint32_t b = base + f;
             const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
@@ -164,16 +216,39 @@ __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t
             for (uint32_t w = 0; w < nw; ++w) {
                 const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
                 if (p0 >= p1) break;
+                int32_t eu;
+                uint32_t m, top, Es;
                 sum_split(s, eu, m, top, Es);
                 if (Es >= 0xffu) return s;
+                if (ua != eu && ub != eu) {
+                    s = warp_serial_add(s, x, p0, p1, buf);
+                    continue;
+                }
                 SumStep st;
                 st.e = __shfl_sync(0xffffffffu, ua == eu ? part.x : part.z, w);
                 st.o = __shfl_sync(0xffffffffu, ua == eu ? part.y : part.w, w);
                 const uint32_t mw = sum_apply(m, st);
-                if ((ua == eu || ub == eu) && mw < top) s = sum_join(Es, mw);
-                else s = warp_serial_add(s, x, p0, p1);
+                if (mw < top) {
+                    s = sum_join(Es, mw);
+                    continue;
+                }
+                // the part crosses: its lanes' runs, the crossing one term by term
+                const uint4 lp = __ldcg(scr.lane + ((size_t)b * 8 + w) * 32 + lane);
+                const uint64_t k = (p1 - p0 + 31u) / 32u;
+                for (uint32_t q = 0; q < 32u;) {
+                    if (sum_is_inf(s)) return s;
+                    const uint32_t g = warp_sum_apply(s, q, false, ua, ub, SumStep{lp.x, lp.y}, SumStep{lp.z, lp.w});
+                    if (g >= 32u) break;
+                    const uint64_t q0 = min(p0 + g * k, p1), q1 = min(q0 + k, p1);
+                    s = warp_serial_add(s, x, q0, q1, buf);
+                    q = g + 1;
+                    sum_split(s, eu, m, top, Es);
+                    if (q < 32u && ua != eu && ub != eu) {   // a binade nobody guessed: the rest one by one
+                        s = warp_serial_add(s, x, q1, p1, buf);
+                        break;
+                    }
+                }
             }
-            pos = f + 1;
         }
     }
     return s;
@@ -189,6 +264,7 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
     static_assert(NT <= 256, "eight warps' pairs per block");
     constexpr uint32_t NW = NT / 32;
     __shared__ uint4 s_part[2][NW];
+    __shared__ __align__(16) float s_add[2][128];
     const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     const uint64_t L = ((n + G - 1) / G + 3) & ~3ull, LW = (L + NW - 1) / NW;
     const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
@@ -197,6 +273,7 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
     for (int j = 0; j < nsum; ++j) {
         const float *x = j ? x1 : x0;
         double v = 0.0;
+#pragma unroll 4
         for (uint64_t k = lo + tid; k < hi; k += NT) v += (double)__ldcg(x + k);
         own[j] = broadcast_sum(block_sum<NT>(v, red));
         if (tid == 0) SumScr(partials, G, j).slice[b] = own[j];
@@ -211,7 +288,7 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
         const int32_t ua = sum_unit(P * (1.0 - wide)), ub = sum_unit((P + own[j]) * (1.0 + wide));
         const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
         SumStep A, B;
-        warp_sum_steps(j ? x1 : x0, p0, p1, ua, ub, A, B);
+        warp_sum_steps(j ? x1 : x0, p0, p1, ua, ub, A, B, scr.lane + ((size_t)b * 8 + w) * 32);
         if (lane == 0) {
             const uint4 r = make_uint4(A.e, A.o, B.e, B.o);
             s_part[j][w] = r;
@@ -237,7 +314,7 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
         __syncthreads();
     }
     if (b == 0 && w < (uint32_t)nsum) {
-        const float s = warp_sum_walk(w ? x1 : x0, n, L, LW, NW, SumScr(partials, G, (int)w), G);
+        const float s = warp_sum_walk(w ? x1 : x0, n, L, LW, NW, SumScr(partials, G, (int)w), G, s_add[w]);
         if (lane == 0) {
             if (w) ctl->fb_p = s;
             else ctl->fb_s = s;
@@ -255,14 +332,14 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
 
 // one serial-mode check of a one-launch loop, undecided by the bounds: the
 // serial sum of the check's terms and, where the previous delta is not exact
-// yet, of its terms decide.  Every block of the grid calls it with the same x.
+// yet, of the previous check's terms decide.  Every block of the grid calls it with the same x.
 template <int NT>
-__device__ __forceinline__ bool grid_serial_form(SerialCheck &x, const LoopyCtl &sc, LoopyCtl *ctl, double *partials,
-                                                 const float *absdiff, uint32_t &gen, uint32_t *s_fail, double *red) {
-    const float *xs = absdiff + (size_t)x.cb * sc.ad_stride;
-    const float *xp = x.p_exact ? nullptr : absdiff + (size_t)sc.prev_buf * sc.ad_stride;
+__device__ __noinline__ bool grid_serial_form(SerialCheck &x, const float *terms, const float *prev_terms,
+                                                 uint64_t n, float tol, LoopyCtl *ctl, double *partials, uint32_t &gen,
+                                                 uint32_t *s_fail, double *red) {
+    const float *xp = x.p_exact ? nullptr : prev_terms;
     float s, p;
-    if (!grid_serial_sums<NT>(partials, xs, xp, sc.n_terms, ctl, gen, s_fail, red, s, p)) return false;
+    if (!grid_serial_sums<NT>(partials, terms, xp, n, ctl, gen, s_fail, red, s, p)) return false;
     x.s = s;
     x.lo = x.hi = (double)s;
     x.s_exact = true;
@@ -272,14 +349,14 @@ __device__ __forceinline__ bool grid_serial_form(SerialCheck &x, const LoopyCtl 
         x.p_exact = x.p_new = true;
         ++x.sums;
     }
-    x.d = serial_decide(x.lo, x.hi, true, x.plo, x.phi, true, sc.tol);
+    x.d = serial_decide(x.lo, x.hi, true, x.plo, x.phi, true, tol);
     return true;
 }
 
 // the returned delta and previous delta of a finished one-launch run, where
 // the loop decided without forming them
 template <int NT>
-__device__ __forceinline__ bool grid_serial_final(LoopyCtl &sc, LoopyCtl *ctl, double *partials, const float *absdiff,
+__device__ __noinline__ bool grid_serial_final(LoopyCtl &sc, LoopyCtl *ctl, double *partials, const float *absdiff,
                                                   uint32_t &gen, uint32_t *s_fail, double *red) {
     const bool cur = !sc.delta_exact, prev = !sc.prev_exact;
     if (!cur && !prev) return true;
