@@ -171,7 +171,6 @@ struct bp_graph {
     size_t staging_bytes = 0;
 
     // host-side copies of small structure arrays (tree waves, edge-variant runs)
-    uint8_t *node_s_host = nullptr;      // [V] state counts
     uint32_t *in_ptr_host = nullptr;     // [V+1], on demand
     uint32_t *run_len = nullptr;         // [nruns] runs of equal state count (device)
     uint8_t *run_s = nullptr;

@@ -177,6 +177,26 @@ __global__ void k_states_u8(const uint32_t *__restrict__ s32, uint32_t V, uint32
     if (v < V) s8[v] = (uint8_t)(s32 ? s32[v] : uniform);
 }
 
+// state counts -> u8, their smallest and largest, and the first node whose
+// count is out of range: out[0] = min, out[1] = max, out[2] = that node
+// (0xffffffff: none); out starts as {~0, 0, ~0}
+__global__ void k_states_scan(const uint32_t *__restrict__ s32, uint32_t V, uint8_t *__restrict__ s8,
+                              uint32_t *__restrict__ out) {
+    const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t s = v < V ? s32[v] : 1u;
+    if (v < V) s8[v] = (uint8_t)s;
+    const bool bad = v < V && (s < 1u || s > (uint32_t)kMaxStates);
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, v < V ? s : 0xffffffffu);
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, v < V ? s : 0u);
+    const uint32_t at = __reduce_min_sync(0xffffffffu, bad ? (uint32_t)v : 0xffffffffu);
+    if ((threadIdx.x & 31u) == 0u) {
+        // most warps change nothing: a plain read first
+        if (lo < *(volatile uint32_t *)out) atomicMin(out, lo);
+        if (hi > *(volatile uint32_t *)(out + 1)) atomicMax(out + 1, hi);
+        if (at != 0xffffffffu) atomicMin(out + 2, at);
+    }
+}
+
 // joint tables, edge-id order with caller strides -> position order [MS][MS]
 template <int MS>
 __global__ void k_gather_joint(const float *__restrict__ jin, uint32_t rs, uint64_t es,
@@ -577,7 +597,6 @@ static void free_graph(bp_graph *g) {
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
     if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
-    free(g->node_s_host);
     free(g->in_ptr_host);
     delete g;
 }
@@ -586,20 +605,36 @@ static int create_impl(bp_graph *g, const bp_graph_desc *d) {
     const uint32_t V = d->num_nodes, E = d->num_edges;
     int st;
     StageTrace trace(g->stream, "create");
-    // ---- state counts (validated on the host when they are host memory)
-    std::vector<uint32_t> s32;
+    // ---- state counts, validated where they lie
     const uint32_t *states = d->node_num_states;
     uint32_t smax = 0, smin = 0xffffffffu;
+    if ((st = dev_alloc(g, (void **)&g->node_s, (size_t)V))) return st;
     if (!states) {
         if (d->uniform_states < 1 || d->uniform_states > BP_MAX_STATES)
             return set_error(BP_ERR_SHAPE, "uniform_states %u not in [1, %d]", d->uniform_states, BP_MAX_STATES);
         smax = smin = d->uniform_states;
-    } else {
-        if (d->memory == BP_MEM_DEVICE) {
-            s32.resize(V);
-            if (V) BP_CUDA(cudaMemcpy(s32.data(), states, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost));
-            states = s32.data();
+    } else if (d->memory == BP_MEM_DEVICE && V) {
+        // one pass and one 12-byte read-back (a copy to the host and a loop
+        // there took 0.4-1.0 ms for 200,000 nodes, 25 us here).  The caller's
+        // array may come from work on the legacy default stream, which the
+        // copy used to wait for.
+        BP_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        uint32_t *out = nullptr, got[3] = {0xffffffffu, 0u, 0xffffffffu};
+        BP_CUDA(cudaMallocAsync((void **)&out, sizeof got, g->stream));
+        BP_CUDA(cudaMemcpyAsync(out, got, sizeof got, cudaMemcpyHostToDevice, g->stream));
+        k_states_scan<<<grid_for(V, 256), 256, 0, g->stream>>>(states, V, g->node_s, out);
+        BP_CUDA(cudaGetLastError());
+        BP_CUDA(cudaMemcpyAsync(got, out, sizeof got, cudaMemcpyDeviceToHost, g->stream));
+        BP_CUDA(cudaStreamSynchronize(g->stream));
+        cudaFreeAsync(out, g->stream);
+        smin = got[0];
+        smax = got[1];
+        if (got[2] != 0xffffffffu) {
+            uint32_t bad = 0;
+            BP_CUDA(cudaMemcpy(&bad, states + got[2], sizeof bad, cudaMemcpyDeviceToHost));
+            return set_error(BP_ERR_SHAPE, "node %u has %u states (must be 1..%d)", got[2], bad, BP_MAX_STATES);
         }
+    } else {
         for (uint32_t v = 0; v < V; ++v) {
             if (states[v] < 1 || states[v] > BP_MAX_STATES)
                 return set_error(BP_ERR_SHAPE, "node %u has %u states (must be 1..%d)", v, states[v], BP_MAX_STATES);
@@ -610,12 +645,6 @@ static int create_impl(bp_graph *g, const bp_graph_desc *d) {
     }
     g->ms = smax;
     g->uniform = (smax == smin) ? smax : 0;
-    g->node_s_host = (uint8_t *)malloc(V ? V : 1);
-    if (!g->node_s_host) return set_error(BP_ERR_NOMEM, "host allocation failed");
-    if (states)
-        for (uint32_t v = 0; v < V; ++v) g->node_s_host[v] = (uint8_t)states[v];
-    else
-        memset(g->node_s_host, (int)d->uniform_states, V);
     trace.mark("state counts");
 
     // ---- device arrays
@@ -626,7 +655,6 @@ static int create_impl(bp_graph *g, const bp_graph_desc *d) {
     if ((st = dev_alloc(g, (void **)&g->in_src, sizeof(uint32_t) * ((size_t)E + kArrayPadEdges)))) return st;
     if ((st = dev_alloc(g, (void **)&g->pos_edge, sizeof(uint32_t) * (size_t)E))) return st;
     // edge_pos (position of each edge id) is built on first use (ensure_edge_pos)
-    if ((st = dev_alloc(g, (void **)&g->node_s, (size_t)V))) return st;
     if (!g->uniform && (st = dev_alloc(g, (void **)&g->pos_dims, (size_t)E))) return st;
     if ((st = dev_alloc(g, (void **)&g->joint, sizeof(float) * ms * ms * ((size_t)E + kArrayPadEdges)))) return st;
     if ((st = dev_alloc(g, (void **)&g->belief, sizeof(float) * ms * ((size_t)V + kArrayPadNodes)))) return st;
@@ -644,12 +672,12 @@ static int create_impl(bp_graph *g, const bp_graph_desc *d) {
     BP_CUDA(cudaMemsetAsync(g->visited, 0, (size_t)V, g->stream));
     trace.mark("allocate + clear");
 
-    // state counts -> u8
-    {
+    // state counts -> u8 (device memory: written by the scan above)
+    if (!states || d->memory == BP_MEM_HOST) {
         void *s_dev = nullptr;
         bool owned = false;
-        if (d->node_num_states) {
-            if ((st = to_device(g, d->node_num_states, sizeof(uint32_t) * V, d->memory, &s_dev, &owned))) return st;
+        if (states) {
+            if ((st = to_device(g, states, sizeof(uint32_t) * V, d->memory, &s_dev, &owned))) return st;
         }
         if (V) {
             k_states_u8<<<grid_for(V, 256), 256, 0, g->stream>>>((const uint32_t *)s_dev, V, d->uniform_states,
@@ -759,10 +787,6 @@ static int create_impl(bp_graph *g, const bp_graph_desc *d) {
             k_permute_u8<<<grid_for(V, 256), 256, 0, g->stream>>>(g->node_s, g->new_to_old, V, s8);
             BP_CUDA(cudaMemcpyAsync(g->node_s, s8, V, cudaMemcpyDeviceToDevice, g->stream));
             cudaFreeAsync(s8, g->stream);
-            if (!g->uniform) {
-                BP_CUDA(cudaMemcpyAsync(g->node_s_host, g->node_s, V, cudaMemcpyDeviceToHost, g->stream));
-                BP_CUDA(cudaStreamSynchronize(g->stream));
-            }
         }
         BP_CUDA(cudaGetLastError());
         cudaFreeAsync(deg, g->stream);

@@ -174,9 +174,9 @@ int tree_build_levels_gpu(bp_graph *g, uint32_t *levels_out, uint32_t *num_level
     BP_CUDA(pb.get(&ckeys, V));
     BP_CUDA(pb.get(&ckeys_sorted, V));
     const size_t bytes = sizeof(uint32_t) * (V ? V : 1);
-    BP_CUDA(cudaMalloc((void **)&t.d_node_level, bytes));
-    BP_CUDA(cudaMalloc((void **)&t.d_node_lidx, bytes));
-    BP_CUDA(cudaMalloc((void **)&t.d_wave_nodes, bytes));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_node_level, bytes, st));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_node_lidx, bytes, st));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_wave_nodes, bytes, st));
     sorted_nodes = t.d_wave_nodes;
     uint32_t hc = 0;
     uint32_t *h_count = &hc;

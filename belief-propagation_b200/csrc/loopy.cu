@@ -1417,18 +1417,27 @@ static int ensure_runs(bp_graph *g) {
     if (g->run_len || g->V == 0) return BP_OK;
     std::vector<uint32_t> len;
     std::vector<uint8_t> s;
-    for (uint32_t v = 0; v < g->V; ++v) {
-        if (s.empty() || s.back() != g->node_s_host[v]) {
-            s.push_back(g->node_s_host[v]);
-            len.push_back(0);
+    if (g->uniform) {
+        len.push_back(g->V);
+        s.push_back((uint8_t)g->uniform);
+    } else {
+        std::vector<uint8_t> all(g->V);
+        BP_CUDA(cudaMemcpyAsync(all.data(), g->node_s, g->V, cudaMemcpyDeviceToHost, g->stream));
+        BP_CUDA(cudaStreamSynchronize(g->stream));
+        for (uint32_t v = 0; v < g->V; ++v) {
+            if (s.empty() || s.back() != all[v]) {
+                s.push_back(all[v]);
+                len.push_back(0);
+            }
+            len.back()++;
         }
-        len.back()++;
     }
     int st;
     if ((st = dev_alloc(g, (void **)&g->run_len, sizeof(uint32_t) * len.size()))) return st;
     if ((st = dev_alloc(g, (void **)&g->run_s, s.size()))) return st;
-    BP_CUDA(cudaMemcpy(g->run_len, len.data(), sizeof(uint32_t) * len.size(), cudaMemcpyHostToDevice));
-    BP_CUDA(cudaMemcpy(g->run_s, s.data(), s.size(), cudaMemcpyHostToDevice));
+    BP_CUDA(cudaMemcpyAsync(g->run_len, len.data(), sizeof(uint32_t) * len.size(), cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaMemcpyAsync(g->run_s, s.data(), s.size(), cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaStreamSynchronize(g->stream));   // the host arrays go out of scope
     g->nruns = (uint32_t)len.size();
     return BP_OK;
 }

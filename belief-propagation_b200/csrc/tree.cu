@@ -389,14 +389,10 @@ __global__ void k_tree_marginalize(uint32_t V, const uint32_t *__restrict__ in_p
 void tree_clear(bp_graph *g) {
     TreeData &t = g->tree;
     if (t.exec) cudaGraphExecDestroy(t.exec);
-    void *sched[] = {t.q_joint, t.q_joff, t.q_lvidx, t.q_y, t.q_pos, t.q_dst, t.s_in, t.s_out, t.s_lidx, t.s_S};
+    void *sched[] = {t.q_joint, t.q_joff, t.q_lvidx, t.q_y, t.q_pos, t.q_dst, t.s_in, t.s_out, t.s_lidx, t.s_S,
+                     t.d_wave_off, t.d_bar, t.d_node_level, t.d_node_lidx, t.d_wave_nodes};
     for (void *p : sched)
-        if (p) cudaFree(p);
-    if (t.d_wave_off) cudaFree(t.d_wave_off);
-    if (t.d_bar) cudaFree(t.d_bar);
-    if (t.d_node_level) cudaFree(t.d_node_level);
-    if (t.d_node_lidx) cudaFree(t.d_node_lidx);
-    if (t.d_wave_nodes) cudaFree(t.d_wave_nodes);
+        if (p) cudaFreeAsync(p, g->stream);
     free(t.levels_host);
     free(t.wave_off);
     free(t.level_wave_begin);
@@ -437,12 +433,13 @@ int tree_prepare_host(bp_graph *g, const uint32_t *levels, uint32_t num_levels) 
     t.total_waves = total;
     t.num_levels = num_levels;
     const size_t bytes = sizeof(uint32_t) * (V ? V : 1);
-    BP_CUDA(cudaMalloc((void **)&t.d_node_level, bytes));
-    BP_CUDA(cudaMalloc((void **)&t.d_node_lidx, bytes));
-    BP_CUDA(cudaMalloc((void **)&t.d_wave_nodes, bytes));
-    BP_CUDA(cudaMemcpy(t.d_node_level, node_level.data(), bytes, cudaMemcpyHostToDevice));
-    BP_CUDA(cudaMemcpy(t.d_node_lidx, node_lidx.data(), bytes, cudaMemcpyHostToDevice));
-    BP_CUDA(cudaMemcpy(t.d_wave_nodes, wave_nodes.data(), bytes, cudaMemcpyHostToDevice));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_node_level, bytes, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_node_lidx, bytes, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_wave_nodes, bytes, g->stream));
+    BP_CUDA(cudaMemcpyAsync(t.d_node_level, node_level.data(), bytes, cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaMemcpyAsync(t.d_node_lidx, node_lidx.data(), bytes, cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaMemcpyAsync(t.d_wave_nodes, wave_nodes.data(), bytes, cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaStreamSynchronize(g->stream));   // the host arrays go out of scope
     t.ready = true;
     return BP_OK;
 }
@@ -468,15 +465,17 @@ static int tree_q_build(bp_graph *g) {
     int st;
     if ((st = ensure_out_csr(g))) return st;
     const size_t ne = E ? E : 1, nv = V ? V : 1;
-    BP_CUDA(cudaMalloc((void **)&t.s_in, sizeof(uint2) * nv));
-    BP_CUDA(cudaMalloc((void **)&t.s_out, sizeof(uint32_t) * (nv + 1)));
-    BP_CUDA(cudaMalloc((void **)&t.s_lidx, sizeof(uint32_t) * nv));
-    BP_CUDA(cudaMalloc((void **)&t.s_S, nv));
-    BP_CUDA(cudaMalloc((void **)&t.q_y, ne));
-    BP_CUDA(cudaMalloc((void **)&t.q_joff, sizeof(uint32_t) * (ne + 1)));
-    BP_CUDA(cudaMalloc((void **)&t.q_lvidx, sizeof(uint2) * ne));
-    BP_CUDA(cudaMalloc((void **)&t.q_pos, sizeof(uint32_t) * ne));
-    BP_CUDA(cudaMalloc((void **)&t.q_dst, sizeof(uint32_t) * ne));
+    StageTrace trace(g->stream, "tree arrays");
+    BP_CUDA(cudaMallocAsync((void **)&t.s_in, sizeof(uint2) * nv, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.s_out, sizeof(uint32_t) * (nv + 1), g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.s_lidx, sizeof(uint32_t) * nv, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.s_S, nv, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.q_y, ne, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.q_joff, sizeof(uint32_t) * (ne + 1), g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.q_lvidx, sizeof(uint2) * ne, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.q_pos, sizeof(uint32_t) * ne, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.q_dst, sizeof(uint32_t) * ne, g->stream));
+    trace.mark("buffers");
     uint32_t *cnt = nullptr;
     BP_CUDA(cudaMallocAsync((void **)&cnt, sizeof(uint32_t) * (std::max(nv, ne) + 1), g->stream));
     BP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (std::max(nv, ne) + 1), g->stream));
@@ -495,19 +494,29 @@ static int tree_q_build(bp_graph *g) {
     BP_CUDA(cudaMemcpyAsync(&total, t.q_joff + E, sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
     BP_CUDA(cudaStreamSynchronize(g->stream));
     cudaFreeAsync(cnt, g->stream);
-    BP_CUDA(cudaMalloc((void **)&t.q_joint, sizeof(float) * ((size_t)total + 4)));
-    BP_CUDA(cudaMalloc((void **)&t.d_wave_off, sizeof(uint32_t) * ((size_t)t.total_waves + 1)));
-    BP_CUDA(cudaMemcpy(t.d_wave_off, t.wave_off, sizeof(uint32_t) * ((size_t)t.total_waves + 1),
-                       cudaMemcpyHostToDevice));
-    BP_CUDA(cudaMalloc((void **)&t.d_bar, 4 * sizeof(uint32_t)));
-    BP_CUDA(cudaMemset(t.d_bar, 0, 4 * sizeof(uint32_t)));
+    trace.mark("sizes");
+    BP_CUDA(cudaMallocAsync((void **)&t.q_joint, sizeof(float) * ((size_t)total + 4), g->stream));
     if (V)
         k_tq_fill<MS><<<grid_for(V, 256), 256, 0, g->stream>>>(V, t.d_wave_nodes, t.s_out, g->out_ptr, g->out_pos,
                                                                g->out_dst, g->node_s, t.q_y, t.q_joff, g->joint,
                                                                t.d_node_level, t.d_node_lidx, t.q_joint, t.q_lvidx,
                                                                t.q_pos, t.q_dst);
     BP_CUDA(cudaGetLastError());
-    BP_CUDA(cudaStreamSynchronize(g->stream));
+    trace.mark("fill");
+    return BP_OK;
+}
+
+// the cooperative tail launches' wave offsets and grid barrier (built before
+// any capture)
+static bool tree_tail_on();
+static int tree_tail_build(bp_graph *g) {
+    TreeData &t = g->tree;
+    if (!tree_tail_on() || t.d_bar) return BP_OK;
+    const size_t bytes = sizeof(uint32_t) * ((size_t)t.total_waves + 1);
+    BP_CUDA(cudaMallocAsync((void **)&t.d_wave_off, bytes, g->stream));
+    BP_CUDA(cudaMemcpyAsync(t.d_wave_off, t.wave_off, bytes, cudaMemcpyHostToDevice, g->stream));
+    BP_CUDA(cudaMallocAsync((void **)&t.d_bar, 4 * sizeof(uint32_t), g->stream));
+    BP_CUDA(cudaMemsetAsync(t.d_bar, 0, 4 * sizeof(uint32_t), g->stream));
     return BP_OK;
 }
 
@@ -657,7 +666,7 @@ static int launch_level(bp_graph *g, uint32_t level, int mode) {
     for (uint32_t w = w0; w < w1; ++w) {
         const uint32_t lo = t.wave_off[w], n = t.wave_off[w + 1] - lo;
         if (!n) continue;
-        if (tree_tail_on() && wave_group(n) == 32) {
+        if (t.d_bar && tree_tail_on() && wave_group(n) == 32) {
             // the run of warp-per-node waves that starts here
             uint32_t we = w + 1;
             while (we < w1 && wave_group(t.wave_off[we + 1] - t.wave_off[we]) == 32) ++we;
@@ -753,7 +762,8 @@ int bp_tree_level(bp_graph *g, uint32_t level) {
     if (level >= g->tree.num_levels) return set_error(BP_ERR_INVALID, "level %u >= num_levels %u", level,
                                                       g->tree.num_levels);
     int st = dispatch_q_build(g);
-    return st ? st : dispatch_level(g, level, 0);
+    if (st || (st = tree_tail_build(g))) return st;
+    return dispatch_level(g, level, 0);
 }
 
 int bp_tree_reset_visited(bp_graph *g) {
@@ -797,6 +807,7 @@ int bp_tree(bp_graph *g, bp_tree_result *res) {
         if ((st = bp_tree_build_levels(g, nullptr, &nl))) return st;
     }
     if ((st = dispatch_q_build(g))) return st;
+    if ((st = tree_tail_build(g))) return st;
     TreeData &t = g->tree;
     const uint32_t L = t.num_levels;
     uint32_t waves = t.level_wave_begin[1] - t.level_wave_begin[0] ? 1 : 0;
@@ -804,6 +815,7 @@ int bp_tree(bp_graph *g, bp_tree_result *res) {
     for (uint32_t l = L - 1; l > 0; --l) waves += t.level_wave_begin[l + 1] - t.level_wave_begin[l];
     // one launch per wave: the sequence is fixed for the levels, so it is
     // captured once into a CUDA graph and replayed
+    StageTrace trace(g->stream, "tree");
     if (!t.exec) {
         cudaGraph_t graph = nullptr;
         BP_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
@@ -814,7 +826,9 @@ int bp_tree(bp_graph *g, bp_tree_result *res) {
             return st;
         }
         if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture", __FILE__, __LINE__);
+        trace.mark("capture");
         cudaError_t ie = cudaGraphInstantiate(&t.exec, graph, 0);
+        trace.mark("instantiate");
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) {
             t.exec = nullptr;
