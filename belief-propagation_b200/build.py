@@ -29,7 +29,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = ["engine.cu", "loopy.cu", "tree.cu", "levels_gpu.cu", "batch.cu", "unrolled.cu"]
 C_SOURCES = ["graph_api.c", "levels.c", "xmlbif.c"]
 HEADERS = ["bp_internal.h", "bp_device.cuh", "bp_levels.h", "bp_serial.cuh", "flood_split.cuh", "edge_loop.cuh",
-           "serial_grid.cuh", "flood_loop.cuh"]
+           "serial_grid.cuh", "flood_loop.cuh", "batch_cluster.cuh"]
 
 
 def _newer(target, deps):

@@ -13,6 +13,7 @@
 //
 // Layout: the networks' arrays are concatenated (network order); inside a
 // network the edges are destination-sorted exactly as in bp_graph.
+#include <cooperative_groups.h>
 #include <errno.h>
 #include <stdio.h>
 #include <sys/stat.h>
@@ -365,6 +366,8 @@ __global__ void k_batch_solve(const BatchArgs a, const uint32_t *__restrict__ or
     }
 }
 
+#include "batch_cluster.cuh"
+
 // beliefs / messages between the caller's concatenated layout and ours
 __global__ void k_batch_msgs_out(const float *__restrict__ m0, const float *__restrict__ m1,
                                  const uint8_t *__restrict__ latest, const NetInfo *__restrict__ info,
@@ -387,6 +390,7 @@ struct Group {
     uint32_t *d_order = nullptr;
     uint32_t block = 0;            // threads per block (0 = not tuned yet)
     uint32_t grid = 0;
+    uint32_t large = 0;            // the first networks of `order`, solved by a cluster each with the f64 delta
 };
 
 }  // namespace bpx
@@ -403,7 +407,7 @@ struct bp_batch {
     float *absdiff = nullptr, *staging = nullptr;
     bpx::NetResult *res = nullptr;
     uint8_t *latest = nullptr;
-    uint32_t *queues = nullptr;   // one counter per group
+    uint32_t *queues = nullptr;   // counters: each group's single blocks, then each group's clusters
     std::vector<bpx::Group> groups;
     cudaGraphExec_t exec = nullptr;
     uint64_t exec_key = 0;
@@ -416,16 +420,51 @@ struct bp_batch {
 
 namespace bpx {
 
+// networks of at least this many edges are solved by a cluster each (f64
+// delta; below, a block's own latency is about the cluster barrier's and more
+// networks run side by side); BP_BATCH_CLUSTER_EDGES overrides (0: none)
+constexpr uint32_t kClusterEdges = 1024;
+
+// the cluster launch of the group's large networks, and a block each for the
+// rest (every network with the serial delta)
+template <int S>
+static int launch_large(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, cudaStream_t s) {
+    BP_CUDA(cudaFuncSetAttribute(k_batch_cluster<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem));
+    // as many clusters as the resident blocks make
+    const uint32_t clusters =
+        std::min<uint32_t>(gr.large, (uint32_t)std::max(1, kClusterPerSm * bt->sm_count / kBatchCluster));
+    k_batch_cluster<S><<<clusters * kBatchCluster, kClusterThreads, kClusterSmem, s>>>(a, gr.d_order, gr.large,
+                                                                                     bt->queues + bt->groups.size() + gi);
+    BP_CUDA(cudaGetLastError());
+    return BP_OK;
+}
+
 template <int S>
 static int launch_group(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, uint32_t block, uint32_t grid,
                         cudaStream_t s) {
+    const uint32_t skip = a.serial ? 0u : gr.large, rest = (uint32_t)gr.order.size() - skip;
+    if (!rest) return BP_OK;
     if (a.serial)
-        k_batch_solve<S, true><<<grid, block, sizeof(float) * 2 * a.sum_ch, s>>>(a, gr.d_order,
-                                                                               (uint32_t)gr.order.size(), bt->queues + gi);
+        k_batch_solve<S, true><<<grid, block, sizeof(float) * 2 * a.sum_ch, s>>>(a, gr.d_order, rest, bt->queues + gi);
     else
-        k_batch_solve<S, false><<<grid, block, 0, s>>>(a, gr.d_order, (uint32_t)gr.order.size(), bt->queues + gi);
+        k_batch_solve<S, false><<<std::min(grid, rest), block, 0, s>>>(a, gr.d_order + skip, rest, bt->queues + gi);
     BP_CUDA(cudaGetLastError());
     return BP_OK;
+}
+
+static int launch_large_s(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, cudaStream_t s) {
+    switch (gr.S) {
+    case 1: return launch_large<1>(bt, gr, a, gi, s);
+    case 2: return launch_large<2>(bt, gr, a, gi, s);
+    case 3: return launch_large<3>(bt, gr, a, gi, s);
+    case 4: return launch_large<4>(bt, gr, a, gi, s);
+    case 5: return launch_large<5>(bt, gr, a, gi, s);
+    case 6: return launch_large<6>(bt, gr, a, gi, s);
+    case 7: return launch_large<7>(bt, gr, a, gi, s);
+    case 8: return launch_large<8>(bt, gr, a, gi, s);
+    case 9: return launch_large<9>(bt, gr, a, gi, s);
+    default: return launch_large<10>(bt, gr, a, gi, s);
+    }
 }
 
 static int launch_group_s(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, uint32_t block, uint32_t grid,
@@ -509,22 +548,32 @@ static uint32_t grid_for_group(bp_batch *bt, const Group &gr, uint32_t block, si
     return std::min<uint32_t>(g, (uint32_t)gr.order.size());
 }
 
-// the whole batched solve on bt->stream: reset queues, fork one stream per
-// state-count group, launch each group's persistent kernel, join
+// the whole batched solve on bt->stream: reset queues, fork the groups'
+// streams (two per group: its clusters, its single blocks), launch the
+// clusters of every group, heaviest first, then the single blocks, join
 static int enqueue_batch(bp_batch *bt, const BatchArgs &a) {
-    BP_CUDA(cudaMemsetAsync(bt->queues, 0, sizeof(uint32_t) * bt->groups.size(), bt->stream));
+    const size_t ng = bt->groups.size();
+    BP_CUDA(cudaMemsetAsync(bt->queues, 0, sizeof(uint32_t) * 2 * ng, bt->stream));
     BP_CUDA(cudaEventRecord(bt->fork_ev, bt->stream));
-    for (size_t gi = 0; gi < bt->groups.size(); ++gi) {
+    for (size_t k = 0; k < 2 * ng; ++k) {
+        const bool large = k < ng;
+        const size_t gi = large ? k : k - ng;
         Group &gr = bt->groups[gi];
-        cudaStream_t s = bt->side[gi];
+        if (large ? (a.serial || !gr.large) : (!a.serial && gr.large == gr.order.size())) continue;
+        cudaStream_t s = bt->side[k];
         BP_CUDA(cudaStreamWaitEvent(s, bt->fork_ev, 0));
-        // serial mode holds 2 sum_ch floats of dynamic shared memory per block
-        const uint32_t grid =
-            a.sum_ch ? std::min(gr.grid, grid_for_group(bt, gr, gr.block, sizeof(float) * 2 * a.sum_ch)) : gr.grid;
-        int st = launch_group_s(bt, gr, a, (uint32_t)gi, gr.block, grid, s);
+        int st;
+        if (large) {
+            st = launch_large_s(bt, gr, a, (uint32_t)gi, s);
+        } else {
+            // serial mode holds 2 sum_ch floats of dynamic shared memory per block
+            const uint32_t grid =
+                a.sum_ch ? std::min(gr.grid, grid_for_group(bt, gr, gr.block, sizeof(float) * 2 * a.sum_ch)) : gr.grid;
+            st = launch_group_s(bt, gr, a, (uint32_t)gi, gr.block, grid, s);
+        }
         if (st) return st;
-        BP_CUDA(cudaEventRecord(bt->side_ev[gi], s));
-        BP_CUDA(cudaStreamWaitEvent(bt->stream, bt->side_ev[gi], 0));
+        BP_CUDA(cudaEventRecord(bt->side_ev[k], s));
+        BP_CUDA(cudaStreamWaitEvent(bt->stream, bt->side_ev[k], 0));
     }
     return BP_OK;
 }
@@ -573,7 +622,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
         // S, S*S floats at a time as float2/float4 when S allows it
         node_f = (node_f + 3) & ~(uint64_t)3;
         msg_f = (msg_f + 3) & ~(uint64_t)3;
-        joint_f = (joint_f + 3) & ~(uint64_t)3;
+        joint_f = (joint_f + 7) & ~(uint64_t)7;   // tables on 32 bytes: the cluster solver loads whole sectors
         h_joint.resize(joint_f, 0.0f);
         NetInfo &ni = bt->info[n];
         ni.V = d.num_nodes;
@@ -615,7 +664,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
     node_f = (node_f + 3) & ~(uint64_t)3;
     msg_f = (msg_f + 3) & ~(uint64_t)3;
     for (const NetInfo &ni : bt->info)
-        if ((ni.node_off | ni.msg_off | ni.joint_off) & 3u)
+        if (((ni.node_off | ni.msg_off) & 3u) || (ni.joint_off & 7u))
             return set_error(BP_ERR_STATE, "internal: unaligned network offsets");
     bt->totV = nodes;
     bt->totE = edges;
@@ -690,11 +739,22 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
     }
     for (auto &gr : bt->groups) {
         std::stable_sort(gr.order.begin(), gr.order.end(), [&](uint32_t x, uint32_t y) { return work(x) > work(y); });
+        gr.block = 256;
+        gr.grid = grid_for_group(bt, gr, gr.block);
+        const char *env = getenv("BP_BATCH_CLUSTER_EDGES");
+        const uint32_t least = env ? (uint32_t)strtoul(env, nullptr, 10) : kClusterEdges;
+        if (least) {
+            // first, largest first: the large ones (order sorts by work, so
+            // by edges up to the nodes' share)
+            auto mid = std::stable_partition(gr.order.begin(), gr.order.end(),
+                                             [&](uint32_t x) { return bt->info[x].E >= least; });
+            gr.large = (uint32_t)(mid - gr.order.begin());
+        }
         BP_CUDA(cudaMalloc((void **)&gr.d_order, sizeof(uint32_t) * gr.order.size()));
         BP_CUDA(cudaMemcpyAsync(gr.d_order, gr.order.data(), sizeof(uint32_t) * gr.order.size(),
                                 cudaMemcpyHostToDevice, bt->stream));
-        gr.block = 256;
-        gr.grid = grid_for_group(bt, gr, gr.block);
+    }
+    for (size_t k = 0; k < 2 * bt->groups.size(); ++k) {
         cudaStream_t s;
         BP_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         bt->side.push_back(s);
@@ -702,7 +762,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
         BP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         bt->side_ev.push_back(e);
     }
-    if ((st = alloc((void **)&bt->queues, sizeof(uint32_t) * bt->groups.size()))) return st;
+    if ((st = alloc((void **)&bt->queues, sizeof(uint32_t) * 2 * bt->groups.size()))) return st;
     BP_CUDA(cudaEventCreateWithFlags(&bt->fork_ev, cudaEventDisableTiming));
     BP_CUDA(cudaEventCreate(&bt->ev0));
     BP_CUDA(cudaEventCreate(&bt->ev1));
@@ -713,15 +773,17 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
 // ---- autotuning of threads per block, cached on disk ---------------------
 // kernel revision in the autotune key: a cached block size belongs to the
 // kernel it was timed on
-constexpr int kTuneRevision = 4;
+constexpr int kTuneRevision = 5;
 
 static std::string tune_key(bp_batch *bt, const Group &gr, int serial) {
+    // the networks that run a block each
     uint64_t V = 0, E = 0;
-    for (uint32_t n : gr.order) {
-        V += bt->info[n].V;
-        E += bt->info[n].E;
+    const size_t skip = serial ? 0 : gr.large;
+    for (size_t k = skip; k < gr.order.size(); ++k) {
+        V += bt->info[gr.order[k]].V;
+        E += bt->info[gr.order[k]].E;
     }
-    const uint64_t cnt = gr.order.size();
+    const uint64_t cnt = gr.order.size() - skip;
     const unsigned mv = (unsigned)(V / cnt), deg10 = (unsigned)(V ? 10 * E / V : 0);
     unsigned lv = 0;
     while ((1u << (lv + 1)) <= mv) ++lv;
@@ -896,6 +958,7 @@ int bp_batch_autotune(bp_batch *bt, const bp_batch_options *o) {
     const BatchArgs a = batch_args(bt, o->tolerance, o->max_iterations, serial, o->init_messages);
     for (size_t gi = 0; gi < bt->groups.size(); ++gi) {
         Group &gr = bt->groups[gi];
+        if (!serial && gr.large == gr.order.size()) continue;   // clusters only: nothing to tune
         const std::string key = tune_key(bt, gr, serial);
         uint32_t best_grid = 0;
         uint32_t best = cache_lookup(key, &best_grid);
