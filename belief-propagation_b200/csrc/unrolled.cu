@@ -167,6 +167,133 @@ __device__ __forceinline__ void sum_log_msgs(const UGraph &g, const float *sm, c
     }
 }
 
+// ---- messages in stored form ------------------------------------------------
+// A message depends on its source's state and its table alone, so the edges
+// that leave a node through the same table and orientation carry the same
+// one: on a grid with one table a node sends two messages to its four
+// neighbours.  Where that makes fewer messages than edges, each iteration
+// leaves them beside its state and the next one only adds them up: an edge
+// then costs a gather of S floats instead of S exponentials, S^2 products and
+// S + 1 logarithms, and the exponentials are taken once per node.  The values
+// and the order they are added in are the same.
+// 512 x 512 grid, 4 states, T = 30, forward and backward: 0.79 -> 0.69 ms; 64
+// grids of 32-256, 8 states, T = 20: 6.75 -> 5.86 ms (the forward's iteration
+// was bound by its instructions, 70 % of them the edges' logarithms).
+constexpr uint32_t kUMaxMsgs = 2 * kUMaxTables;
+struct UMsgs {
+    uint32_t n;                    // messages per node
+    const uint32_t *in_msg;        // [E] message of the edge at position p: (its table) * V + source
+    uint8_t table[kUMaxMsgs];      // message c uses table sm[table[c]] (2k, or 2k + 1 transposed)
+};
+
+// the messages of node v with log-state x
+template <int S>
+__device__ __forceinline__ void put_msgs(const UMsgs &ms, const float *sm, const float *x, uint32_t v, uint32_t V,
+                                         float *__restrict__ msgs) {
+    float e[S];
+    shifted_exp<S>(x, e);
+    for (uint32_t c = 0; c < ms.n; ++c) {
+        float sr[S], z = 0.0f;
+        row_sums<S>(sm + (uint32_t)ms.table[c] * S * S, e, sr);
+#pragma unroll
+        for (int i = 0; i < S; ++i) z += sr[i];
+        z = logf(z);
+#pragma unroll
+        for (int i = 0; i < S; ++i) sr[i] = logf(sr[i]) - z;
+        stv<S>(msgs + ((size_t)c * V + v) * S, sr);
+    }
+}
+
+// P += the stored messages of the in-edges [r0, r1), in order
+template <int S>
+__device__ __forceinline__ void sum_msgs(const uint32_t *__restrict__ in_msg, const float *__restrict__ msgs,
+                                         uint32_t r0, uint32_t r1, float *P) {
+    constexpr int B = u_batch<S>();
+    for (uint32_t p0 = r0; p0 < r1; p0 += B) {
+        float lm[B][S];
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (p0 + b < r1) ldv<S>(msgs + (size_t)in_msg[p0 + b] * S, lm[b]);
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (p0 + b < r1) {
+#pragma unroll
+                for (int i = 0; i < S; ++i) P[i] += lm[b][i];
+            }
+    }
+}
+
+// the priors' log-softmax and its messages
+template <int S>
+__global__ void __launch_bounds__(kUThreads) k_u_start_m(const UGraph g, const UMsgs ms, const float *__restrict__ theta,
+                                                         float *__restrict__ lb0, float *__restrict__ msgs) {
+    __shared__ __align__(16) float sm[2 * kUMaxTables * S * S];
+    griddep_launch_dependents();
+    load_tables_smem<S>(g, sm);
+    griddep_wait();
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= g.V) return;
+    float t[S];
+    ldv<S>(theta + (size_t)v * S, t);
+    const float z = lse<S>(t);
+#pragma unroll
+    for (int i = 0; i < S; ++i) t[i] -= z;
+    stv<S>(lb0 + (size_t)v * S, t);
+    put_msgs<S>(ms, sm, t, v, g.V, msgs);
+}
+
+// the messages of stored states (a recomputed segment's first iteration)
+template <int S>
+__global__ void __launch_bounds__(kUThreads) k_u_send_m(const UGraph g, const UMsgs ms, const float *__restrict__ x,
+                                                        float *__restrict__ msgs) {
+    __shared__ __align__(16) float sm[2 * kUMaxTables * S * S];
+    griddep_launch_dependents();
+    load_tables_smem<S>(g, sm);
+    griddep_wait();
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= g.V) return;
+    float t[S];
+    ldv<S>(x + (size_t)v * S, t);
+    put_msgs<S>(ms, sm, t, v, g.V, msgs);
+}
+
+// FIRST: lQ = lb + sum_in lm, no new belief (k_u_gather_q); else one forward
+// iteration (k_u_iter).  msgs_out null: nobody reads the next messages; lq_out
+// null: nor the next send state
+template <int S, bool FIRST>
+__global__ void __launch_bounds__(kUThreads) k_u_iter_m(const UGraph g, const UMsgs ms, const float *__restrict__ lb_in,
+                                                        const float *__restrict__ msgs, float *__restrict__ lb_out,
+                                                        float *__restrict__ lq_out, float *__restrict__ msgs_out) {
+    __shared__ __align__(16) float sm[2 * kUMaxTables * S * S];
+    griddep_launch_dependents();
+    load_tables_smem<S>(g, sm);
+    griddep_wait();
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= g.V) return;
+    float qo[S];
+    if constexpr (FIRST) {
+        ldv<S>(lb_in + (size_t)v * S, qo);
+        sum_msgs<S>(ms.in_msg, msgs, g.in_ptr[v], g.in_ptr[v + 1], qo);
+    } else {
+        float P[S], a[S];
+#pragma unroll
+        for (int i = 0; i < S; ++i) P[i] = 0.0f;
+        ldv<S>(lb_in + (size_t)v * S, a);
+        sum_msgs<S>(ms.in_msg, msgs, g.in_ptr[v], g.in_ptr[v + 1], P);
+#pragma unroll
+        for (int i = 0; i < S; ++i) a[i] += P[i];
+        const float z = lse<S>(a);
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            a[i] -= z;
+            qo[i] = a[i] + P[i];
+        }
+        stv<S>(lb_out + (size_t)v * S, a);
+    }
+    if (lq_out) stv<S>(lq_out + (size_t)v * S, qo);
+    if (msgs_out) put_msgs<S>(ms, sm, qo, v, g.V, msgs_out);
+}
+
 // sum of the x adjoint terms in the source-sorted slots [q0, q1), added in
 // slot order; the loads of up to two slots are issued together
 template <int S>
@@ -972,6 +1099,9 @@ struct bp_unrolled {
     uint32_t *out_dst = nullptr;             // [E] destination of source-sorted slot q (pull form)
     uint8_t *out_tab = nullptr;              // [E] its table id (pull form)
     float *pbv[2] = {nullptr, nullptr};      // [V][S] Pbar of steps t and t+1 (pull form)
+    bpx::UMsgs ms = {};                      // stored messages (n == 0: recomputed per edge)
+    uint32_t *in_msg = nullptr;              // [E]
+    float *msgs[2] = {nullptr, nullptr};     // [ms.n][V][S] of this iteration and the next
     float *pbar = nullptr;                   // [V][S] node-step adjoint Pbar (several tables only)
     double *epart = nullptr;
     float *theta_buf = nullptr, *gtheta_buf = nullptr, *glogp_buf = nullptr;
@@ -1030,11 +1160,20 @@ static int u_forward(bp_unrolled *u) {
     const size_t VS = (size_t)u->V * S;
     const unsigned gv = grid_for(u->V, kUThreads);
     cudaStream_t st = u->stream;
-    int rc;
-    if ((rc = u_launch(k_u_logsoftmax<S>, gv, kUThreads, st, u->V, (const float *)u->theta_buf, u->ck_b))) return rc;
-    if ((rc = u_launch(k_u_gather_q<S>, gv, kUThreads, st, g, (const float *)u->ck_b, (const float *)u->ck_b,
-                       u->ck_q)))
-        return rc;
+    int rc, mc = 0;   // mc: the message buffer read next
+    if (u->ms.n) {
+        if ((rc = u_launch(k_u_start_m<S>, gv, kUThreads, st, g, u->ms, (const float *)u->theta_buf, u->ck_b, u->msgs[0])))
+            return rc;
+        if ((rc = u_launch(k_u_iter_m<S, true>, gv, kUThreads, st, g, u->ms, (const float *)u->ck_b,
+                           (const float *)u->msgs[0], (float *)nullptr, u->ck_q, u->msgs[1])))
+            return rc;
+        mc = 1;
+    } else {
+        if ((rc = u_launch(k_u_logsoftmax<S>, gv, kUThreads, st, u->V, (const float *)u->theta_buf, u->ck_b))) return rc;
+        if ((rc = u_launch(k_u_gather_q<S>, gv, kUThreads, st, g, (const float *)u->ck_b, (const float *)u->ck_b,
+                           u->ck_q)))
+            return rc;
+    }
     // state t (lb_t, lQ_{t+1}) lives in checkpoint slot t/ck when t % ck == 0;
     // inside the last segment in its slot of the segment buffer, where the
     // backward reads it without recomputing; else in pp[t&1]
@@ -1053,9 +1192,46 @@ static int u_forward(bp_unrolled *u) {
     for (uint32_t t = 1; t <= u->T; ++t) {
         float *bo = (t == u->T) ? u->bT : loc_b(t);
         float *qo = (t == u->T) ? u->pp_q + (t & 1) * VS : loc_q(t);
+        if (u->ms.n) {
+            const bool last = t == u->T;
+            if ((rc = u_launch(k_u_iter_m<S, false>, gv, kUThreads, st, g, u->ms, (const float *)loc_b(t - 1),
+                               (const float *)u->msgs[mc], bo, last ? (float *)nullptr : qo,
+                               last ? (float *)nullptr : u->msgs[mc ^ 1])))
+                return rc;
+            mc ^= 1;
+            continue;
+        }
         if ((rc = u_launch(k_u_iter<S>, gv, kUThreads, st, g, (const float *)loc_b(t - 1), (const float *)loc_q(t - 1),
                            bo, qo)))
             return rc;
+    }
+    return BP_OK;
+}
+
+// segment s's states from its checkpoint, on the side stream (on the
+// forward's grid, a thread per node: on smaller grids beside the adjoint,
+// 80-296 blocks, it became the critical path)
+template <int S>
+static int u_recompute(bp_unrolled *u, const UGraph &g, uint32_t s) {
+    const size_t VS = (size_t)u->V * S;
+    const unsigned gv = grid_for(u->V, kUThreads);
+    const uint32_t t0 = s * u->ck, t_end = std::min(t0 + u->ck, u->T);
+    const float *ckb = u->ck_b + (size_t)s * VS, *ckq = u->ck_q + (size_t)s * VS;
+    float *sb = u->seg_b + (size_t)(s & 1u) * u->ck * VS, *sq = u->seg_q + (size_t)(s & 1u) * u->ck * VS;
+    int rc, mc = 0;
+    for (uint32_t j = 1; j + t0 < t_end; ++j) {
+        const float *bi = (j == 1) ? ckb : sb + (j - 1) * VS;
+        const float *qi = (j == 1) ? ckq : sq + (j - 1) * VS;
+        if (u->ms.n) {
+            if (j == 1 && (rc = u_launch(k_u_send_m<S>, gv, kUThreads, u->side, g, u->ms, ckq, u->msgs[0]))) return rc;
+            const bool last = j + 1 + t0 >= t_end;
+            rc = u_launch(k_u_iter_m<S, false>, gv, kUThreads, u->side, g, u->ms, bi, (const float *)u->msgs[mc],
+                          sb + j * VS, sq + j * VS, last ? (float *)nullptr : u->msgs[mc ^ 1]);
+            mc ^= 1;
+        } else {
+            rc = u_launch(k_u_iter<S>, gv, kUThreads, u->side, g, bi, qi, sb + j * VS, sq + j * VS);
+        }
+        if (rc) return rc;
     }
     return BP_OK;
 }
@@ -1108,17 +1284,6 @@ static int u_backward_pull(bp_unrolled *u) {
         const uint32_t nseg = (u->T + u->ck - 1) / u->ck;
         auto seg_b = [&](uint32_t s, uint32_t j) { return u->seg_b + ((size_t)(s & 1u) * u->ck + j) * VS; };
         auto seg_q = [&](uint32_t s, uint32_t j) { return u->seg_q + ((size_t)(s & 1u) * u->ck + j) * VS; };
-        auto recompute = [&](uint32_t s) -> int {
-            const uint32_t t0 = s * u->ck, t_end = std::min(t0 + u->ck, u->T);
-            const float *ckb = u->ck_b + (size_t)s * VS, *ckq = u->ck_q + (size_t)s * VS;
-            for (uint32_t j = 1; j + t0 < t_end; ++j) {
-                const float *bi = (j == 1) ? ckb : seg_b(s, j - 1);
-                const float *qi = (j == 1) ? ckq : seg_q(s, j - 1);
-                int r = u_launch(k_u_iter<S>, gv, kUThreads, u->side, g, bi, qi, seg_b(s, j), seg_q(s, j));
-                if (r) return r;
-            }
-            return BP_OK;
-        };
         int bc = 0, pc = 0;
         const float *pn = nullptr;   // Pbar of step t+1 (none at t = T)
         BP_CUDA(cudaEventRecord(u->ev_fork, st));
@@ -1127,7 +1292,7 @@ static int u_backward_pull(bp_unrolled *u) {
         for (int s = (int)nseg - 1; s >= 0; --s) {
             if (s >= 1) {
                 if ((uint32_t)s + 1 < nseg) BP_CUDA(cudaStreamWaitEvent(u->side, u->ev_bwd[(s + 1) & 1], 0));
-                if ((rc = recompute((uint32_t)s - 1))) return rc;
+                if ((rc = u_recompute<S>(u, g, (uint32_t)s - 1))) return rc;
                 BP_CUDA(cudaEventRecord(u->ev_rec[(s - 1) & 1], u->side));
             }
             BP_CUDA(cudaStreamWaitEvent(st, u->ev_rec[s & 1], 0));
@@ -1176,9 +1341,6 @@ static int u_backward(bp_unrolled *u) {
     // 85 registers (3 blocks per SM) instead of 64 (4 blocks)
     const int minb = ubwd_env("BP_UBWD_MINB", 4, 3);
     const unsigned gb = mma ? grid_for(u->V, kMmaThreads * 2) : grid_for(u->V, BT * npt);
-    // the recompute keeps the forward's grid, a thread per node: on smaller
-    // grids beside the adjoint (80-296 blocks) it became the critical path
-    const unsigned rgrid = gv;
     cudaStream_t st = u->stream;
     int rc = BP_OK;
     auto adjoint = [&](int mode, const float *send, const float *b_t, const float *gbar, const float *xn, float *out,
@@ -1218,17 +1380,6 @@ static int u_backward(bp_unrolled *u) {
     // two share nothing but the double-buffered segment states (buffer s & 1)
     auto seg_b = [&](uint32_t s, uint32_t j) { return u->seg_b + ((size_t)(s & 1u) * u->ck + j) * VS; };
     auto seg_q = [&](uint32_t s, uint32_t j) { return u->seg_q + ((size_t)(s & 1u) * u->ck + j) * VS; };
-    auto recompute = [&](uint32_t s) -> int {
-        const uint32_t t0 = s * u->ck, t_end = std::min(t0 + u->ck, u->T);
-        const float *ckb = u->ck_b + (size_t)s * VS, *ckq = u->ck_q + (size_t)s * VS;
-        for (uint32_t j = 1; j + t0 < t_end; ++j) {
-            const float *bi = (j == 1) ? ckb : seg_b(s, j - 1);
-            const float *qi = (j == 1) ? ckq : seg_q(s, j - 1);
-            int r = u_launch(k_u_iter<S>, rgrid, kUThreads, u->side, g, bi, qi, seg_b(s, j), seg_q(s, j));
-            if (r) return r;
-        }
-        return BP_OK;
-    };
     // the last segment's states are the forward's own (u_forward)
     BP_CUDA(cudaEventRecord(u->ev_fork, st));
     BP_CUDA(cudaStreamWaitEvent(u->side, u->ev_fork, 0));
@@ -1237,7 +1388,7 @@ static int u_backward(bp_unrolled *u) {
         if (s >= 1) {
             // buffer (s-1)&1 was last read by the adjoint of segment s+1
             if ((uint32_t)s + 1 < nseg) BP_CUDA(cudaStreamWaitEvent(u->side, u->ev_bwd[(s + 1) & 1], 0));
-            if ((rc = recompute((uint32_t)s - 1))) return rc;
+            if ((rc = u_recompute<S>(u, g, (uint32_t)s - 1))) return rc;
             BP_CUDA(cudaEventRecord(u->ev_rec[(s - 1) & 1], u->side));
         }
         BP_CUDA(cudaStreamWaitEvent(st, u->ev_rec[s & 1], 0));
@@ -1274,7 +1425,7 @@ static void u_free(bp_unrolled *u) {
     void *ptrs[] = {u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables, u->ck_b, u->ck_q,
                     u->seg_b, u->seg_q, u->pp_b, u->pp_q, u->bT, u->bbar[0], u->bbar[1], u->xc[0],
                     u->xc[1], u->epart, u->theta_buf, u->gtheta_buf, u->glogp_buf, u->pbar, u->out_dst,
-                    u->out_tab, u->pbv[0], u->pbv[1]};
+                    u->out_tab, u->pbv[0], u->pbv[1], u->in_msg, u->msgs[0], u->msgs[1]};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (u->fwd_exec) cudaGraphExecDestroy(u->fwd_exec);
@@ -1431,6 +1582,37 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
             otab[q] = tab[e];
         }
     }
+    // stored messages (see UMsgs): one per node and table orientation in use,
+    // where that leaves at least a quarter of the edges' own out (two tables on
+    // a grid, four messages against four edges: 560 us stored, 554 us
+    // recomputed per edge on the 201 x 201 grid of 5 states; BP_UNROLLED_MSG=0:
+    // never, 1: always)
+    std::vector<uint32_t> in_msg;
+    {
+        uint8_t index[256];
+        memset(index, 0xff, sizeof index);
+        uint32_t n = 0;
+        bool fits = true;
+        for (uint32_t p = 0; p < E && fits; ++p) {
+            const uint8_t t = ptab[p] & 0x7fu, o = (ptab[p] & 0x80u) ? 1 : 0;
+            uint8_t &at = index[2 * t + o];
+            if (at != 0xff) continue;
+            fits = n < kUMaxMsgs;
+            if (fits) {
+                u->ms.table[n] = (uint8_t)(2 * t + o);
+                at = (uint8_t)n++;
+            }
+        }
+        const char *env = getenv("BP_UNROLLED_MSG");
+        bool use = (uint64_t)n * V <= (uint64_t)E - E / 4;
+        if (env && (env[0] == '0' || env[0] == '1')) use = env[0] == '1';
+        if (use && fits && E && (uint64_t)n * V <= 0xffffffffull) {
+            u->ms.n = n;
+            in_msg.resize(E);
+            for (uint32_t p = 0; p < E; ++p)
+                in_msg[p] = index[2 * (ptab[p] & 0x7fu) + ((ptab[p] & 0x80u) ? 1 : 0)] * V + in_src[p];
+        }
+    }
     const size_t VS = (size_t)V * S;
     u->nblk = grid_for(V, 64);   // partial slots for the smallest backward block
     auto alloc = [&](void **p, size_t bytes) {
@@ -1452,6 +1634,9 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
                             alloc((void **)&u->pbv[0], sizeof(float) * VS) &&
                             alloc((void **)&u->pbv[1], sizeof(float) * VS))) &&
               alloc((void **)&u->epart, sizeof(double) * K * u->nblk * S * S) &&
+              (u->ms.n == 0 || (alloc((void **)&u->in_msg, 4 * (size_t)E) &&
+                                alloc((void **)&u->msgs[0], sizeof(float) * VS * u->ms.n) &&
+                                alloc((void **)&u->msgs[1], sizeof(float) * VS * u->ms.n))) &&
               (K == 1 || alloc((void **)&u->pbar, sizeof(float) * VS)) &&
               alloc((void **)&u->theta_buf, sizeof(float) * VS) && alloc((void **)&u->gtheta_buf, sizeof(float) * VS) &&
               alloc((void **)&u->glogp_buf, sizeof(float) * K * S * S);
@@ -1459,6 +1644,8 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
         u_free(u);
         return set_error(BP_ERR_NOMEM, "device allocation failed for the unrolled graph");
     }
+    u->ms.in_msg = u->in_msg;
+    if (u->ms.n) cudaMemcpyAsync(u->in_msg, in_msg.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
     cudaMemcpyAsync(u->in_ptr, in_ptr.data(), 4 * (V + 1), cudaMemcpyHostToDevice, u->stream);
     cudaMemcpyAsync(u->out_ptr, out_ptr.data(), 4 * (V + 1), cudaMemcpyHostToDevice, u->stream);
     if (E) {
