@@ -69,6 +69,8 @@ __global__ void __launch_bounds__(kSendThreads, send_min_blocks<MS>()) k_flood_s
     constexpr uint32_t NT = kSendThreads;
     __shared__ double red[NT / 32];
     LoopyCtl *ctl = a.ctl;
+    griddep_launch_dependents();   // the next pass's blocks come up as this one's leave
+    griddep_wait();
     if (*(volatile uint32_t *)&ctl->done) return;
     const uint32_t it = ctl->it, ce = ctl->check_every;
     const bool want = (ce <= 1) || ((it + 1) % ce == 0);
@@ -162,6 +164,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_flood_nodes(const SplitArgs a)
     __shared__ bool s_last;
     __shared__ __align__(16) float sbuf[CAP];
     LoopyCtl *ctl = a.ctl;
+    griddep_launch_dependents();   // the next pass's blocks come up as this one's leave
+    griddep_wait();
     if (*(volatile uint32_t *)&ctl->done) return;
     const uint32_t it = ctl->it, ce = ctl->check_every;
     const bool want = (ce <= 1) || ((it + 1) % ce == 0);

@@ -42,13 +42,18 @@ namespace bpx {
 template <int MS> constexpr int flood_nt() { return MS <= 2 ? 128 : (MS <= 4 ? 256 : 128); }
 template <int MS> constexpr int flood_smem_floats() { return MS <= 2 ? 2048 : 8192; }
 // in-edges per thread per phase-1 round of k_flood (tables held in registers)
-template <int MS> constexpr int flood_unroll() { return MS <= 2 ? 1 : (MS <= 4 ? 2 : 1); }
-// resident blocks per SM the register allocation must allow.  With 1-2
-// states, 48 warps of one edge per thread at 40 registers measured fastest on
-// the 16M-node graph: 0.93 ms against 1.07 ms for 32 warps of 4 edges per
-// thread at 64 registers; more warps hide the gather better than more
-// gathers per warp.
-template <int MS, int FU> constexpr int flood_min_blocks() { return MS <= 2 ? (FU >= 4 ? 8 : 12) : 1; }
+template <int MS> constexpr int flood_unroll() { return 1; }
+// resident blocks per SM the register allocation must allow; more warps hide
+// the gather better than more gathers per warp.  1-2 states: 48 warps of one
+// edge per thread at 40 registers took 0.93 ms on the 16M-node graph, 32
+// warps of 4 edges at 64 registers 1.07 ms.  3-4 states: 32 warps of one edge
+// at 64 registers take 34.1 us an iteration on 300,000 nodes and 1.2M edges of
+// 4 states (101 us on 1M / 4M), 16 warps of two edges at 118 registers 38.5
+// (118); 40 and 48 warps spill: 41.9 and 64.0.  From 5 states on the natural
+// allocation is as fast as any cap.
+template <int MS, int FU> constexpr int flood_min_blocks() { return MS <= 2 ? (FU >= 4 ? 8 : 12) : (MS <= 4 ? 4 : 1); }
+// the serial-delta form carries the serial sum's code: a cap would spill
+template <int MS, int FU> constexpr int flood_min_blocks_serial() { return MS <= 2 ? flood_min_blocks<MS, FU>() : 1; }
 
 struct FloodArgs {
     uint32_t V;          // tiles cover nodes [v_base, V)
@@ -755,6 +760,8 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood(const FloodArgs a,
     __shared__ bool s_last;
 
     LoopyCtl *ctl = a.ctl;
+    griddep_launch_dependents();   // the next iteration's blocks come up as this one's leave
+    griddep_wait();
     if (*(volatile uint32_t *)&ctl->done) return;
     const uint32_t it = ctl->it, ce = ctl->check_every;
     const bool want = (ce <= 1) || ((it + 1) % ce == 0);
@@ -1585,18 +1592,35 @@ static int resident_blocks(int *bps) {
     return resident_blocks_mb<MS, UNI, FU, flood_min_blocks<MS, FU>()>(bps);
 }
 
+// one iteration's kernel, launched with programmatic stream serialisation: its
+// blocks may come up while the last of the kernel ahead drain, and wait for
+// that grid before they read anything
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_iteration(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // launch of the block-tile kernel with the register cap block_min_blocks()
 template <int MS, bool UNI, int FU>
-static void launch_block_tiles(unsigned grid, cudaStream_t st, const FloodArgs &a, uint32_t ntiles, bool serial) {
+static cudaError_t launch_block_tiles(unsigned grid, cudaStream_t st, const FloodArgs &a, uint32_t ntiles, bool serial) {
     constexpr int NT = flood_nt<MS>();
     constexpr int MB = flood_min_blocks<MS, FU>();
-    if (serial) return k_flood<MS, UNI, FU, MB, true><<<grid, NT, 0, st>>>(a, ntiles);
+    if (serial) return launch_iteration(k_flood<MS, UNI, FU, MB, true>, grid, NT, st, a, ntiles);
     if constexpr (MS <= 2) {
         const int mb = block_min_blocks();
-        if (mb == 10) return k_flood<MS, UNI, FU, 10><<<grid, NT, 0, st>>>(a, ntiles);
-        if (mb == 16) return k_flood<MS, UNI, FU, 16><<<grid, NT, 0, st>>>(a, ntiles);
+        if (mb == 10) return launch_iteration(k_flood<MS, UNI, FU, 10>, grid, NT, st, a, ntiles);
+        if (mb == 16) return launch_iteration(k_flood<MS, UNI, FU, 16>, grid, NT, st, a, ntiles);
     }
-    k_flood<MS, UNI, FU><<<grid, NT, 0, st>>>(a, ntiles);
+    return launch_iteration(k_flood<MS, UNI, FU>, grid, NT, st, a, ntiles);
 }
 
 // block-tile grid: one block per tile, or (default; BP_FLOOD_PERSIST=0
@@ -1709,9 +1733,8 @@ static int split_run_nv(bp_graph *g, uint32_t k, uint32_t *nparts) {
     if (nparts) *nparts = ga;
     const SplitArgs a = split_args(g, ga);
     for (uint32_t i = 0; i < k; ++i) {
-        k_flood_send<MS, SER><<<ga, kSendThreads, 0, g->stream>>>(a);
-        k_flood_nodes<MS, SER, NV><<<gb, kNodeThreads, 0, g->stream>>>(a);
-        BP_CUDA(cudaGetLastError());
+        BP_CUDA((launch_iteration(k_flood_send<MS, SER>, ga, kSendThreads, g->stream, a)));
+        BP_CUDA((launch_iteration(k_flood_nodes<MS, SER, NV>, gb, kNodeThreads, g->stream, a)));
     }
     return BP_OK;
 }
@@ -1823,13 +1846,16 @@ static int enqueue_node_iterations(bp_graph *g, uint32_t k, bool serial, int var
     for (uint32_t i = 0; i < k; ++i) {
         if (!warp_tiled) {
             if constexpr (MS <= 2) {
-                if (unroll == 1) launch_block_tiles<MS, UNI, 1>(grid, g->stream, a, ntiles, serial);
-                else if (unroll == 2) launch_block_tiles<MS, UNI, 2>(grid, g->stream, a, ntiles, serial);
-                else launch_block_tiles<MS, UNI, 4>(grid, g->stream, a, ntiles, serial);
+                if (unroll == 1) BP_CUDA((launch_block_tiles<MS, UNI, 1>(grid, g->stream, a, ntiles, serial)));
+                else if (unroll == 2) BP_CUDA((launch_block_tiles<MS, UNI, 2>(grid, g->stream, a, ntiles, serial)));
+                else BP_CUDA((launch_block_tiles<MS, UNI, 4>(grid, g->stream, a, ntiles, serial)));
             } else {
                 constexpr int FU = flood_unroll<MS>();
-                if (serial) k_flood<MS, UNI, FU, flood_min_blocks<MS, FU>(), true><<<grid, NT, 0, g->stream>>>(a, ntiles);
-                else k_flood<MS, UNI, FU><<<grid, NT, 0, g->stream>>>(a, ntiles);
+                if (serial)
+                    BP_CUDA((launch_iteration(k_flood<MS, UNI, FU, flood_min_blocks_serial<MS, FU>(), true>, grid, NT,
+                                              g->stream, a, ntiles)));
+                else
+                    BP_CUDA((launch_iteration(k_flood<MS, UNI, FU>, grid, NT, g->stream, a, ntiles)));
             }
         } else if constexpr (MS <= 2) {
             if (unroll == 1) k_flood_w<MS, UNI, 1><<<grid, 256, 0, g->stream>>>(a);
@@ -2465,6 +2491,7 @@ static int noalloc_run(uint32_t V, uint32_t E, const uint32_t *in_ptr, const uin
     a.msg1 = messages + (size_t)E * MS;
     a.q0 = (float *)(b + off_q0);
     a.q1 = (float *)(b + off_q0 + qbytes);
+    a.pipe = 1;
     a.partials = (double *)(b + off_part);
     a.ctl = ctl;
     k_gather_q<MS, true><<<grid_for(V, 256), 256, 0, stream>>>(V, in_ptr, nullptr, beliefs, msg_latest, a.q0);
