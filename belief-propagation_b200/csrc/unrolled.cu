@@ -1036,6 +1036,197 @@ __global__ void __launch_bounds__(kPullThreads, MB) k_u_bwd_pull(
     }
 }
 
+// ---- the pull form with two tables (S <= 8) --------------------------------
+// k_u_bwd_pull's steps with four message kinds instead of two (each table, each
+// orientation).  A node's out-edges are sorted by kind, so one kind's row sums
+// and adjoint are live at a time, and a kind no out-edge uses costs nothing.
+// The scatter form it replaces takes a launch per table to recompute every
+// edge's sums for the table adjoint, on top of the step's own, and holds two
+// E x S slot arrays: 201 x 201 grid, 5 states, T = 10, forward and backward
+// 555 us with it, 270 us here.  Bound by each node's chain of loads (its
+// out-edges' Pbar, kind after kind) at 4 to 8 blocks of 4 warps per SM, as many
+// as the registers of S states leave without large spills.
+constexpr int kPull2Tables = 2;
+template <int S> constexpr int pull2_min_blocks() { return S <= 2 ? 8 : (S <= 4 ? 6 : (S <= 6 ? 5 : 4)); }
+
+template <int S>
+__global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_pull2(
+    const UGraph g, const uint32_t *__restrict__ out_dst, const uint8_t *__restrict__ out_tab, int mode,
+    const float *__restrict__ x_next, const float *__restrict__ pbar_next, const float *__restrict__ lb_t,
+    const float *__restrict__ gin, float *__restrict__ gout, float *__restrict__ pbar_out, double *__restrict__ epart) {
+    static_assert(S >= 1 && S <= 8, "pull form: up to 8 states");
+    constexpr bool MMA = S >= 5;
+    constexpr int KT = kPull2Tables, NT = kPullThreads, NW = NT / 32;
+    __shared__ __align__(16) float sm[2 * KT * S * S];
+    __shared__ __align__(16) float st_n[MMA ? NW : 1][32][8];
+    __shared__ __align__(16) float st_t[MMA ? NW : 1][32][8];
+    __shared__ __align__(16) float st_e[MMA ? NW : 1][32][8];
+    __shared__ float dred[MMA ? NW : 1][16][8];
+    __shared__ float wred[NW][MMA ? 1 : S * S];
+    griddep_launch_dependents();
+    load_tables_smem<S>(g, sm);
+    griddep_wait();
+    const bool edges = x_next != nullptr;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+    float acc[KT][MMA ? 1 : S * S], d[KT][4];
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+#pragma unroll
+        for (int i = 0; i < (MMA ? 1 : S * S); ++i) acc[k][i] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[k][i] = 0.0f;
+    }
+    for (uint32_t base = (blockIdx.x * NW + warp) * 32u;; base += gridDim.x * (uint32_t)NT) {
+        const uint32_t u = base + lane;
+        const bool active = u < g.V;
+        if (!__any_sync(0xffffffffu, active)) break;
+        float e[S], xb[S];
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            e[i] = 0.0f;
+            xb[i] = 0.0f;
+        }
+        uint32_t q = 0, q1 = 0;
+        if (active && edges) {
+            q = g.out_ptr[u];
+            q1 = g.out_ptr[u + 1];
+            float x[S];
+            ldv<S>(x_next + (size_t)u * S, x);
+            shifted_exp<S, true>(x, e);
+        }
+        if (edges) {
+#pragma unroll
+            for (int k = 0; k < KT; ++k) {
+                float cc[2][S];
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    float *c = cc[o];
+#pragma unroll
+                    for (int i = 0; i < S; ++i) c[i] = 0.0f;
+                    const uint8_t kind = (uint8_t)(k | (o ? 0x80 : 0));
+                    const float *J = sm + (2 * k + o) * S * S;
+                    if (q < q1 && out_tab[q] == kind) {
+                        float r[S], z = 0.0f;
+                        row_sums<S>(J, e, r);
+#pragma unroll
+                        for (int i = 0; i < S; ++i) z += r[i];
+#pragma unroll
+                        for (int i = 0; i < S; ++i) r[i] = __fdividef(1.0f, r[i]);
+                        const float iz = __fdividef(1.0f, z);
+                        do {
+                            float p[S], s = 0.0f;
+                            ldv<S>(pbar_next + (size_t)out_dst[q] * S, p);
+#pragma unroll
+                            for (int i = 0; i < S; ++i) s += p[i];
+                            const float a = s * iz;
+#pragma unroll
+                            for (int i = 0; i < S; ++i) c[i] += p[i] * r[i] - a;
+                            ++q;
+                        } while (q < q1 && out_tab[q] == kind);
+#pragma unroll
+                        for (int j = 0; j < S; ++j) {
+                            float t = 0.0f;
+#pragma unroll
+                            for (int i = 0; i < S; ++i) t += c[i] * J[i * S + j];
+                            xb[j] += t;
+                        }
+                    }
+                }
+                // table k's adjoint from cN and cT (zero on idle lanes)
+                if constexpr (!MMA) {
+#pragma unroll
+                    for (int i = 0; i < S; ++i)
+#pragma unroll
+                        for (int j = 0; j < S; ++j) acc[k][i * S + j] += cc[0][i] * e[j] + cc[1][j] * e[i];
+                } else {
+                    float pn[8], pt[8], pe[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        pn[i] = i < S ? cc[0][i < S ? i : 0] : 0.0f;
+                        pt[i] = i < S ? cc[1][i < S ? i : 0] : 0.0f;
+                        pe[i] = i < S ? e[i < S ? i : 0] : 0.0f;
+                    }
+                    reinterpret_cast<float4 *>(st_n[warp][lane])[0] = make_float4(pn[0], pn[1], pn[2], pn[3]);
+                    reinterpret_cast<float4 *>(st_n[warp][lane])[1] = make_float4(pn[4], pn[5], pn[6], pn[7]);
+                    reinterpret_cast<float4 *>(st_t[warp][lane])[0] = make_float4(pt[0], pt[1], pt[2], pt[3]);
+                    reinterpret_cast<float4 *>(st_t[warp][lane])[1] = make_float4(pt[4], pt[5], pt[6], pt[7]);
+                    if (k == 0) {
+                        reinterpret_cast<float4 *>(st_e[warp][lane])[0] = make_float4(pe[0], pe[1], pe[2], pe[3]);
+                        reinterpret_cast<float4 *>(st_e[warp][lane])[1] = make_float4(pe[4], pe[5], pe[6], pe[7]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        const int k0 = h * 8 + tq, k1 = k0 + 4;
+                        const float af[4] = {st_n[warp][k0][gq], st_t[warp][k0][gq], st_n[warp][k1][gq],
+                                             st_t[warp][k1][gq]};
+                        const float bf[2] = {st_e[warp][k0][gq], st_e[warp][k1][gq]};
+                        uint32_t ah[4], al[4], bh[2], bl[2];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) split_tf32(af[i], ah[i], al[i]);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) split_tf32(bf[i], bh[i], bl[i]);
+                        mma_tf32_16x8x8(d[k], ah, bh);
+                        mma_tf32_16x8x8(d[k], ah, bl);
+                        mma_tf32_16x8x8(d[k], al, bh);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        if (active) {
+            float gi[S], out[S], pb[S], gs = 0.0f;
+            ldv<S>(gin + (size_t)u * S, gi);
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                xb[i] *= e[i];
+                gi[i] += xb[i];
+                gs += gi[i];
+            }
+            if (mode == 1) {
+#pragma unroll
+                for (int i = 0; i < S; ++i) {
+                    out[i] = gi[i];
+                    pb[i] = xb[i];
+                }
+            } else {
+                float lb[S];
+                ldv<S>((mode == 0 ? lb_t : x_next) + (size_t)u * S, lb);
+#pragma unroll
+                for (int i = 0; i < S; ++i) {
+                    out[i] = gi[i] - expf(lb[i]) * gs;
+                    pb[i] = out[i] + xb[i];
+                }
+            }
+            stv<S>(gout + (size_t)u * S, out);
+            if (mode != 2) stv<S>(pbar_out + (size_t)u * S, pb);
+        }
+    }
+    if (!edges) return;   // uniform over the grid: no table adjoint in this launch
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        double *row = epart + ((size_t)k * gridDim.x + blockIdx.x) * S * S;
+        const float *J = sm + 2 * k * S * S;
+        if constexpr (MMA) {
+            dred[warp][gq][2 * tq] = d[k][0];
+            dred[warp][gq][2 * tq + 1] = d[k][1];
+            dred[warp][gq + 8][2 * tq] = d[k][2];
+            dred[warp][gq + 8][2 * tq + 1] = d[k][3];
+            __syncthreads();
+            // logJbar[a][b] += J[a][b] * (N[a][b] + T[b][a])
+            for (int i = threadIdx.x; i < S * S; i += NT) {
+                const int ra = i / S, cb = i % S;
+                double t = 0.0;
+                for (int w = 0; w < NW; ++w) t += (double)dred[w][ra][cb] + (double)dred[w][8 + cb][ra];
+                row[i] += (double)J[ra * S + cb] * t;
+            }
+        } else {
+            block_partial_add<S, NT, true>(acc[k], nullptr, wred, row, J);
+        }
+        __syncthreads();   // the reduction buffer is free for the next table
+    }
+}
+
 // the initial step's end: lbbar_0(s) = add(s) + the x adjoint terms of s's
 // out-edges, then through the log-softmax of the priors:
 // theta_bar = lbbar_0 - softmax(theta) * sum(lbbar_0)
@@ -1253,7 +1444,7 @@ static int u_backward_pull(bp_unrolled *u) {
         const unsigned gp = grid_for(u->V, kPullThreads * 2);
         cudaStream_t st = u->stream;
         int rc = BP_OK;
-        BP_CUDA(cudaMemsetAsync(u->epart, 0, sizeof(double) * gp * S * S, st));
+        BP_CUDA(cudaMemsetAsync(u->epart, 0, sizeof(double) * u->K * gp * S * S, st));
         // 4-8 states: the register cap, in resident blocks per SM, may be set
         // to 4, 5, 6 or 8 (BP_UBWD_PULL_MB; default pull_min_blocks)
         int mb = 0;
@@ -1265,6 +1456,9 @@ static int u_backward_pull(bp_unrolled *u) {
                         float *pout) -> int {
             const uint32_t *od = u->out_dst;
             const uint8_t *ot = u->out_tab;
+            if (u->K == (uint32_t)kPull2Tables)
+                return u_launch(k_u_bwd_pull2<S>, gp, kPullThreads, st, g, od, ot, mode, xn, pn, b_t, gin, gout, pout,
+                                u->epart);
             if constexpr (S >= 4) {
                 switch (mb) {
                 case 4: return u_launch(k_u_bwd_pull<S, 4>, gp, kPullThreads, st, g, od, ot, mode, xn, pn, b_t, gin,
@@ -1320,7 +1514,7 @@ static int u_backward_pull(bp_unrolled *u) {
         pn = u->pbv[pc];
         // the initial gather's edges (x = lb_0) and the priors' log-softmax
         if ((rc = step(2, u->ck_b, pn, nullptr, u->bbar[bc], u->gtheta_buf, nullptr))) return rc;
-        return u_launch(k_u_reduce_pair, S * S, 256u, st, (const double *)u->epart, gp, (uint32_t)(S * S),
+        return u_launch(k_u_reduce_pair, u->K * S * S, 256u, st, (const double *)u->epart, gp, (uint32_t)(S * S),
                         u->glogp_buf);
     }
 }
@@ -1569,8 +1763,8 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
     }
     std::vector<uint32_t> ofill(out_ptr.begin(), out_ptr.end() - 1);
     for (uint32_t e = 0; e < E; ++e) pos_out[pos_of[e]] = ofill[src[e]]++;
-    // one table and up to 8 states: the adjoint in pull form (BP_UBWD_PULL=0: the scatter form)
-    u->pull = K == 1 && S <= 8 && ubwd_env("BP_UBWD_PULL", 1, 0) == 1;
+    // one or two tables and up to 8 states: the adjoint in pull form (BP_UBWD_PULL=0: the scatter form)
+    u->pull = K <= (uint32_t)kPull2Tables && S <= 8 && ubwd_env("BP_UBWD_PULL", 1, 0) == 1;
     std::vector<uint32_t> odst;
     std::vector<uint8_t> otab;
     if (u->pull) {
@@ -1580,6 +1774,34 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
             const uint32_t q = pos_out[pos_of[e]];
             odst[q] = dst[e];
             otab[q] = tab[e];
+        }
+        // two tables: each node's out-edges by kind (table, then orientation)
+        auto kind = [](uint8_t t) { return 2u * (t & 0x7fu) + (t >> 7); };
+        std::vector<std::pair<uint8_t, uint32_t>> many;
+        for (uint32_t v = 0; K > 1 && v < V; ++v) {
+            const uint32_t a = out_ptr[v], b = out_ptr[v + 1];
+            if (b - a <= 32) {   // in place, by insertion
+                for (uint32_t q = a + 1; q < b; ++q) {
+                    const uint8_t t = otab[q];
+                    const uint32_t w = odst[q];
+                    uint32_t p = q;
+                    for (; p > a && kind(otab[p - 1]) > kind(t); --p) {
+                        otab[p] = otab[p - 1];
+                        odst[p] = odst[p - 1];
+                    }
+                    otab[p] = t;
+                    odst[p] = w;
+                }
+                continue;
+            }
+            many.clear();
+            for (uint32_t q = a; q < b; ++q) many.push_back({otab[q], odst[q]});
+            std::stable_sort(many.begin(), many.end(),
+                             [&](const auto &x, const auto &y) { return kind(x.first) < kind(y.first); });
+            for (uint32_t q = a; q < b; ++q) {
+                otab[q] = many[q - a].first;
+                odst[q] = many[q - a].second;
+            }
         }
     }
     // stored messages (see UMsgs): one per node and table orientation in use,
@@ -1637,7 +1859,7 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
               (u->ms.n == 0 || (alloc((void **)&u->in_msg, 4 * (size_t)E) &&
                                 alloc((void **)&u->msgs[0], sizeof(float) * VS * u->ms.n) &&
                                 alloc((void **)&u->msgs[1], sizeof(float) * VS * u->ms.n))) &&
-              (K == 1 || alloc((void **)&u->pbar, sizeof(float) * VS)) &&
+              (K == 1 || u->pull || alloc((void **)&u->pbar, sizeof(float) * VS)) &&
               alloc((void **)&u->theta_buf, sizeof(float) * VS) && alloc((void **)&u->gtheta_buf, sizeof(float) * VS) &&
               alloc((void **)&u->glogp_buf, sizeof(float) * K * S * S);
     if (!ok) {
