@@ -216,6 +216,34 @@ __global__ void k_gather_joint(const float *__restrict__ jin, uint32_t rs, uint6
     jout[p * (MS * MS) + k] = v;
 }
 
+// the same from dense 16-byte aligned tables (row stride MS, edge stride MS^2)
+// of an even state count: a thread per float4 (MS = 2: a table), so a table
+// is whole 16-byte loads and stores instead of a thread, two index loads and a
+// division per float.  400,000 tables of 8 x 8 with 2-8 states (a new tree of
+// 200,000 nodes): 137 -> 38 us; 4M tables of 2 x 2: 81 -> 49 us (ncu).
+template <int MS>
+__global__ void k_gather_joint_dense(const float4 *__restrict__ jin, const uint32_t *__restrict__ pos_edge,
+                                     const uint8_t *__restrict__ pos_dims, uint32_t E,
+                                     float4 *__restrict__ jout) {
+    constexpr uint32_t N = MS * MS / 4;   // float4s per table
+    static_assert(MS % 2 == 0, "tables of whole float4s");
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t p = t / N;
+    if (p >= E) return;
+    const uint32_t k = (uint32_t)(t % N);
+    float4 v = __ldcs(jin + (uint64_t)pos_edge[p] * N + k);
+    if (pos_dims) {   // mixed: zero beyond the two state counts
+        const uint32_t d = pos_dims[p], x = d & 15u, y = d >> 4;
+        float *f = reinterpret_cast<float *>(&v);
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) {
+            const uint32_t i = (4 * k + c) / MS, j = (4 * k + c) % MS;
+            if (i >= x || j >= y) f[c] = 0.0f;
+        }
+    }
+    jout[t] = v;
+}
+
 // beliefs [V][ld] <-> [V][MS] (zero beyond S_v)
 __global__ void k_beliefs_in(const float *__restrict__ in, uint32_t ld, uint32_t V, uint32_t ms,
                              const uint8_t *__restrict__ node_s, uint32_t uniform, const uint32_t *__restrict__ perm,
@@ -410,6 +438,14 @@ template <int MS, bool UNI>
 static int launch_gather_joint(bp_graph *g, const float *jin, uint32_t rs, uint64_t es, const uint32_t *dst_e) {
     uint64_t n = (uint64_t)g->E * MS * MS;
     if (n == 0) return BP_OK;
+    if constexpr (MS % 2 == 0) {
+        if (rs == MS && es == (uint64_t)MS * MS && ((uintptr_t)jin & 15u) == 0) {
+            k_gather_joint_dense<MS><<<grid_for(n / 4, 256), 256, 0, g->stream>>>(
+                (const float4 *)jin, g->pos_edge, g->pos_dims, g->E, (float4 *)g->joint);
+            BP_CUDA(cudaGetLastError());
+            return BP_OK;
+        }
+    }
     k_gather_joint<MS><<<grid_for(n, 256), 256, 0, g->stream>>>(jin, rs, es, g->pos_edge, g->in_src, dst_e,
                                                                  g->node_s, g->uniform, g->E, g->joint);
     BP_CUDA(cudaGetLastError());

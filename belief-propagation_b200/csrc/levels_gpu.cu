@@ -166,7 +166,7 @@ int tree_build_levels_gpu(bp_graph *g, uint32_t *levels_out, uint32_t *num_level
     BP_CUDA(pb.get(&iota, V));
     BP_CUDA(pb.get(&lv, V));
     BP_CUDA(pb.get(&cand, V));
-    BP_CUDA(pb.get(&counter, 2));
+    BP_CUDA(pb.get(&counter, 4));
     BP_CUDA(pb.get(&wave, V));
     BP_CUDA(pb.get(&starts, V));
     BP_CUDA(pb.get(&run_level, V));
@@ -238,16 +238,19 @@ int tree_build_levels_gpu(bp_graph *g, uint32_t *levels_out, uint32_t *num_level
     bool converged = V == 0;
     if (V) {
         BP_CUDA(cudaMemsetAsync(wave, 0, bytes, st));
-        for (uint32_t r = 0; r < kMaxWaveRounds; ++r) {
-            BP_CUDA(cudaMemsetAsync(counter, 0, sizeof(uint32_t), st));
-            k_wave_round<<<gv, 256, 0, st>>>(V, g->in_ptr, g->in_src, t.d_node_level, t.d_node_lidx, wave, counter);
+        // kRoundsPerCheck rounds between read-backs (a read-back costs about
+        // a round; rounds past the fixed point change nothing)
+        constexpr uint32_t kRoundsPerCheck = 4;
+        for (uint32_t r = 0; r < kMaxWaveRounds && !converged; r += kRoundsPerCheck) {
+            uint32_t changed[kRoundsPerCheck];
+            BP_CUDA(cudaMemsetAsync(counter, 0, sizeof changed, st));
+            for (uint32_t k = 0; k < kRoundsPerCheck; ++k)
+                k_wave_round<<<gv, 256, 0, st>>>(V, g->in_ptr, g->in_src, t.d_node_level, t.d_node_lidx, wave,
+                                                 counter + k);
             BP_CUDA(cudaGetLastError());
-            BP_CUDA(cudaMemcpyAsync(h_count, counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+            BP_CUDA(cudaMemcpyAsync(changed, counter, sizeof changed, cudaMemcpyDeviceToHost, st));
             BP_CUDA(cudaStreamSynchronize(st));
-            if (*h_count == 0) {
-                converged = true;
-                break;
-            }
+            converged = changed[kRoundsPerCheck - 1] == 0;
         }
     }
 

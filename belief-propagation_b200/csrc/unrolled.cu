@@ -186,6 +186,17 @@ struct UMsgs {
     uint8_t table[kUMaxMsgs];      // message c uses table sm[table[c]] (2k, or 2k + 1 transposed)
 };
 
+// in_msg from the positions' sources and tables
+__global__ void k_u_in_msg(uint32_t E, uint32_t V, const uint32_t *__restrict__ in_src,
+                           const uint8_t *__restrict__ pos_tab, const UMsgs ms, uint32_t *__restrict__ in_msg) {
+    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= E) return;
+    const uint32_t t = pos_tab[p], want = 2u * (t & 0x7fu) + (t >> 7);
+    uint32_t c = 0;
+    while (c + 1 < ms.n && ms.table[c] != want) ++c;
+    in_msg[p] = c * V + in_src[p];
+}
+
 // the messages of node v with log-state x
 template <int S>
 __device__ __forceinline__ void put_msgs(const UMsgs &ms, const float *sm, const float *x, uint32_t v, uint32_t V,
@@ -1336,6 +1347,15 @@ static int u_launch(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaS
     return BP_OK;
 }
 
+// Below this many nodes a launch of 256 threads per block and two nodes per
+// thread leaves SMs idle: 128 threads and one node.  Forward and backward,
+// T = 10: 128 x 128 grid of 4 states 268 -> 205 us, 201 x 201 of 5 (two tables)
+// 265 -> 210, 300 x 300 of 8 289 -> 241; 512 x 512 of 4 273 -> 283, so it keeps
+// the larger launch.
+constexpr uint32_t kUSmallNodes = 150000;
+static unsigned u_threads(uint32_t V) { return V < kUSmallNodes ? 128u : (unsigned)kUThreads; }
+static unsigned pull_nodes(uint32_t V) { return V < kUSmallNodes ? 1u : 2u; }
+
 // in-edges per batch of the adjoint kernel (BP_UBWD_BATCH=2|4, 1-4 states)
 // and nodes per thread (BP_UBWD_NPT=1|2); every choice gives the same results
 static int ubwd_env(const char *name, int dflt, int alt) {
@@ -1349,19 +1369,19 @@ template <int S>
 static int u_forward(bp_unrolled *u) {
     const UGraph g{u->V, u->K, u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables};
     const size_t VS = (size_t)u->V * S;
-    const unsigned gv = grid_for(u->V, kUThreads);
+    const unsigned ut = u_threads(u->V), gv = grid_for(u->V, ut);
     cudaStream_t st = u->stream;
     int rc, mc = 0;   // mc: the message buffer read next
     if (u->ms.n) {
-        if ((rc = u_launch(k_u_start_m<S>, gv, kUThreads, st, g, u->ms, (const float *)u->theta_buf, u->ck_b, u->msgs[0])))
+        if ((rc = u_launch(k_u_start_m<S>, gv, ut, st, g, u->ms, (const float *)u->theta_buf, u->ck_b, u->msgs[0])))
             return rc;
-        if ((rc = u_launch(k_u_iter_m<S, true>, gv, kUThreads, st, g, u->ms, (const float *)u->ck_b,
+        if ((rc = u_launch(k_u_iter_m<S, true>, gv, ut, st, g, u->ms, (const float *)u->ck_b,
                            (const float *)u->msgs[0], (float *)nullptr, u->ck_q, u->msgs[1])))
             return rc;
         mc = 1;
     } else {
-        if ((rc = u_launch(k_u_logsoftmax<S>, gv, kUThreads, st, u->V, (const float *)u->theta_buf, u->ck_b))) return rc;
-        if ((rc = u_launch(k_u_gather_q<S>, gv, kUThreads, st, g, (const float *)u->ck_b, (const float *)u->ck_b,
+        if ((rc = u_launch(k_u_logsoftmax<S>, gv, ut, st, u->V, (const float *)u->theta_buf, u->ck_b))) return rc;
+        if ((rc = u_launch(k_u_gather_q<S>, gv, ut, st, g, (const float *)u->ck_b, (const float *)u->ck_b,
                            u->ck_q)))
             return rc;
     }
@@ -1385,14 +1405,14 @@ static int u_forward(bp_unrolled *u) {
         float *qo = (t == u->T) ? u->pp_q + (t & 1) * VS : loc_q(t);
         if (u->ms.n) {
             const bool last = t == u->T;
-            if ((rc = u_launch(k_u_iter_m<S, false>, gv, kUThreads, st, g, u->ms, (const float *)loc_b(t - 1),
+            if ((rc = u_launch(k_u_iter_m<S, false>, gv, ut, st, g, u->ms, (const float *)loc_b(t - 1),
                                (const float *)u->msgs[mc], bo, last ? (float *)nullptr : qo,
                                last ? (float *)nullptr : u->msgs[mc ^ 1])))
                 return rc;
             mc ^= 1;
             continue;
         }
-        if ((rc = u_launch(k_u_iter<S>, gv, kUThreads, st, g, (const float *)loc_b(t - 1), (const float *)loc_q(t - 1),
+        if ((rc = u_launch(k_u_iter<S>, gv, ut, st, g, (const float *)loc_b(t - 1), (const float *)loc_q(t - 1),
                            bo, qo)))
             return rc;
     }
@@ -1405,7 +1425,7 @@ static int u_forward(bp_unrolled *u) {
 template <int S>
 static int u_recompute(bp_unrolled *u, const UGraph &g, uint32_t s) {
     const size_t VS = (size_t)u->V * S;
-    const unsigned gv = grid_for(u->V, kUThreads);
+    const unsigned ut = u_threads(u->V), gv = grid_for(u->V, ut);
     const uint32_t t0 = s * u->ck, t_end = std::min(t0 + u->ck, u->T);
     const float *ckb = u->ck_b + (size_t)s * VS, *ckq = u->ck_q + (size_t)s * VS;
     float *sb = u->seg_b + (size_t)(s & 1u) * u->ck * VS, *sq = u->seg_q + (size_t)(s & 1u) * u->ck * VS;
@@ -1414,13 +1434,13 @@ static int u_recompute(bp_unrolled *u, const UGraph &g, uint32_t s) {
         const float *bi = (j == 1) ? ckb : sb + (j - 1) * VS;
         const float *qi = (j == 1) ? ckq : sq + (j - 1) * VS;
         if (u->ms.n) {
-            if (j == 1 && (rc = u_launch(k_u_send_m<S>, gv, kUThreads, u->side, g, u->ms, ckq, u->msgs[0]))) return rc;
+            if (j == 1 && (rc = u_launch(k_u_send_m<S>, gv, ut, u->side, g, u->ms, ckq, u->msgs[0]))) return rc;
             const bool last = j + 1 + t0 >= t_end;
-            rc = u_launch(k_u_iter_m<S, false>, gv, kUThreads, u->side, g, u->ms, bi, (const float *)u->msgs[mc],
+            rc = u_launch(k_u_iter_m<S, false>, gv, ut, u->side, g, u->ms, bi, (const float *)u->msgs[mc],
                           sb + j * VS, sq + j * VS, last ? (float *)nullptr : u->msgs[mc ^ 1]);
             mc ^= 1;
         } else {
-            rc = u_launch(k_u_iter<S>, gv, kUThreads, u->side, g, bi, qi, sb + j * VS, sq + j * VS);
+            rc = u_launch(k_u_iter<S>, gv, ut, u->side, g, bi, qi, sb + j * VS, sq + j * VS);
         }
         if (rc) return rc;
     }
@@ -1440,8 +1460,8 @@ static int u_backward_pull(bp_unrolled *u) {
     } else {
         const UGraph g{u->V, u->K, u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables};
         const size_t VS = (size_t)u->V * S;
-        const unsigned gv = grid_for(u->V, kUThreads);
-        const unsigned gp = grid_for(u->V, kPullThreads * 2);
+        const unsigned ut = u_threads(u->V), gv = grid_for(u->V, ut);
+        const unsigned gp = grid_for(u->V, kPullThreads * pull_nodes(u->V));
         cudaStream_t st = u->stream;
         int rc = BP_OK;
         BP_CUDA(cudaMemsetAsync(u->epart, 0, sizeof(double) * u->K * gp * S * S, st));
@@ -1523,7 +1543,7 @@ template <int S>
 static int u_backward(bp_unrolled *u) {
     const UGraph g{u->V, u->K, u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables};
     const size_t VS = (size_t)u->V * S;
-    const unsigned gv = grid_for(u->V, kUThreads);
+    const unsigned ut = u_threads(u->V), gv = grid_for(u->V, ut);
     constexpr int BT = bwd_threads<S>();
     // one table and 5..8 states: the table adjoint on the tensor cores
     const bool mma = S >= 5 && S <= 8 && u->K == 1;
@@ -1607,7 +1627,7 @@ static int u_backward(bp_unrolled *u) {
     const float *b0 = u->ck_b;
     if ((rc = adjoint(1, b0, nullptr, u->bbar[bc], xc_next, u->bbar[bc ^ 1], u->xc[rn], pbar))) return rc;
     if ((rc = pair_grads(b0))) return rc;
-    if ((rc = u_launch(k_u_bwd_src<S>, gv, kUThreads, st, g, (const float *)u->xc[rn], (const float *)u->bbar[bc ^ 1],
+    if ((rc = u_launch(k_u_bwd_src<S>, gv, ut, st, g, (const float *)u->xc[rn], (const float *)u->bbar[bc ^ 1],
                        b0, u->gtheta_buf)))
         return rc;
     return u_launch(k_u_reduce_pair, u->K * S * S, 256u, st, (const double *)u->epart, gb, (uint32_t)(S * S),
@@ -1619,7 +1639,7 @@ static void u_free(bp_unrolled *u) {
     void *ptrs[] = {u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables, u->ck_b, u->ck_q,
                     u->seg_b, u->seg_q, u->pp_b, u->pp_q, u->bT, u->bbar[0], u->bbar[1], u->xc[0],
                     u->xc[1], u->epart, u->theta_buf, u->gtheta_buf, u->glogp_buf, u->pbar, u->out_dst,
-                    u->out_tab, u->pbv[0], u->pbv[1], u->in_msg, u->msgs[0], u->msgs[1]};
+                    u->out_tab, u->pbv[0], u->pbv[1], u->in_msg, u->msgs[0]};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (u->fwd_exec) cudaGraphExecDestroy(u->fwd_exec);
@@ -1728,9 +1748,11 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
     if (K < 1 || K > kUMaxTables) return set_error(BP_ERR_SHAPE, "num_tables %u not in [1, %u]", K, kUMaxTables);
     if (V == 0 || T == 0) return set_error(BP_ERR_SHAPE, "need nodes and at least one iteration");
     if (ck == 0) ck = 1;
+    uint8_t used[256] = {};   // table ids in use, transposed or not
     for (uint32_t e = 0; e < E; ++e) {
         if (src[e] >= V || dst[e] >= V) return set_error(BP_ERR_INVALID, "edge %u endpoint out of range", e);
         if ((tab[e] & 0x7fu) >= K) return set_error(BP_ERR_INVALID, "edge %u table %u >= %u", e, tab[e] & 0x7f, K);
+        used[tab[e]] = 1;
     }
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return set_error(BP_ERR_NO_DEVICE, "no CUDA device");
@@ -1809,31 +1831,15 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
     // a grid, four messages against four edges: 560 us stored, 554 us
     // recomputed per edge on the 201 x 201 grid of 5 states; BP_UNROLLED_MSG=0:
     // never, 1: always)
-    std::vector<uint32_t> in_msg;
     {
-        uint8_t index[256];
-        memset(index, 0xff, sizeof index);
         uint32_t n = 0;
-        bool fits = true;
-        for (uint32_t p = 0; p < E && fits; ++p) {
-            const uint8_t t = ptab[p] & 0x7fu, o = (ptab[p] & 0x80u) ? 1 : 0;
-            uint8_t &at = index[2 * t + o];
-            if (at != 0xff) continue;
-            fits = n < kUMaxMsgs;
-            if (fits) {
-                u->ms.table[n] = (uint8_t)(2 * t + o);
-                at = (uint8_t)n++;
-            }
-        }
+        for (uint32_t t = 0; t < 256; ++t) n += used[t];   // at most 2 K <= kUMaxMsgs
         const char *env = getenv("BP_UNROLLED_MSG");
         bool use = (uint64_t)n * V <= (uint64_t)E - E / 4;
         if (env && (env[0] == '0' || env[0] == '1')) use = env[0] == '1';
-        if (use && fits && E && (uint64_t)n * V <= 0xffffffffull) {
-            u->ms.n = n;
-            in_msg.resize(E);
-            for (uint32_t p = 0; p < E; ++p)
-                in_msg[p] = index[2 * (ptab[p] & 0x7fu) + ((ptab[p] & 0x80u) ? 1 : 0)] * V + in_src[p];
-        }
+        if (use && E && (uint64_t)n * V <= 0xffffffffull)
+            for (uint32_t t = 0; t < 256; ++t)
+                if (used[t]) u->ms.table[u->ms.n++] = (uint8_t)(2 * (t & 0x7fu) + (t >> 7));
     }
     const size_t VS = (size_t)V * S;
     u->nblk = grid_for(V, 64);   // partial slots for the smallest backward block
@@ -1841,7 +1847,7 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
         return cudaMalloc(p, bytes ? bytes : 16) == cudaSuccess;
     };
     bool ok = alloc((void **)&u->in_ptr, sizeof(uint32_t) * (V + 1)) && alloc((void **)&u->in_src, 4 * (size_t)E) &&
-              alloc((void **)&u->out_ptr, sizeof(uint32_t) * (V + 1)) && alloc((void **)&u->pos_out, 4 * (size_t)E) &&
+              alloc((void **)&u->out_ptr, sizeof(uint32_t) * (V + 1)) && (u->pull || alloc((void **)&u->pos_out, 4 * (size_t)E)) &&
               alloc((void **)&u->pos_tab, (size_t)E) && alloc((void **)&u->tables, sizeof(float) * K * S * S) &&
               alloc((void **)&u->ck_b, sizeof(float) * VS * u->nck) &&
               alloc((void **)&u->ck_q, sizeof(float) * VS * u->nck) &&
@@ -1857,8 +1863,7 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
                             alloc((void **)&u->pbv[1], sizeof(float) * VS))) &&
               alloc((void **)&u->epart, sizeof(double) * K * u->nblk * S * S) &&
               (u->ms.n == 0 || (alloc((void **)&u->in_msg, 4 * (size_t)E) &&
-                                alloc((void **)&u->msgs[0], sizeof(float) * VS * u->ms.n) &&
-                                alloc((void **)&u->msgs[1], sizeof(float) * VS * u->ms.n))) &&
+                                alloc((void **)&u->msgs[0], sizeof(float) * (2 * VS * u->ms.n + 4)))) &&
               (K == 1 || u->pull || alloc((void **)&u->pbar, sizeof(float) * VS)) &&
               alloc((void **)&u->theta_buf, sizeof(float) * VS) && alloc((void **)&u->gtheta_buf, sizeof(float) * VS) &&
               alloc((void **)&u->glogp_buf, sizeof(float) * K * S * S);
@@ -1867,13 +1872,15 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
         return set_error(BP_ERR_NOMEM, "device allocation failed for the unrolled graph");
     }
     u->ms.in_msg = u->in_msg;
-    if (u->ms.n) cudaMemcpyAsync(u->in_msg, in_msg.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
+    if (u->ms.n) u->msgs[1] = u->msgs[0] + ((VS * u->ms.n + 3) & ~(size_t)3);   // 16-byte aligned
     cudaMemcpyAsync(u->in_ptr, in_ptr.data(), 4 * (V + 1), cudaMemcpyHostToDevice, u->stream);
     cudaMemcpyAsync(u->out_ptr, out_ptr.data(), 4 * (V + 1), cudaMemcpyHostToDevice, u->stream);
     if (E) {
         cudaMemcpyAsync(u->in_src, in_src.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
-        cudaMemcpyAsync(u->pos_out, pos_out.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
+        if (!u->pull) cudaMemcpyAsync(u->pos_out, pos_out.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
         cudaMemcpyAsync(u->pos_tab, ptab.data(), (size_t)E, cudaMemcpyHostToDevice, u->stream);
+        if (u->ms.n)
+            k_u_in_msg<<<grid_for(E, 256), 256, 0, u->stream>>>(E, V, u->in_src, u->pos_tab, u->ms, u->in_msg);
         if (u->pull) {
             cudaMemcpyAsync(u->out_dst, odst.data(), 4 * (size_t)E, cudaMemcpyHostToDevice, u->stream);
             cudaMemcpyAsync(u->out_tab, otab.data(), (size_t)E, cudaMemcpyHostToDevice, u->stream);
