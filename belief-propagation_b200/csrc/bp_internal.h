@@ -61,9 +61,8 @@ struct LoopyCtl {
     float delta_f, prev_f;
     uint32_t pad0;
     double delta_d, prev_d;
-    // grid barrier of the fused (one-launch) loop: arrivals, generation, and
-    // a flag a block sets when its bounded wait ran out
-    uint32_t bar_count, bar_gen, bar_fail;
+    // set by a block of a one-launch loop whose bounded barrier wait ran out
+    uint32_t bar_fail;
     // test hook of that bounded wait (BP_DEBUG_BARRIER_SKIP): block
     // bar_skip - 1 does not arrive at the first barrier, so the others' waits
     // run out; 0 = off
@@ -182,9 +181,10 @@ struct bp_graph {
     struct LoopPlan {
         int state = 0;                   // 0 not planned yet
         uint32_t grid = 0, smem = 0;     // no grid: the graph has too many tiles
-        bool wide = false;
+        bool wide = false, fused = false;
     } loop_plan[2];
     uint64_t *loop_flags = nullptr;      // [grid] its barrier's flags (device)
+    uint32_t *grid_bar = nullptr;        // the one-launch loops' grid barrier (device)
     uint64_t loop_runs = 0;              // runs so far: every run's flags lie above the last one's
 
     // cached CUDA graphs of the iteration loop

@@ -46,6 +46,7 @@ struct EdgeArgs {
     const uint32_t *run_len;
     const uint8_t *run_s;
     uint32_t nruns;
+    uint32_t *bar;       // the graph's grid barrier
 };
 
 constexpr int kEdgeThreads = 256;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
     __shared__ uint32_t s_fail;
 
     LoopyCtl *ctl = a.ctl;
+    GridBar gb(ctl, a.bar);
     if (threadIdx.x == 0) {
         s_ctl = *ctl;
         s_fail = 0;
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
     // the copied part of the padded array, in floats and odd bytes
     const uint64_t nbytes = (uint64_t)a.E * 10u, nfull = nbytes / 4u;
     const uint32_t keep = 0xffffffffu << (8u * (uint32_t)(nbytes & 3u));
-    uint32_t gen = 0;
+    bool narrow = true;   // narrowing has decided every check that needed it so far
     while (!s_ctl.done) {
         const uint32_t it = s_ctl.it, ce = s_ctl.check_every;
         const bool acc = s_ctl.acc_edge != 0;
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
         const double t = block_sum<NT>(dsum, red);
         double *part = a.partials + (size_t)(it & 1u) * gridDim.x;
         if (threadIdx.x == 0) part[blockIdx.x] = t;
-        if (!grid_barrier(ctl, gen, &s_fail)) break;
+        if (!grid_barrier(gb, &s_fail)) break;
 
         // the nodes: combine, in edge order
         const uint32_t i_batch = (it / 10u) * 10u;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
             SerialCheck x = serial_check(&s_ctl, broadcast_sum(tot));
             if (x.d < 0 && !grid_serial_form<NT>(x, a.absdiff + (size_t)x.cb * s_ctl.ad_stride,
                                                  a.absdiff + (size_t)s_ctl.prev_buf * s_ctl.ad_stride, s_ctl.n_terms,
-                                                 s_ctl.tol, ctl, a.partials, gen, &s_fail, red))
+                                                 s_ctl.tol, ctl, a.partials, gb, &s_fail, red, narrow))
                 break;
             __syncthreads();   // every thread has read s_ctl
             if (threadIdx.x == 0) serial_commit(&s_ctl, x);
@@ -234,8 +236,8 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_loop(const EdgeArgs a) {
         }
         __syncthreads();
         // the next iteration's sends read the beliefs combined here
-        if (!s_ctl.done && !grid_barrier(ctl, gen, &s_fail)) break;
+        if (!s_ctl.done && !grid_barrier(gb, &s_fail)) break;
     }
-    if (SER && !s_fail && s_ctl.done) grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red);
+    if (SER && !s_fail && s_ctl.done) grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gb, &s_fail, red);
     if (first == 0 && !s_fail) publish_ctl(ctl, s_ctl);
 }

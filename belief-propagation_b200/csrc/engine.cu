@@ -621,7 +621,7 @@ static void free_graph(bp_graph *g) {
     void *ptrs[] = {g->new_to_old, g->in_ptr, g->in_src, g->pos_edge, g->edge_pos, g->pos_dims, g->node_s, g->joint,
                     g->belief, g->msg[0], g->msg[1], g->q[0], g->q[1], g->out_ptr, g->out_pos,
                     g->out_dst, g->pos_dst, g->partials, g->absdiff, g->ctl, g->visited, g->staging,
-                    g->run_len, g->run_s, g->loop_flags};
+                    g->run_len, g->run_s, g->loop_flags, g->grid_bar};
     for (void *p : ptrs)
         if (p) cudaFreeAsync(p, g->stream);
     split_free(g);

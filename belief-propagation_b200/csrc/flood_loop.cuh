@@ -55,6 +55,7 @@ template <int MS> constexpr uint32_t loop_table_stride() {
 
 struct LoopArgs {
     FloodArgs f;
+    uint32_t *bar;       // the graph's grid barrier
     uint64_t *flags;     // [G] one per block, rising over the runs of a graph
     uint64_t run_tag;    // above every tag of earlier runs; + iteration + 1
     uint32_t smem;       // dynamic shared memory per block, bytes
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
     const FloodArgs &a = la.f;
     LoopyCtl *ctl = a.ctl;
     const uint32_t tid = threadIdx.x, G = gridDim.x;
+    GridBar gb(ctl, la.bar);
     if (tid == 0) {
         s_ctl = *ctl;
         s_fail = 0;
@@ -247,9 +249,9 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
     double d_d = 0.0, dlo = 0.0, dhi = 0.0, p_d = s_ctl.prev_d, plo = s_ctl.plo, phi = s_ctl.phi;
     float d_f = 0.0f, p_f = s_ctl.prev_f;
     bool d_exact = true, p_exact = true, stop = false;
-    uint32_t d_buf = 0, p_buf = 0, sums = 0, it = 0;
+    uint32_t d_buf = 0, p_buf = 0, sums = 0, refines = 0, it = 0;
+    bool narrow = true, d_ref = false, p_ref = false;   // intervals narrowed
     double tot = 0.0;   // a lone tile's sum needs no exchange
-    uint32_t gen = 0;
     uint32_t cur = 0;   // buffer of the latest messages
     bool ok = true;
     for (uint32_t t = 0;; ++t) {
@@ -308,6 +310,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                     plo = dlo;
                     phi = dhi;
                     p_exact = d_exact;
+                    p_ref = d_ref;
                     p_buf = d_buf;
                 }
                 d_d = tot;
@@ -318,7 +321,8 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                     x.plo = plo;
                     x.phi = phi;
                     x.p_exact = p_exact;
-                    x.p_ref = x.s_exact = x.s_ref = x.p_new = false;
+                    x.p_ref = p_ref;
+                    x.s_exact = x.s_ref = x.p_new = false;
                     x.sums = x.refines = 0;
                     x.cb = d_buf = check_index(t - 1, ce) % 3u;
                     x.s = d_f;
@@ -333,19 +337,23 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
                             if (!p_exact) write_terms(tp, ms + (size_t)p2 * ne * MS, ms + (size_t)p1 * ne * MS);
                         }
                         if (solo) __syncthreads();
-                        else if (ce <= 1) ok = grid_barrier(ctl, gen, &s_fail);
-                        ok = ok && grid_serial_form<NT>(x, tc, tp, s_ctl.n_terms, tol, ctl, a.partials, gen, &s_fail, red_b);
+                        else if (ce <= 1) ok = grid_barrier(gb, &s_fail);
+                        ok = ok && grid_serial_form<NT>(x, tc, tp, s_ctl.n_terms, tol, ctl, a.partials, gb, &s_fail,
+                                                         red_b, narrow);
+                        refines += x.refines;
                         if (!ok) break;
-                        if (!p_exact) p_f = (float)x.plo;
+                        if (x.p_exact) p_f = (float)x.plo;
                         plo = x.plo;
                         phi = x.phi;
                         p_exact = x.p_exact;
+                        p_ref = x.p_ref;
                         sums += x.sums;
                     }
                     d_f = x.s;
                     dlo = x.lo;
                     dhi = x.hi;
                     d_exact = x.s_exact;
+                    d_ref = x.s_ref;
                     stop = x.d == 1;
                 } else {
                     stop = tot < (double)tol || fabs(tot - p_d) < (double)tol;
@@ -438,7 +446,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
         else if (tid == 0) a.partials[(size_t)(t & 1u) * G + blockIdx.x] = warps_total<NW>(red);
         if (solo) __syncthreads();
         else if (G <= kFlagBlocks) ok = flag_barrier(ctl, la.flags, la.run_tag + t + 1u, skip, t == 0, wait_ms, &s_fail);
-        else ok = grid_barrier(ctl, gen, &s_fail);
+        else ok = grid_barrier(gb, &s_fail);
         if (!ok) break;
     }
 
@@ -471,6 +479,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
             s_ctl.cur_buf = d_buf;
             s_ctl.prev_buf = p_buf;
             s_ctl.serial_sums = sums;
+            s_ctl.serial_refines = refines;
         }
     }
     __syncthreads();
@@ -487,8 +496,8 @@ __global__ void __launch_bounds__(flood_nt<MS>(), loop_min_blocks<MS, WIDE>()) k
         }
         if (!s_ctl.delta_exact || !s_ctl.prev_exact) {
             if (solo) __syncthreads();
-            else ok = grid_barrier(ctl, gen, &s_fail);
-            ok = ok && grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gen, &s_fail, red_b);
+            else ok = grid_barrier(gb, &s_fail);
+            ok = ok && grid_serial_final<NT>(s_ctl, ctl, a.partials, a.absdiff, gb, &s_fail, red_b);
         }
     }
     if (ok && resident) {

@@ -791,37 +791,75 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood(const FloodArgs a,
 // the next iteration's while others may still read this one's.
 constexpr uint64_t kBarrierWaitNs = 2000000000ull;   // 2 s
 
+// More than kBarFlat blocks are counted on two levels, kBarSubs counters of
+// every 32nd block and a root, each on a line of its own and apart from the
+// generation the waiters poll.  An iteration of 150,000 nodes of 2 states
+// (1,172 blocks) took 16.2 us with one counter beside the generation, 15.1
+// with two levels; of 50,000 nodes (391 blocks) 10.5 and 11.0, the second
+// level's atomic being the longer way there.  The generation rises over the runs of a graph; a run
+// starts from the value it finds, which cannot move before its own last block
+// arrives.  The buffer is the graph's (bp_graph::grid_bar), zeroed when made and
+// after a run that gave up.
+//
 // The wait is bounded by kBarrierWaitNs, or by c->wait_ms when the host set
 // one.  Test hook: with c->bar_skip == blockIdx.x + 1 this block does not
-// arrive at the first barrier (gen 0) and goes on, so the other blocks' waits
+// arrive at the run's first barrier and goes on, so the other blocks' waits
 // run out and the run ends with bar_fail; every later wait of this block is
 // bounded the same way, so the launch still ends.
-__device__ __forceinline__ bool grid_barrier(LoopyCtl *c, uint32_t &gen, uint32_t *s_fail) {
+constexpr uint32_t kBarSubs = 32, kBarStride = 32;   // counters, u32s between them
+constexpr uint32_t kBarFlat = 640;                   // up to here one counter
+constexpr uint32_t kBarWords = (kBarSubs + 2) * kBarStride;
+
+struct GridBar {
+    LoopyCtl *c;
+    uint32_t *bar;   // [root][kBarSubs counters][generation]
+    uint32_t gen, first;
+
+    // one thread's view; every thread of the block keeps the same one
+    __device__ __forceinline__ GridBar(LoopyCtl *c_, uint32_t *b) : c(c_), bar(b) {
+        gen = first = *(volatile uint32_t *)(bar + (kBarSubs + 1) * kBarStride);
+    }
+};
+
+__device__ __forceinline__ bool grid_barrier(GridBar &gb, uint32_t *s_fail) {
     __syncthreads();
-    if (threadIdx.x == 0 && !*s_fail && !(gen == 0 && c->bar_skip == blockIdx.x + 1u)) {
-        const uint32_t g0 = gen;
-        const uint64_t limit = c->wait_ms ? (uint64_t)c->wait_ms * 1000000ull : kBarrierWaitNs;
-        __threadfence();
-        if (atomicAdd(&c->bar_count, 1u) == gridDim.x - 1) {
-            c->bar_count = 0;   // untouched until the generation moves
-            __threadfence();
-            atomicExch(&c->bar_gen, g0 + 1u);
+    LoopyCtl *c = gb.c;
+    if (threadIdx.x == 0 && !*(volatile uint32_t *)s_fail && !(gb.gen == gb.first && c->bar_skip == blockIdx.x + 1u)) {
+        uint32_t *root = gb.bar, *gen = gb.bar + (kBarSubs + 1) * kBarStride;
+        const uint32_t j = blockIdx.x % kBarSubs, G = gridDim.x;
+        uint32_t *sub = gb.bar + (1 + j) * kBarStride;
+        fence_acq_rel();
+        bool last = false;
+        if (G <= kBarFlat) {
+            last = atomicAdd(root, 1u) == G - 1;
+        } else if (atomicAdd(sub, 1u) == (G - j + kBarSubs - 1) / kBarSubs - 1) {
+            *(volatile uint32_t *)sub = 0;   // untouched until the generation moves
+            fence_acq_rel();
+            last = atomicAdd(root, 1u) == min(G, kBarSubs) - 1;
+        }
+        if (last) {
+            *(volatile uint32_t *)root = 0;
+            fence_acq_rel();
+            atomicExch(gen, gb.gen + 1u);
         } else {
-            const uint64_t t0 = global_ns();
-            while (*(volatile uint32_t *)&c->bar_gen == g0) {
-                if (global_ns() - t0 > limit) {
+            const uint64_t limit = c->wait_ms ? (uint64_t)c->wait_ms * 1000000ull : kBarrierWaitNs;
+            uint64_t t0 = 0;
+            for (uint32_t spin = 0; (int32_t)(*(volatile uint32_t *)gen - gb.gen) <= 0; ++spin) {
+                if ((spin & 255u) != 255u) continue;
+                const uint64_t t = global_ns();
+                if (t0 == 0) t0 = t;
+                if (t - t0 > limit) {
                     *s_fail = 1;
                     atomicExch(&c->bar_fail, 1u);
                     break;
                 }
-                __nanosleep(64);
             }
         }
-        __threadfence();
+        fence_acq_rel();
     }
     __syncthreads();
-    gen += 1;
-    return *s_fail == 0;
+    gb.gen += 1;
+    return *(volatile uint32_t *)s_fail == 0;
 }
 
 // the run's outcome from a block's copy of the control block (one thread)
@@ -852,6 +890,50 @@ __device__ __forceinline__ void publish_ctl(LoopyCtl *ctl, const LoopyCtl &sc) {
 
 #include "serial_grid.cuh"
 #include "flood_loop.cuh"
+
+// Every iteration of a run with the f64 delta in one cooperative launch, the
+// tile's data read from memory as k_flood reads it: see loop_plan for where it
+// is taken instead of k_flood_loop and of a launch per iteration.
+template <int MS, bool UNI, int FU, int MB = flood_min_blocks<MS, FU>()>
+__global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood_fused(const FloodArgs a, uint32_t *bar) {
+    constexpr int NT = flood_nt<MS>();
+    constexpr uint32_t EMAX = flood_smem_floats<MS>() / MS;
+    __shared__ __align__(16) float sm[EMAX * MS];
+    __shared__ double red[NT / 32];
+    __shared__ LoopyCtl s_ctl;
+    __shared__ uint32_t s_fail;
+
+    LoopyCtl *ctl = a.ctl;
+    GridBar gb(ctl, bar);
+    if (threadIdx.x == 0) {
+        s_ctl = *ctl;
+        s_fail = 0;
+    }
+    __syncthreads();
+    const uint64_t keep = l2_evict_last_policy();
+    while (!s_ctl.done) {
+        const uint32_t it = s_ctl.it, ce = s_ctl.check_every;
+        const bool want = (ce <= 1) || ((it + 1) % ce == 0);
+        const int mp = (int)((s_ctl.msg_parity0 + it) & 1u), qp = (int)((s_ctl.q_parity0 + it) & 1u);
+        const float *__restrict__ m_old = mp ? a.msg1 : a.msg0;
+        float *__restrict__ m_new = mp ? a.msg0 : a.msg1;
+        const float *__restrict__ q_in = qp ? a.q1 : a.q0;
+        float *__restrict__ q_out = qp ? a.q0 : a.q1;
+        double dsum = 0.0;
+        flood_tile<MS, UNI, FU>(a, blockIdx.x, want, nullptr, m_old, m_new, q_in, q_out, keep, sm, dsum);
+        __syncthreads();
+        const double t = block_sum<NT>(dsum, red);
+        double *part = a.partials + (size_t)(it & 1u) * gridDim.x;
+        if (threadIdx.x == 0) part[blockIdx.x] = t;
+        if (!grid_barrier(gb, &s_fail)) break;
+        double acc = 0.0;
+        for (uint32_t k = threadIdx.x; k < gridDim.x; k += NT) acc += __ldcg(part + k);
+        const double tot = block_sum<NT>(acc, red);
+        if (threadIdx.x == 0) finalize(&s_ctl, want, (float)tot, tot);
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !s_fail) publish_ctl(ctl, s_ctl);
+}
 
 // Staged form of k_flood for uniform 2-state graphs (the layout is written
 // for 2 or 4 states; 4-state tables do not leave room for two stages of a
@@ -1410,12 +1492,19 @@ static int ensure_absdiff(bp_graph *g) {
     return BP_OK;
 }
 
-// the one-launch loop's barrier flags, one per block; zero below every run's tag
+// the one-launch loops' barrier flags, one per block (zero: below every run's
+// tag), and grid barrier
 static int ensure_loop_flags(bp_graph *g, uint32_t n) {
-    if (g->loop_flags) return BP_OK;
-    int st = dev_alloc(g, (void **)&g->loop_flags, sizeof(uint64_t) * n);
-    if (st) return st;
-    BP_CUDA(cudaMemsetAsync(g->loop_flags, 0, sizeof(uint64_t) * n, g->stream));
+    if (n && !g->loop_flags) {
+        int st = dev_alloc(g, (void **)&g->loop_flags, sizeof(uint64_t) * n);
+        if (st) return st;
+        BP_CUDA(cudaMemsetAsync(g->loop_flags, 0, sizeof(uint64_t) * n, g->stream));
+    }
+    if (!g->grid_bar) {
+        int st = dev_alloc(g, (void **)&g->grid_bar, sizeof(uint32_t) * kBarWords);
+        if (st) return st;
+        BP_CUDA(cudaMemsetAsync(g->grid_bar, 0, sizeof(uint32_t) * kBarWords, g->stream));
+    }
     return BP_OK;
 }
 
@@ -1525,6 +1614,7 @@ static EdgeArgs edge_args(bp_graph *g) {
     a.run_len = g->run_len;
     a.run_s = g->run_s;
     a.nruns = g->nruns;
+    a.bar = g->grid_bar;
     return a;
 }
 
@@ -1982,12 +2072,32 @@ static int loop_plan(bp_graph *g, bool serial) {
     BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint32_t tiles = grid_for(g->V, flood_nt<MS>()), per_sm = (tiles + sms - 1) / sms;
     int st = BP_OK;
-    if (per_sm <= (uint32_t)loop_min_blocks<MS, true>())
-        st = serial ? loop_plan_of<MS, UNI, true, true>(g, tiles, per_sm, &p)
-                    : loop_plan_of<MS, UNI, false, true>(g, tiles, per_sm, &p);
-    else if (per_sm <= (uint32_t)loop_min_blocks<MS, false>())
-        st = serial ? loop_plan_of<MS, UNI, true, false>(g, tiles, per_sm, &p)
-                    : loop_plan_of<MS, UNI, false, false>(g, tiles, per_sm, &p);
+    if (serial) {
+        if (per_sm <= (uint32_t)loop_min_blocks<MS, true>())
+            st = loop_plan_of<MS, UNI, true, true>(g, tiles, per_sm, &p);
+        else if (per_sm <= (uint32_t)loop_min_blocks<MS, false>())
+            st = loop_plan_of<MS, UNI, true, false>(g, tiles, per_sm, &p);
+    } else {
+        // A tile kept on chip (k_flood_loop) pays while it has an SM and its
+        // L2 share nearly to itself, and to a full set of SMs where the tables
+        // are large.  60 iterations, us, on chip / from memory / launches:
+        // 9,000 nodes of 2, 7, 10 states 472, 618, 625 / 576, 782, 929 / 651,
+        // 948, 1250; 37,000 nodes 706, 970, 2654 / 592, 1046, 1332 / 694,
+        // 1658, 1437; 25,000 nodes (98 tiles) of 3 states 667 / 560 / 656.
+        // Where the tiles are not all resident a launch per iteration is taken
+        // (level with the cooperative launch at the last sizes that are).
+        if (tiles <= sms / 2u || (MS >= 7 && tiles <= (uint32_t)sms)) {
+            st = loop_plan_of<MS, UNI, false, true>(g, tiles, per_sm, &p);
+        } else {
+            int bps = 0;
+            BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_flood_fused<MS, UNI, flood_unroll<MS>()>,
+                                                                  flood_nt<MS>(), 0));
+            if ((int)per_sm <= bps) {
+                p.grid = tiles;
+                p.fused = true;
+            }
+        }
+    }
     p.state = st ? 0 : 1;
     return st;
 }
@@ -1997,14 +2107,21 @@ static int launch_loop(bp_graph *g, bool serial) {
     const bp_graph::LoopPlan &p = g->loop_plan[serial ? 1 : 0];
     LoopArgs a;
     a.f = flood_args(g);
+    if (p.fused) {
+        void *args[] = {(void *)&a.f, (void *)&g->grid_bar};
+        BP_CUDA(cudaLaunchCooperativeKernel((const void *)k_flood_fused<MS, UNI, flood_unroll<MS>()>, dim3(p.grid),
+                                            dim3(flood_nt<MS>()), args, 0, g->stream));
+        return BP_OK;
+    }
     a.flags = g->loop_flags;
+    a.bar = g->grid_bar;
     a.run_tag = ++g->loop_runs << 32;
     a.smem = p.smem;
     const void *fn;
     if (p.wide)
         fn = serial ? (const void *)k_flood_loop<MS, UNI, true, true> : (const void *)k_flood_loop<MS, UNI, false, true>;
     else
-        fn = serial ? (const void *)k_flood_loop<MS, UNI, true, false> : (const void *)k_flood_loop<MS, UNI, false, false>;
+        fn = (const void *)k_flood_loop<MS, UNI, true, false>;
     // the limit is the function's, shared by every graph: set for this launch
     BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
     void *args[] = {(void *)&a};
@@ -2214,8 +2331,8 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
     }
     if (const uint32_t one = std::max(fgrid, egrid)) {
         // double-buffered partials, and in serial mode the serial sums' scratch
-        grid_blocks = (2u + (serial ? kSumScratch : 0u)) * one;
-        if (fgrid && (st = ensure_loop_flags(g, fgrid))) return st;
+        grid_blocks = 2u * one + (serial ? kSumScratch * std::min(one, kSumBlocks) : 0u);
+        if ((st = ensure_loop_flags(g, fgrid))) return st;
     } else if ((st = flood_grid(g, variant, &grid_blocks, serial))) {
         return st;
     }
@@ -2329,6 +2446,11 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
     BP_CUDA(cudaMemcpyAsync(g->ctl_host, g->ctl, sizeof(LoopyCtl), cudaMemcpyDeviceToHost, g->stream));
     BP_CUDA(cudaStreamSynchronize(g->stream));
     c = *g->ctl_host;
+    if (c.bar_fail && g->grid_bar) {
+        // arrivals of the barrier that gave up are still counted
+        BP_CUDA(cudaMemsetAsync(g->grid_bar, 0, sizeof(uint32_t) * kBarWords, g->stream));
+        BP_CUDA(cudaStreamSynchronize(g->stream));
+    }
     if (c.done == 3 || c.bar_fail)
         return set_error(BP_ERR_TIMEOUT, "a bounded device wait of the iteration kernel timed out");
     if (!c.done) return set_error(BP_ERR_STATE, "loop ended without a stop decision (it=%u)", c.it);
