@@ -271,6 +271,9 @@ __global__ void __cluster_dims__(kBatchCluster, 1, 1) __launch_bounds__(kCluster
     __shared__ double red[kClusterThreads / 32];
     __shared__ uint32_t s_next, s_bound[2];
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    // a block's shared memory may be written by its peers only once it runs:
+    // every block of the cluster has started behind this barrier
+    cluster.sync();
     for (;;) {
         if (cluster.block_rank() == 0 && threadIdx.x == 0) {
             const uint32_t k = atomicAdd(queue, 1u);

@@ -1,0 +1,32 @@
+"""Orders that kernels must keep and that no run can show (a store that comes
+too early is lost only now and then): read from the source."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "belief-propagation_b200", "csrc")
+
+
+def _code(name):
+    """A source file without its comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+
+
+def _body(code, start):
+    """The brace-delimited body that follows the first match of `start`."""
+    at = code.index("{", re.search(start, code).end())
+    depth = 0
+    for k in range(at, len(code)):
+        depth += {"{": 1, "}": -1}.get(code[k], 0)
+        if depth == 0:
+            return code[at:k + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def test_cluster_kernel_meets_before_it_touches_its_peers_shared_memory():
+    """Distributed shared memory is defined only once every block of the
+    cluster has started, which a cluster barrier shows."""
+    body = _body(_code("batch_cluster.cuh"), r"k_batch_cluster\(")
+    assert "map_shared_rank" in body
+    assert "cluster.sync()" in body[:body.index("map_shared_rank")]
