@@ -2053,7 +2053,12 @@ static int loop_plan_of(bp_graph *g, uint32_t tiles, uint32_t per_sm, bp_graph::
     const uint64_t avg = g->E / tiles + 1;
     const uint64_t want = 4 * (2 * (uint64_t)flood_nt<MS>() * MS + 2 * avg * ((SER ? 3 : 2) * MS + 1 + loop_table_stride<MS>()) + 32);
     const int64_t smem = std::min<int64_t>(most, (int64_t)std::max<uint64_t>(least, want)) & ~127ll;
-    BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The limit belongs to the function, for every graph and host thread of
+    // the process: always the most a block can have on this device, so that
+    // no graph lowers it between another's plan and launch.  A launch takes
+    // only the size it asks for.
+    BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 per_block - (int)fa.sharedSizeBytes));
     int bps = 0;
     BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, flood_nt<MS>(), (size_t)smem));
     if (bps < (int)per_sm) return BP_OK;
@@ -2122,8 +2127,6 @@ static int launch_loop(bp_graph *g, bool serial) {
         fn = serial ? (const void *)k_flood_loop<MS, UNI, true, true> : (const void *)k_flood_loop<MS, UNI, false, true>;
     else
         fn = (const void *)k_flood_loop<MS, UNI, true, false>;
-    // the limit is the function's, shared by every graph: set for this launch
-    BP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
     void *args[] = {(void *)&a};
     BP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.grid), dim3(flood_nt<MS>()), args, p.smem, g->stream));
     return BP_OK;
