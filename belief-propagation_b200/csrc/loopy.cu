@@ -802,10 +802,10 @@ constexpr uint64_t kBarrierWaitNs = 2000000000ull;   // 2 s
 // after a run that gave up.
 //
 // The wait is bounded by kBarrierWaitNs, or by c->wait_ms when the host set
-// one.  Test hook: with c->bar_skip == blockIdx.x + 1 this block does not
-// arrive at the run's first barrier and goes on, so the other blocks' waits
-// run out and the run ends with bar_fail; every later wait of this block is
-// bounded the same way, so the launch still ends.
+// one.  Test hook: with c->bar_skip == blockIdx.x + 1 this block arrives at no
+// barrier of the run and does not wait at the first, so every other block's
+// wait runs out, this block's at its second barrier too, and the run ends with
+// bar_fail.
 constexpr uint32_t kBarSubs = 32, kBarStride = 32;   // counters, u32s between them
 constexpr uint32_t kBarFlat = 640;                   // up to here one counter
 constexpr uint32_t kBarWords = (kBarSubs + 2) * kBarStride;
@@ -814,23 +814,27 @@ struct GridBar {
     LoopyCtl *c;
     uint32_t *bar;   // [root][kBarSubs counters][generation]
     uint32_t gen, first;
+    bool held;       // the test hook's block
 
     // one thread's view; every thread of the block keeps the same one
     __device__ __forceinline__ GridBar(LoopyCtl *c_, uint32_t *b) : c(c_), bar(b) {
         gen = first = *(volatile uint32_t *)(bar + (kBarSubs + 1) * kBarStride);
+        held = c->bar_skip == blockIdx.x + 1u;
     }
 };
 
 __device__ __forceinline__ bool grid_barrier(GridBar &gb, uint32_t *s_fail) {
     __syncthreads();
     LoopyCtl *c = gb.c;
-    if (threadIdx.x == 0 && !*(volatile uint32_t *)s_fail && !(gb.gen == gb.first && c->bar_skip == blockIdx.x + 1u)) {
+    if (threadIdx.x == 0 && !*(volatile uint32_t *)s_fail && !(gb.held && gb.gen == gb.first)) {
         uint32_t *root = gb.bar, *gen = gb.bar + (kBarSubs + 1) * kBarStride;
         const uint32_t j = blockIdx.x % kBarSubs, G = gridDim.x;
         uint32_t *sub = gb.bar + (1 + j) * kBarStride;
         fence_acq_rel();
         bool last = false;
-        if (G <= kBarFlat) {
+        if (gb.held) {
+            // never counted
+        } else if (G <= kBarFlat) {
             last = atomicAdd(root, 1u) == G - 1;
         } else if (atomicAdd(sub, 1u) == (G - j + kBarSubs - 1) / kBarSubs - 1) {
             *(volatile uint32_t *)sub = 0;   // untouched until the generation moves
