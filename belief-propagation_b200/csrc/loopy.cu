@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood(const FloodArgs a,
 
 // ---- one cooperative launch for a whole run --------------------------------
 // Blocks that are all resident at once loop over the iterations themselves and
-// meet at a grid barrier (its wait bounded by kBarrierWaitNs; a block that
+// meet at a grid barrier (its wait is bounded; a block that
 // gives up sets bar_fail, and the others then give up at the next barrier).
 // Each block keeps a copy of the control block and sums the per-block delta
 // partials in the same fixed order, so every block takes the same stopping
@@ -801,8 +801,8 @@ constexpr uint64_t kBarrierWaitNs = 2000000000ull;   // 2 s
 // arrives.  The buffer is the graph's (bp_graph::grid_bar), zeroed when made and
 // after a run that gave up.
 //
-// The wait is bounded by kBarrierWaitNs, or by c->wait_ms when the host set
-// one.  Test hook: with c->bar_skip == blockIdx.x + 1 this block arrives at no
+// The wait is bounded by c->wait_ms, which the host sets from the graph
+// (bp_loopy), else by kBarrierWaitNs.  Test hook: with c->bar_skip == blockIdx.x + 1 this block arrives at no
 // barrier of the run and does not wait at the first, so every other block's
 // wait runs out, this block's at its second barrier too, and the run ends with
 // bar_fail.
@@ -2367,13 +2367,17 @@ int bp_loopy(bp_graph *g, const bp_loopy_options *opt, bp_loopy_result *res) {
     c.plo = c.phi = -1.0;
     c.prev_exact = 1;
     c.delta_exact = 1;
-    // the edge loop's barriers also wait for one thread's work: node 0's
-    // normalisations over the runs of equal state counts, and the serial sum
-    // where it has to be formed
-    if (egrid) c.wait_ms = 2000u + g->nruns / 1000u + (serial ? (uint32_t)(c.n_terms / 50000u) : 0u);
-    // test hook of the one-launch loop's bounded grid barrier: a shorter
-    // wait limit, and a block that does not arrive at the first barrier
-    if (const char *env = getenv("BP_DEBUG_WAIT_MS")) c.wait_ms = (uint32_t)strtoul(env, nullptr, 10);
+    // The one-launch loops' barriers also wait for work that one thread does
+    // in order: the in-edges of the largest node (27-43 ns each; E bounds
+    // them), node 0's normalisations and their runs in the edge schedule (120
+    // ns), and the serial sum where it has to be formed term by term (5 ns).
+    // The limit leaves a microsecond, and 20 ns a term, above a base of 2 s.
+    // Test hooks: another base, and a block that no barrier counts.
+    uint32_t wait_base = 2000u;
+    if (const char *env = getenv("BP_DEBUG_WAIT_MS")) wait_base = (uint32_t)strtoul(env, nullptr, 10);
+    if (fgrid || egrid)
+        c.wait_ms = wait_base + g->E / 1000u + (egrid ? g->V / 1000u + g->nruns / 1000u : 0u) +
+                    (serial ? (uint32_t)(c.n_terms / 50000u) : 0u);
     if (const char *env = getenv("BP_DEBUG_BARRIER_SKIP")) c.bar_skip = (uint32_t)strtoul(env, nullptr, 10) + 1u;
     *g->ctl_host = c;
     BP_CUDA(cudaMemcpyAsync(g->ctl, g->ctl_host, sizeof(LoopyCtl), cudaMemcpyHostToDevice, g->stream));

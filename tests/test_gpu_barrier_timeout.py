@@ -1,6 +1,6 @@
 """The one-launch loops' counter barrier gives up after a bounded wait: a block
-is held back from every barrier (BP_DEBUG_BARRIER_SKIP) and the limit cut to
-50 ms (BP_DEBUG_WAIT_MS).  The call returns BP_ERR_TIMEOUT, nothing of it
+is held back from every barrier (BP_DEBUG_BARRIER_SKIP) and the limit's base cut
+to 50 ms (BP_DEBUG_WAIT_MS).  The call returns BP_ERR_TIMEOUT, nothing of it
 stays in the barrier's counters, and the same graph then solves as it did
 before.  One counter and two levels of them, both schedules, both deltas."""
 import re
@@ -59,3 +59,22 @@ def test_barrier_wait_runs_out_and_graph_stays_usable(bp, synth, monkeypatch, V,
             after = solve(g)
             assert after[:2] == before[:2]
             np.testing.assert_array_equal(after[2], before[2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("schedule,delta", [("edge", "f64"), ("edge", "serial"), ("node", "f64"), ("node", "serial")])
+def test_barriers_wait_for_the_largest_node(bp, synth, monkeypatch, schedule, delta):
+    """One node with a million in-edges: one thread multiplies their messages,
+    27-43 ns each, while every other block waits.  The limit grows with the
+    edges, so it does not run out even with a base of 1 ms."""
+    from belief_propagation_b200.engine import BPGraph
+    V, E, S = 1000, 1000000, 2
+    rng = np.random.default_rng(5)
+    j = rng.random((E, S, S), dtype=np.float32)
+    net = synth.Network(np.full(V, S, np.uint32), np.full((V, S), 0.5, np.float32), np.zeros(V, np.uint8),
+                        np.sort(rng.integers(1, V, E)).astype(np.uint32), np.zeros(E, np.uint32), j, name="hub")
+    monkeypatch.setenv("BP_DEBUG_WAIT_MS", "1")
+    with BPGraph.from_network(net) as g:
+        g.latest_slot = 1
+        g.init_messages()
+        assert g.loopy(0.0, 2, schedule=schedule, delta=delta)["executed"] == 2
