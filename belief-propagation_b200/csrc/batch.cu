@@ -390,7 +390,8 @@ struct Group {
     uint32_t *d_order = nullptr;
     uint32_t block = 0;            // threads per block (0 = not tuned yet)
     uint32_t grid = 0;
-    uint32_t large = 0;            // the first networks of `order`, solved by a cluster each with the f64 delta
+    uint32_t large_n = 0;          // the first networks of `order` are large enough for a cluster
+    uint32_t large = 0;            // of these solved by a cluster each with the f64 delta: all or none
 };
 
 }  // namespace bpx
@@ -400,9 +401,6 @@ struct bp_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     std::vector<bpx::NetInfo> info;
-    // the batch is more work than its largest network once per SM: tuned block
-    // launches (bp_batch_autotune) then do without clusters
-    bool work_bound = false;
     uint64_t totV = 0, totE = 0, totNodeF = 0, totMsgF = 0, totJointF = 0, totPtr = 0;
     bpx::NetInfo *d_info = nullptr;
     uint32_t *in_ptr = nullptr, *in_src = nullptr, *pos_edge = nullptr, *net_of_edge = nullptr;
@@ -427,6 +425,7 @@ namespace bpx {
 // delta; below, a block's own latency is about the cluster barrier's and more
 // networks run side by side); BP_BATCH_CLUSTER_EDGES overrides (0: none)
 constexpr uint32_t kClusterEdges = 1024;
+constexpr uint32_t kDefaultBlock = 256;   // threads per network block, until tuned
 
 // the cluster launch of the group's large networks, and a block each for the
 // rest (every network with the serial delta)
@@ -742,26 +741,16 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
     }
     const char *env = getenv("BP_BATCH_CLUSTER_EDGES");
     const uint32_t least = env ? (uint32_t)strtoul(env, nullptr, 10) : kClusterEdges;
-    if (!env) {
-        double all = 0.0, most = 0.0;
-        for (const auto &gr : bt->groups)
-            for (uint32_t x : gr.order) {
-                const double w = (double)bt->info[x].E * gr.S * gr.S;
-                all += w;
-                most = std::max(most, w);
-            }
-        bt->work_bound = all > most * bt->sm_count;
-    }
     for (auto &gr : bt->groups) {
         std::stable_sort(gr.order.begin(), gr.order.end(), [&](uint32_t x, uint32_t y) { return work(x) > work(y); });
-        gr.block = 256;
+        gr.block = kDefaultBlock;
         gr.grid = grid_for_group(bt, gr, gr.block);
         if (least) {
             // first, largest first: the large ones (order sorts by work, so
             // by edges up to the nodes' share)
             auto mid = std::stable_partition(gr.order.begin(), gr.order.end(),
                                              [&](uint32_t x) { return bt->info[x].E >= least; });
-            gr.large = (uint32_t)(mid - gr.order.begin());
+            gr.large = gr.large_n = (uint32_t)(mid - gr.order.begin());
         }
         BP_CUDA(cudaMalloc((void **)&gr.d_order, sizeof(uint32_t) * gr.order.size()));
         BP_CUDA(cudaMemcpyAsync(gr.d_order, gr.order.data(), sizeof(uint32_t) * gr.order.size(),
@@ -786,7 +775,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
 // ---- autotuning of threads per block, cached on disk ---------------------
 // kernel revision in the autotune key: a cached block size belongs to the
 // kernel it was timed on
-constexpr int kTuneRevision = 5;
+constexpr int kTuneRevision = 6;
 
 static std::string tune_key(bp_batch *bt, const Group &gr, int serial) {
     // the networks that run a block each
@@ -797,7 +786,7 @@ static std::string tune_key(bp_batch *bt, const Group &gr, int serial) {
         E += bt->info[gr.order[k]].E;
     }
     const uint64_t cnt = gr.order.size() - skip;
-    const unsigned mv = (unsigned)(V / cnt), deg10 = (unsigned)(V ? 10 * E / V : 0);
+    const unsigned mv = cnt ? (unsigned)(V / cnt) : 0u, deg10 = (unsigned)(V ? 10 * E / V : 0);
     unsigned lv = 0;
     while ((1u << (lv + 1)) <= mv) ++lv;
     cudaDeviceProp prop;
@@ -854,6 +843,142 @@ static void cache_store(const std::string &key, uint32_t block, uint32_t grid) {
     if (!f) return;
     fprintf(f, "%s %u %u\n", key.c_str(), block, grid);
     fclose(f);
+}
+
+// what trial runs overwrite: the beliefs and which messages are the latest
+struct TuneState {
+    float *belief = nullptr;
+    std::vector<uint8_t> latest;
+    ~TuneState() { cudaFree(belief); }
+    int save(bp_batch *bt) {
+        latest.resize(bt->N);
+        BP_CUDA(cudaMalloc((void **)&belief, sizeof(float) * (bt->totNodeF + 1)));
+        BP_CUDA(cudaMemcpyAsync(belief, bt->belief, sizeof(float) * bt->totNodeF, cudaMemcpyDeviceToDevice, bt->stream));
+        BP_CUDA(cudaMemcpyAsync(latest.data(), bt->latest, bt->N, cudaMemcpyDeviceToHost, bt->stream));
+        BP_CUDA(cudaStreamSynchronize(bt->stream));
+        return BP_OK;
+    }
+    int restore(bp_batch *bt) const {
+        if (!belief) return BP_OK;
+        BP_CUDA(cudaMemcpyAsync(bt->belief, belief, sizeof(float) * bt->totNodeF, cudaMemcpyDeviceToDevice, bt->stream));
+        BP_CUDA(cudaMemcpyAsync(bt->latest, latest.data(), bt->N, cudaMemcpyHostToDevice, bt->stream));
+        return BP_OK;
+    }
+};
+
+// the second of two runs of `launch` from the saved state, in ms
+template <typename F>
+static int time_trial(bp_batch *bt, const TuneState &keep, F launch, float *ms) {
+    int st;
+    for (int rep = 0; rep < 2; ++rep) {
+        if ((st = keep.restore(bt))) return st;
+        BP_CUDA(cudaEventRecord(bt->ev0, bt->stream));
+        if ((st = launch())) return st;
+        BP_CUDA(cudaEventRecord(bt->ev1, bt->stream));
+        BP_CUDA(cudaEventSynchronize(bt->ev1));
+        BP_CUDA(cudaEventElapsedTime(ms, bt->ev0, bt->ev1));
+    }
+    return BP_OK;
+}
+
+// threads per block, and blocks in flight, of the networks that run a block
+// each, group by group: a block keeps its network's arrays in L2 across its
+// iterations, so fewer blocks than the GPU holds can be faster once the
+// networks in flight outgrow L2
+static int tune_blocks(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
+    for (size_t gi = 0; gi < bt->groups.size(); ++gi) {
+        Group &gr = bt->groups[gi];
+        if (!a.serial && gr.large == gr.order.size()) continue;   // clusters only: nothing to tune
+        const std::string key = tune_key(bt, gr, a.serial);
+        uint32_t best_grid = 0;
+        uint32_t best = cache_lookup(key, &best_grid);
+        if (!best) {
+            float best_ms = 1e30f;
+            std::vector<std::pair<uint32_t, uint32_t>> trials;
+            for (uint32_t c : {64u, 128u, 256u, 512u}) {
+                const uint32_t occ = grid_for_group(bt, gr, c, sizeof(float) * 2 * a.sum_ch);
+                trials.push_back({c, occ});
+                for (uint32_t per_sm : {1u, 2u, 4u, 8u}) {
+                    const uint32_t g = per_sm * (uint32_t)bt->sm_count;
+                    if (g < occ) trials.push_back({c, g});
+                }
+            }
+            for (const auto &tr : trials) {
+                float ms = 0.0f;
+                const int st = time_trial(bt, keep, [&]() -> int {
+                    BP_CUDA(cudaMemsetAsync(bt->queues + gi, 0, sizeof(uint32_t), bt->stream));
+                    return launch_group_s(bt, gr, a, (uint32_t)gi, tr.first, tr.second, bt->stream);
+                }, &ms);
+                if (st) return st;
+                if (ms < best_ms) {
+                    best_ms = ms;
+                    best = tr.first;
+                    best_grid = tr.second;
+                }
+            }
+            cache_store(key, best, best_grid);
+        }
+        gr.block = best;
+        const uint32_t occ = grid_for_group(bt, gr, best);
+        gr.grid = best_grid ? std::min(best_grid, occ) : occ;
+    }
+    return BP_OK;
+}
+
+// how a batch with networks large enough for clusters is launched
+enum BatchPlan : uint32_t { kPlanClusters = 1, kPlanClustersTuned = 2, kPlanBlocksTuned = 3 };
+
+// the launch of a plan: clusters for the large networks or a block for every
+// one, with the launch shape that batch_create_impl gives
+static void set_plan(bp_batch *bt, bool clusters) {
+    for (auto &gr : bt->groups) {
+        gr.large = clusters ? gr.large_n : 0;
+        gr.block = kDefaultBlock;
+        gr.grid = grid_for_group(bt, gr, gr.block);
+    }
+}
+
+// One group's best launch alone need not be the batch's, whose groups run side
+// by side, and clusters shorten the longest networks while blocks with a tuned
+// number in flight keep more of each network on its SM.  So whole batches are
+// timed: as created, clusters with the rest tuned, and tuned blocks for all,
+// the last only where untuned blocks come within twice the clusters' time
+// (tuning has gained them 1.6x: 4096 networks 178 -> 112 ms, clusters 116;
+// 1024 networks 104, clusters 29).
+static int tune_batch(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
+    bool any = false;
+    for (const auto &gr : bt->groups) any = any || gr.large_n;
+    if (a.serial || !any) return tune_blocks(bt, a, keep);
+    int st;
+    set_plan(bt, true);
+    std::string key = "plan";
+    for (const auto &gr : bt->groups) {
+        const std::string k = tune_key(bt, gr, 0);
+        key += "|" + std::to_string(std::hash<std::string>()(k) & 0xffffffu) + "," + std::to_string(gr.large_n);
+    }
+    key += "|rev=" + std::to_string(kTuneRevision);
+    uint32_t unused = 0, plan = cache_lookup(key, &unused);
+    if (!plan) {
+        auto whole = [&](float *ms) { return time_trial(bt, keep, [&] { return enqueue_batch(bt, a); }, ms); };
+        float created = 0.0f, blocks = 0.0f, ms = 0.0f, best = 0.0f;
+        if ((st = whole(&created))) return st;
+        plan = kPlanClusters;
+        best = created;
+        if ((st = tune_blocks(bt, a, keep)) || (st = whole(&ms))) return st;
+        if (ms < best) {
+            plan = kPlanClustersTuned;
+            best = ms;
+        }
+        set_plan(bt, false);
+        if ((st = whole(&blocks))) return st;
+        if (blocks < 2.0f * created) {
+            if ((st = tune_blocks(bt, a, keep)) || (st = whole(&ms))) return st;
+            if (ms < best) plan = kPlanBlocksTuned;
+        }
+        cache_store(key, plan, 0);
+    }
+    set_plan(bt, plan != kPlanBlocksTuned);
+    return plan == kPlanClusters ? BP_OK : tune_blocks(bt, a, keep);
 }
 
 }  // namespace bpx
@@ -958,85 +1083,21 @@ void bp_batch_default_options(bp_batch_options *o) {
 
 int bp_batch_autotune(bp_batch *bt, const bp_batch_options *o) {
     if (!bt || !o) return set_error(BP_ERR_INVALID, "null argument");
-    static const uint32_t cand[] = {64, 128, 256, 512};
     const int serial = o->delta_mode == BP_DELTA_SERIAL_F32;
     if (serial && !bt->absdiff) BP_CUDA(cudaMalloc((void **)&bt->absdiff, sizeof(float) * 2 * (bt->totMsgF + 4)));
-    // beliefs are overwritten by trial runs: keep them
-    float *keep = nullptr;
-    BP_CUDA(cudaMalloc((void **)&keep, sizeof(float) * (bt->totNodeF + 1)));
-    BP_CUDA(cudaMemcpyAsync(keep, bt->belief, sizeof(float) * bt->totNodeF, cudaMemcpyDeviceToDevice, bt->stream));
-    std::vector<uint8_t> latest0(bt->N);
-    BP_CUDA(cudaMemcpyAsync(latest0.data(), bt->latest, bt->N, cudaMemcpyDeviceToHost, bt->stream));
-    BP_CUDA(cudaStreamSynchronize(bt->stream));
-    const BatchArgs a = batch_args(bt, o->tolerance, o->max_iterations, serial, o->init_messages);
-    // a cluster shortens the longest networks; where the batch is bound by all
-    // its work, a block each with a tuned number in flight keeps more of a
-    // network on its SM: 4096 networks 113-114 ms tuned, 117 with clusters and 178
-    // (clusters 111) untuned.  1024 networks: clusters 26, blocks 104.
-    if (!serial && bt->work_bound)
-        for (auto &gr : bt->groups) gr.large = 0;
-    for (size_t gi = 0; gi < bt->groups.size(); ++gi) {
-        Group &gr = bt->groups[gi];
-        if (!serial && gr.large == gr.order.size()) continue;   // clusters only: nothing to tune
-        const std::string key = tune_key(bt, gr, serial);
-        uint32_t best_grid = 0;
-        uint32_t best = cache_lookup(key, &best_grid);
-        if (!best) {
-            float best_ms = 1e30f;
-            // block sizes, and networks in flight: a block keeps its
-            // network's arrays in L2 across its iterations, so fewer blocks
-            // than the GPU holds can be faster once the networks in flight
-            // outgrow L2
-            std::vector<std::pair<uint32_t, uint32_t>> trials;
-            for (uint32_t c : cand) {
-                const uint32_t occ = grid_for_group(bt, gr, c, sizeof(float) * 2 * a.sum_ch);
-                trials.push_back({c, occ});
-                for (uint32_t per_sm : {1u, 2u, 4u, 8u}) {
-                    const uint32_t g = per_sm * (uint32_t)bt->sm_count;
-                    if (g < occ) trials.push_back({c, g});
-                }
-            }
-            for (const auto &tr : trials) {
-                const uint32_t c = tr.first, grid = tr.second;
-                float tot = 0.0f;
-                for (int rep = 0; rep < 2; ++rep) {
-                    BP_CUDA(cudaMemcpyAsync(bt->belief, keep, sizeof(float) * bt->totNodeF, cudaMemcpyDeviceToDevice,
-                                            bt->stream));
-                    BP_CUDA(cudaMemcpyAsync(bt->latest, latest0.data(), bt->N, cudaMemcpyHostToDevice, bt->stream));
-                    BP_CUDA(cudaMemsetAsync(bt->queues + gi, 0, sizeof(uint32_t), bt->stream));
-                    BP_CUDA(cudaEventRecord(bt->ev0, bt->stream));
-                    int st = launch_group_s(bt, gr, a, (uint32_t)gi, c, grid, bt->stream);
-                    if (st) {
-                        cudaFree(keep);
-                        return st;
-                    }
-                    BP_CUDA(cudaEventRecord(bt->ev1, bt->stream));
-                    BP_CUDA(cudaEventSynchronize(bt->ev1));
-                    float ms = 0.0f;
-                    cudaEventElapsedTime(&ms, bt->ev0, bt->ev1);
-                    if (rep) tot += ms;
-                }
-                if (tot < best_ms) {
-                    best_ms = tot;
-                    best = c;
-                    best_grid = grid;
-                }
-            }
-            cache_store(key, best, best_grid);
-        }
-        gr.block = best;
-        const uint32_t occ = grid_for_group(bt, gr, best);
-        gr.grid = best_grid ? std::min(best_grid, occ) : occ;
+    TuneState keep;
+    int st = keep.save(bt);
+    if (!st) {
+        const BatchArgs a = batch_args(bt, o->tolerance, o->max_iterations, serial, o->init_messages);
+        st = tune_batch(bt, a, keep);
     }
-    BP_CUDA(cudaMemcpyAsync(bt->belief, keep, sizeof(float) * bt->totNodeF, cudaMemcpyDeviceToDevice, bt->stream));
-    BP_CUDA(cudaMemcpyAsync(bt->latest, latest0.data(), bt->N, cudaMemcpyHostToDevice, bt->stream));
-    BP_CUDA(cudaStreamSynchronize(bt->stream));
-    cudaFree(keep);
+    const int back = keep.restore(bt);
+    cudaStreamSynchronize(bt->stream);
     if (bt->exec) {
         cudaGraphExecDestroy(bt->exec);
         bt->exec = nullptr;
     }
-    return BP_OK;
+    return st ? st : back;
 }
 
 int bp_batch_get_groups(const bp_batch *bt, uint32_t *states, uint32_t *max_nodes, uint32_t *block, uint32_t *grid,

@@ -344,9 +344,10 @@ void bp_batch_default_options(bp_batch_options *o);
  * nodes of a state count form a group of their own, with its own launch
  * shape, work queue and stream.
  * bp_batch_autotune times 64/128/256/512 threads per network block, and
- * blocks in flight, for each group on this batch, keeps the fastest (results
- * cached in $BP_AUTOTUNE_CACHE, default ~/.cache/bp_b200_autotune.txt);
- * beliefs and messages are restored */
+ * blocks in flight, for each group on this batch and, where networks are
+ * large enough for clusters, the whole batch with clusters and with a block
+ * per network, and keeps the fastest (results cached in $BP_AUTOTUNE_CACHE,
+ * default ~/.cache/bp_b200_autotune.txt); beliefs and messages are restored */
 int bp_batch_autotune(bp_batch *b, const bp_batch_options *o);
 /* per group (at most *count entries; *count returns the number of groups):
  * its state count and threads per block (a state count appears once per size
