@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood(const FloodArgs a,
     __shared__ bool s_last;
 
     LoopyCtl *ctl = a.ctl;
-    griddep_launch_dependents();   // the next iteration's blocks come up as this one's leave
+    griddep_launch_dependents();   // launched to overlap (block_tiles): the next one's blocks come up as these leave
     griddep_wait();
     if (*(volatile uint32_t *)&ctl->done) return;
     const uint32_t it = ctl->it, ce = ctl->check_every;
@@ -1686,18 +1686,19 @@ static int resident_blocks(int *bps) {
     return resident_blocks_mb<MS, UNI, FU, flood_min_blocks<MS, FU>()>(bps);
 }
 
-// one iteration's kernel, launched with programmatic stream serialisation: its
-// blocks may come up while the last of the kernel ahead drain, and wait for
-// that grid before they read anything
+// one iteration's kernel; with `overlap` launched with programmatic stream
+// serialisation: its blocks may come up while the last of the kernel ahead
+// drain, and wait for that grid before they read anything
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_iteration(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t st, Args... args) {
+static cudaError_t launch_iteration(void (*kern)(KArgs...), unsigned grid, unsigned block, bool overlap,
+                                    cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, args...);
@@ -1705,24 +1706,36 @@ static cudaError_t launch_iteration(void (*kern)(KArgs...), unsigned grid, unsig
 
 // launch of the block-tile kernel with the register cap block_min_blocks()
 template <int MS, bool UNI, int FU>
-static cudaError_t launch_block_tiles(unsigned grid, cudaStream_t st, const FloodArgs &a, uint32_t ntiles, bool serial) {
+static cudaError_t launch_block_tiles(unsigned grid, bool overlap, cudaStream_t st, const FloodArgs &a, uint32_t ntiles,
+                                      bool serial) {
     constexpr int NT = flood_nt<MS>();
     constexpr int MB = flood_min_blocks<MS, FU>();
-    if (serial) return launch_iteration(k_flood<MS, UNI, FU, MB, true>, grid, NT, st, a, ntiles);
+    if (serial) return launch_iteration(k_flood<MS, UNI, FU, MB, true>, grid, NT, overlap, st, a, ntiles);
     if constexpr (MS <= 2) {
         const int mb = block_min_blocks();
-        if (mb == 10) return launch_iteration(k_flood<MS, UNI, FU, 10>, grid, NT, st, a, ntiles);
-        if (mb == 16) return launch_iteration(k_flood<MS, UNI, FU, 16>, grid, NT, st, a, ntiles);
+        if (mb == 10) return launch_iteration(k_flood<MS, UNI, FU, 10>, grid, NT, overlap, st, a, ntiles);
+        if (mb == 16) return launch_iteration(k_flood<MS, UNI, FU, 16>, grid, NT, overlap, st, a, ntiles);
     }
-    return launch_iteration(k_flood<MS, UNI, FU>, grid, NT, st, a, ntiles);
+    return launch_iteration(k_flood<MS, UNI, FU>, grid, NT, overlap, st, a, ntiles);
 }
 
 // block-tile grid: one block per tile, or (default; BP_FLOOD_PERSIST=0
 // turns it off) a persistent grid of resident blocks x SMs walking the tiles
+//
+// overlap: whether the iterations' launches may overlap.  The blocks of the
+// next iteration then come up wherever a block of this one leaves, so an SM
+// whose blocks had a tile less gets the low block ids, all of which have one
+// more.  That is worth it only where the last round of tiles is nearly full: us
+// per iteration overlapped / not at a last round 0.98 full 26.7 / 27.4 (2
+// states, 677,000 nodes), 27.8 / 28.3 (3, 452,000), 56.6 / 57.5 (4, 906,000);
+// 0.9 full 26.8 / 27.0, 28.5 / 28.2, 56.1 / 56.9; 0.8 full 21.2 / 20.1 (3,
+// 273,000), 30.1 / 29.0 (4, 424,000); 0.4 full 24.8 / 23.6, 26.7 / 23.9, 28.3 /
+// 26.9.
 template <int MS, bool UNI>
-static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles) {
+static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles, bool *overlap) {
     *ntiles = grid_for(g->V, flood_nt<MS>());
     *grid = *ntiles;
+    *overlap = false;
     const char *env = getenv("BP_FLOOD_PERSIST");
     if (env && env[0] == '0') return BP_OK;
     int bps = 0, st;
@@ -1737,7 +1750,11 @@ static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles) {
     int dev = 0, sms = 0;
     BP_CUDA(cudaGetDevice(&dev));
     BP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (bps > 0) *grid = (unsigned)std::min<uint64_t>(*ntiles, (uint64_t)bps * sms);
+    if (bps > 0 && *ntiles) {
+        const uint32_t round = (uint32_t)bps * (uint32_t)sms;   // tiles at once
+        *grid = std::min(*ntiles, round);
+        *overlap = (*ntiles - 1u) % round + 1u >= round - round / 8u;
+    }
     return BP_OK;
 }
 
@@ -1827,8 +1844,8 @@ static int split_run_nv(bp_graph *g, uint32_t k, uint32_t *nparts) {
     if (nparts) *nparts = ga;
     const SplitArgs a = split_args(g, ga);
     for (uint32_t i = 0; i < k; ++i) {
-        BP_CUDA((launch_iteration(k_flood_send<MS, SER>, ga, kSendThreads, g->stream, a)));
-        BP_CUDA((launch_iteration(k_flood_nodes<MS, SER, NV>, gb, kNodeThreads, g->stream, a)));
+        BP_CUDA((launch_iteration(k_flood_send<MS, SER>, ga, kSendThreads, true, g->stream, a)));
+        BP_CUDA((launch_iteration(k_flood_nodes<MS, SER, NV>, gb, kNodeThreads, true, g->stream, a)));
     }
     return BP_OK;
 }
@@ -1931,8 +1948,9 @@ static int enqueue_node_iterations(bp_graph *g, uint32_t k, bool serial, int var
     const bool warp_tiled = variant != BP_KERNEL_BLOCK_TILE;
     unsigned grid = grid_for(g->V, 256);
     uint32_t ntiles = 0;
+    bool overlap = false;
     if (!warp_tiled) {
-        int st = block_tiles<MS, UNI>(g, &grid, &ntiles);
+        int st = block_tiles<MS, UNI>(g, &grid, &ntiles, &overlap);
         if (st) return st;
     }
     const FloodArgs a = flood_args(g);
@@ -1940,16 +1958,16 @@ static int enqueue_node_iterations(bp_graph *g, uint32_t k, bool serial, int var
     for (uint32_t i = 0; i < k; ++i) {
         if (!warp_tiled) {
             if constexpr (MS <= 2) {
-                if (unroll == 1) BP_CUDA((launch_block_tiles<MS, UNI, 1>(grid, g->stream, a, ntiles, serial)));
-                else if (unroll == 2) BP_CUDA((launch_block_tiles<MS, UNI, 2>(grid, g->stream, a, ntiles, serial)));
-                else BP_CUDA((launch_block_tiles<MS, UNI, 4>(grid, g->stream, a, ntiles, serial)));
+                if (unroll == 1) BP_CUDA((launch_block_tiles<MS, UNI, 1>(grid, overlap, g->stream, a, ntiles, serial)));
+                else if (unroll == 2) BP_CUDA((launch_block_tiles<MS, UNI, 2>(grid, overlap, g->stream, a, ntiles, serial)));
+                else BP_CUDA((launch_block_tiles<MS, UNI, 4>(grid, overlap, g->stream, a, ntiles, serial)));
             } else {
                 constexpr int FU = flood_unroll<MS>();
                 if (serial)
                     BP_CUDA((launch_iteration(k_flood<MS, UNI, FU, flood_min_blocks_serial<MS, FU>(), true>, grid, NT,
-                                              g->stream, a, ntiles)));
+                                              overlap, g->stream, a, ntiles)));
                 else
-                    BP_CUDA((launch_iteration(k_flood<MS, UNI, FU>, grid, NT, g->stream, a, ntiles)));
+                    BP_CUDA((launch_iteration(k_flood<MS, UNI, FU>, grid, NT, overlap, g->stream, a, ntiles)));
             }
         } else if constexpr (MS <= 2) {
             if (unroll == 1) k_flood_w<MS, UNI, 1><<<grid, 256, 0, g->stream>>>(a);
@@ -2017,7 +2035,8 @@ static int flood_grid(bp_graph *g, int variant, uint32_t *grid, bool serial) {
     }
     if (variant == BP_KERNEL_BLOCK_TILE) {
         uint32_t ntiles = 0;
-        auto tiles = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, block_tiles, g, grid, &ntiles); };
+        bool overlap = false;
+        auto tiles = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, block_tiles, g, grid, &ntiles, &overlap); };
         return tiles();
     }
     *grid = grid_for(g->V, 256);
