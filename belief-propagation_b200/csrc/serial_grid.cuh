@@ -6,10 +6,8 @@
 // increment that depends on m only through its parity, so a run of terms is
 // a pair of increments (SumStep) and runs compose.  Every block takes one
 // slice of the terms and every warp a part of it; from the slice's f64 prefix
-// it guesses the binade(s) the running sum has there -- one, the two on either
-// side of a crossing, or three where the fp32 sum may have drifted from the
-// prefix by more than a binade is wide (from 5.6M terms on: the lowest, the
-// highest and the one below it) -- and composes its terms' steps for each guess.
+// it guesses the binade(s) the running sum has there -- one, or the two on
+// either side of a crossing -- and composes its terms' steps for each guess.
 // One warp then walks the slices in order: the walk knows the exact running
 // sum, so a slice's pair counts only when it was made for the binade the sum
 // is in and the sum stays below the binade's top; otherwise that slice is
@@ -23,26 +21,22 @@
 // had not decided).  Now 80k terms (79 blocks) take 50 us and 600k terms (782
 // blocks) 70 us, two sums at once the same: half of it the walk, a few
 // thousand cycles for each of the half dozen slices that cross, the rest four
-// grid barriers.  10M terms: 0.6 ms; without the third guess 46 ms, since half
-// of the slices then fit no pair and one warp adds them.
+// grid barriers.  10M terms: 0.5 ms.
 #pragma once
 
 // doubles of scratch per block behind the grid's 2 x G delta partials: two
-// sums' slice sum, record, warps' pairs and lanes' pairs, and warps' and lanes'
-// third pairs
-constexpr uint32_t kSumScratch = 2 * (1 + 4 + 16 + 512 + 8 + 256);
+// sums' slice sum, record, warps' pairs and lanes' pairs
+constexpr uint32_t kSumScratch = 2 * (1 + 4 + 16 + 512);
 constexpr int32_t kAnyUnit = 0x7fffffff;   // an empty slice: nothing to add in any binade
 
 constexpr uint32_t kSumBlocks = 1184;   // eight per SM: bounds the scratch
 
 struct SumRec {
-    int32_t ua, ub;   // unit exponents of the lowest and the highest guess: a, b
-    SumStep a, b, c;  // c: for ub - 1, where that is a third (sum_third)
+    int32_t ua, ub;   // unit exponents the two pairs were made for
+    SumStep a, b;
+    uint32_t pad[2];
 };
 static_assert(sizeof(SumRec) == 32, "two 16-byte loads");
-
-// is the binade below the highest guess one that neither pair is made for
-__device__ __forceinline__ bool sum_third(int32_t ua, int32_t ub) { return ua != kAnyUnit && ub - ua >= 2; }
 
 // the scratch arrays of sum j (0: the check's terms, 1: the previous check's)
 struct SumScr {
@@ -50,16 +44,12 @@ struct SumScr {
     SumRec *rec;     // [G]
     uint4 *part;     // [G][8] the warps' pairs: a.e, a.o, b.e, b.o
     uint4 *lane;     // [G][8][32] the lanes' pairs
-    uint2 *part_c;   // [G][8] the warps' third pairs, where there are any
-    uint2 *lane_c;   // [G][8][32] the lanes'
     __device__ SumScr(double *partials, uint32_t G, int j) {
         double *base = partials + 2 * (size_t)gridDim.x;
         slice = base + (size_t)j * G;
         rec = reinterpret_cast<SumRec *>(base + 2 * (size_t)G) + (size_t)j * G;
         part = reinterpret_cast<uint4 *>(base + 10 * (size_t)G) + (size_t)j * G * 8;
         lane = reinterpret_cast<uint4 *>(base + 42 * (size_t)G) + (size_t)j * G * 256;
-        part_c = reinterpret_cast<uint2 *>(base + 1066 * (size_t)G) + (size_t)j * G * 8;
-        lane_c = reinterpret_cast<uint2 *>(base + 1082 * (size_t)G) + (size_t)j * G * 256;
     }
 };
 
@@ -67,6 +57,27 @@ struct SumScr {
 __device__ __forceinline__ int32_t sum_unit(double s) {
     if (!(s >= 0x1p-126)) return -149;
     return min(ilogb(s), 127) - 23;
+}
+
+// The units guessed for a slice with f64 prefix P and sum `own` among n terms:
+// the fp32 sum lies within n 2^-24 of the prefix (a half at most).  From 5.6M
+// terms on that can span three binades; a slice inside one then takes its own
+// and the nearer neighbour's, which leaves a drift of 29 % or more to either
+// side unguessed.  The lowest and the highest of the three, without the
+// prefix's own, made 10M terms take 46 ms; a third pair made every sum's code,
+// and the loop around it, spill (40,000 edges of 2 states 2.4 % slower).
+__device__ __forceinline__ void sum_guess(double P, double own, uint64_t n, int32_t &ua, int32_t &ub) {
+    const double wide = fmin(0.5, (double)n * 0x1p-24);
+    ua = sum_unit(P * (1.0 - wide));
+    ub = sum_unit((P + own) * (1.0 + wide));
+    if (wide > 1.0 / 3.0 && ub - ua >= 2) {
+        ua = sum_unit(P);
+        ub = sum_unit(P + own);
+        if (ua == ub) {
+            if (sum_unit(P * 0x1.6a09e667f3bcdp+0) == ua) ua -= 1;   // P below sqrt(2) of its binade
+            else ub += 1;
+        }
+    }
 }
 
 // sum_term's pair without its branches: term t added in the binade with unit
@@ -85,17 +96,6 @@ __device__ __forceinline__ SumStep sum_step(float t, int32_t eu) {
     st.e = fl + (up | (tie & fl & 1u));
     st.o = fl + (up | (tie & ~fl & 1u));
     return st;
-}
-
-// the pairs of the warp's lanes in order, in lane 0
-__device__ __forceinline__ void warp_sum_fold(SumStep &A) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        SumStep o;
-        o.e = __shfl_down_sync(0xffffffffu, A.e, d);
-        o.o = __shfl_down_sync(0xffffffffu, A.o, d);
-        if ((threadIdx.x & (2u * d - 1u)) == 0u) A = sum_compose(A, o);
-    }
 }
 
 // terms x[lo, hi) in order, composed for unit exponents ua and ub; lane 0 of
@@ -124,22 +124,18 @@ __device__ __forceinline__ void warp_sum_steps(const float *__restrict__ x, uint
     }
     if (ub == ua) B = A;
     lanes[lane] = make_uint4(A.e, A.o, B.e, B.o);
-    warp_sum_fold(A);
-    warp_sum_fold(B);
-}
-
-// the same for one more unit exponent: the terms are read again (they lie in
-// L2), which costs the sums without a third guess nothing
-__device__ __noinline__ void warp_sum_steps_c(const float *__restrict__ x, uint64_t lo, uint64_t hi, int32_t uc,
-                                              SumStep &C, uint2 *lanes) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t k = (hi - lo + 31u) / 32u;
-    const uint64_t p0 = min(lo + lane * k, hi), p1 = min(p0 + k, hi);
-    C = SumStep{0u, 0u};
-#pragma unroll 4
-    for (uint64_t p = p0; p < p1; ++p) C = sum_compose(C, sum_step(__ldcg(x + p), uc));
-    lanes[lane] = make_uint2(C.e, C.o);
-    warp_sum_fold(C);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        SumStep oa, ob;
+        oa.e = __shfl_down_sync(0xffffffffu, A.e, d);
+        oa.o = __shfl_down_sync(0xffffffffu, A.o, d);
+        ob.e = __shfl_down_sync(0xffffffffu, B.e, d);
+        ob.o = __shfl_down_sync(0xffffffffu, B.o, d);
+        if ((lane & (2u * d - 1u)) == 0u) {
+            A = sum_compose(A, oa);
+            B = sum_compose(B, ob);
+        }
+    }
 }
 
 // a float's binade: unit exponent, m, and the m the binade ends at
@@ -190,18 +186,13 @@ __device__ __forceinline__ float warp_serial_add(float s, const float *__restric
 // s is in) from run `pos` on, applied up to the first that leaves the binade
 // or has no pair for it; returns that run (32: none)
 __device__ __forceinline__ uint32_t warp_sum_apply(float &s, uint32_t pos, bool any, int32_t ua, int32_t ub, SumStep a,
-                                                   SumStep b, SumStep c) {
+                                                   SumStep b) {
     const uint32_t lane = threadIdx.x & 31u;
     int32_t eu;
     uint32_t m, top, Es;
     sum_split(s, eu, m, top, Es);
     SumStep inc{0u, 0u};
-    if (lane >= pos && !any) {
-        if (ua == eu) inc = a;
-        else if (ub == eu) inc = b;
-        else if (sum_third(ua, ub) && ub - 1 == eu) inc = c;
-        else inc = SumStep{kSumSat, kSumSat};
-    }
+    if (lane >= pos && !any) inc = ua == eu ? a : (ub == eu ? b : SumStep{kSumSat, kSumSat});
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         SumStep o;
@@ -235,22 +226,18 @@ __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t
         r.ub = (int32_t)n0.y;
         r.a = SumStep{n0.z, n0.w};
         r.b = SumStep{n1.x, n1.y};
-        r.c = SumStep{n1.z, n1.w};
         n0 = record(base + 32 + lane, 0);   // the next 32 records, while these are walked
         n1 = record(base + 32 + lane, 1);
         for (uint32_t pos = 0; pos < cnt;) {
             if (sum_is_inf(s)) return s;   // inf stays
-            const uint32_t f = warp_sum_apply(s, pos, r.ua == kAnyUnit, r.ua, r.ub, r.a, r.b, r.c);
+            const uint32_t f = warp_sum_apply(s, pos, r.ua == kAnyUnit, r.ua, r.ub, r.a, r.b);
             if (f >= cnt) break;
             pos = f + 1;
             // slice base + f, one warp's part after another
             const uint32_t b = base + f;
             const uint64_t lo = min(n, (uint64_t)b * L), hi = min(n, lo + L);
             const int32_t ua = __shfl_sync(0xffffffffu, r.ua, f), ub = __shfl_sync(0xffffffffu, r.ub, f);
-            const bool third = sum_third(ua, ub);
             const uint4 part = lane < nw ? __ldcg(scr.part + (size_t)b * 8 + lane) : make_uint4(0, 0, 0, 0);
-            const uint2 part_c = third && lane < nw ? __ldcg(scr.part_c + (size_t)b * 8 + lane) : make_uint2(0, 0);
-            auto guessed = [&](int32_t eu) { return ua == eu || ub == eu || (third && ub - 1 == eu); };
             for (uint32_t w = 0; w < nw; ++w) {
                 const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
                 if (p0 >= p1) break;
@@ -258,13 +245,13 @@ __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t
                 uint32_t m, top, Es;
                 sum_split(s, eu, m, top, Es);
                 if (Es >= 0xffu) return s;
-                if (!guessed(eu)) {
+                if (ua != eu && ub != eu) {
                     s = warp_serial_add(s, x, p0, p1, buf);
                     continue;
                 }
                 SumStep st;
-                st.e = __shfl_sync(0xffffffffu, ua == eu ? part.x : (ub == eu ? part.z : part_c.x), w);
-                st.o = __shfl_sync(0xffffffffu, ua == eu ? part.y : (ub == eu ? part.w : part_c.y), w);
+                st.e = __shfl_sync(0xffffffffu, ua == eu ? part.x : part.z, w);
+                st.o = __shfl_sync(0xffffffffu, ua == eu ? part.y : part.w, w);
                 const uint32_t mw = sum_apply(m, st);
                 if (mw < top) {
                     s = sum_join(Es, mw);
@@ -272,18 +259,16 @@ __device__ float warp_sum_walk(const float *__restrict__ x, uint64_t n, uint64_t
                 }
                 // the part crosses: its lanes' runs, the crossing one term by term
                 const uint4 lp = __ldcg(scr.lane + ((size_t)b * 8 + w) * 32 + lane);
-                const uint2 lc = third ? __ldcg(scr.lane_c + ((size_t)b * 8 + w) * 32 + lane) : make_uint2(0, 0);
                 const uint64_t k = (p1 - p0 + 31u) / 32u;
                 for (uint32_t q = 0; q < 32u;) {
                     if (sum_is_inf(s)) return s;
-                    const uint32_t g = warp_sum_apply(s, q, false, ua, ub, SumStep{lp.x, lp.y}, SumStep{lp.z, lp.w},
-                                                      SumStep{lc.x, lc.y});
+                    const uint32_t g = warp_sum_apply(s, q, false, ua, ub, SumStep{lp.x, lp.y}, SumStep{lp.z, lp.w});
                     if (g >= 32u) break;
                     const uint64_t q0 = min(p0 + g * k, p1), q1 = min(q0 + k, p1);
                     s = warp_serial_add(s, x, q0, q1, buf);
                     q = g + 1;
                     sum_split(s, eu, m, top, Es);
-                    if (q < 32u && !guessed(eu)) {   // a binade nobody guessed: the rest one by one
+                    if (q < 32u && ua != eu && ub != eu) {   // a binade nobody guessed: the rest one by one
                         s = warp_serial_add(s, x, q1, p1, buf);
                         break;
                     }
@@ -304,7 +289,6 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
     static_assert(NT <= 256, "eight warps' pairs per block");
     constexpr uint32_t NW = NT / 32;
     __shared__ uint4 s_part[2][NW];
-    __shared__ uint2 s_part_c[2][NW];
     __shared__ __align__(16) float s_add[2][128];
     // the first kSumBlocks blocks take a slice each
     const uint32_t G = min(gridDim.x, kSumBlocks), b = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
@@ -322,38 +306,32 @@ __device__ __noinline__ bool grid_serial_sums(double *partials, const float *x0,
         if (tid == 0) SumScr(partials, G, j).slice[b] = own[j];
     }
     if (grid && !grid_barrier(gb, s_fail)) return false;
-    const double wide = fmin(0.5, (double)n * 0x1p-24);
     for (int j = 0; b < G && j < nsum; ++j) {
         const SumScr scr(partials, G, j);
         double v = 0.0;
         for (uint32_t k = tid; k < b; k += NT) v += __ldcg(scr.slice + k);
         const double P = broadcast_sum(block_sum<NT>(v, red));
-        const int32_t ua = sum_unit(P * (1.0 - wide)), ub = sum_unit((P + own[j]) * (1.0 + wide));
+        int32_t ua, ub;
+        sum_guess(P, own[j], n, ua, ub);
         const uint64_t p0 = min(hi, lo + w * LW), p1 = min(hi, p0 + LW);
-        const bool third = lo < hi && sum_third(ua, ub);   // the same in every warp
         SumStep A, B;
-        const size_t pw = (size_t)b * 8 + w;
-        warp_sum_steps(j ? x1 : x0, p0, p1, ua, ub, A, B, scr.lane + pw * 32);
+        warp_sum_steps(j ? x1 : x0, p0, p1, ua, ub, A, B, scr.lane + ((size_t)b * 8 + w) * 32);
         if (lane == 0) {
             const uint4 r = make_uint4(A.e, A.o, B.e, B.o);
             s_part[j][w] = r;
-            scr.part[pw] = r;
-        }
-        if (third) {
-            warp_sum_steps_c(j ? x1 : x0, p0, p1, ub - 1, A, scr.lane_c + pw * 32);
-            if (lane == 0) s_part_c[j][w] = scr.part_c[pw] = make_uint2(A.e, A.o);
+            scr.part[(size_t)b * 8 + w] = r;
         }
         __syncthreads();
         if (tid == 0) {
             SumRec r;
-            r.a = r.b = r.c = SumStep{0u, 0u};
+            r.a = r.b = SumStep{0u, 0u};
             for (uint32_t k = 0; k < NW; ++k) {
                 r.a = sum_compose(r.a, SumStep{s_part[j][k].x, s_part[j][k].y});
                 r.b = sum_compose(r.b, SumStep{s_part[j][k].z, s_part[j][k].w});
-                if (third) r.c = sum_compose(r.c, SumStep{s_part_c[j][k].x, s_part_c[j][k].y});
             }
             r.ua = lo < hi ? ua : kAnyUnit;
             r.ub = ub;
+            r.pad[0] = r.pad[1] = 0;
             scr.rec[b] = r;
         }
     }

@@ -1,5 +1,6 @@
 """Serial fp32 sums of 7M terms (csrc/serial_grid.cuh): so long a sum may drift
-from the f64 prefix by more than a binade, and its slices carry a third pair.
+from the f64 prefix by half of it, and its slices guess the prefix's own binade
+and the nearer neighbour.
 The one-launch loop's deltas against a launch per iteration, whose sums one
 block forms; the edge schedule's against the oracle."""
 import numpy as np
@@ -32,8 +33,8 @@ def test_node_schedule(bp, net, monkeypatch):
     for k in ("iterations", "delta", "previous_delta"):
         assert one[k] == launches[k], k
     assert one["serial_sums"] >= 4
-    # a slice that no pair fits is added by one warp, which takes a block as long
-    # as its own sums; with a third pair the loop took a sixtieth of that
+    # a slice that no guess fits is added by one warp, which takes as long as the
+    # one block's sums; guessed, the loop took a sixtieth of that
     assert 4 * one["elapsed_ms"] < launches["elapsed_ms"]
 
 
