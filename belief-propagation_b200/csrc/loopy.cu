@@ -1667,11 +1667,11 @@ static int block_min_blocks() {
     return (v == 10 || v == 16) ? v : 0;
 }
 
-template <int MS, bool UNI, int FU, int MB>
+template <int MS, bool UNI, int FU, int MB, bool SER = false>
 static int resident_blocks_mb(int *bps) {
     static int cached = 0;
     if (!cached)
-        BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached, k_flood<MS, UNI, FU, MB>, flood_nt<MS>(), 0));
+        BP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached, k_flood<MS, UNI, FU, MB, SER>, flood_nt<MS>(), 0));
     *bps = cached;
     return BP_OK;
 }
@@ -1732,7 +1732,7 @@ static cudaError_t launch_block_tiles(unsigned grid, bool overlap, cudaStream_t 
 // 273,000), 30.1 / 29.0 (4, 424,000); 0.4 full 24.8 / 23.6, 26.7 / 23.9, 28.3 /
 // 26.9.
 template <int MS, bool UNI>
-static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles, bool *overlap) {
+static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles, bool *overlap, bool serial) {
     *ntiles = grid_for(g->V, flood_nt<MS>());
     *grid = *ntiles;
     *overlap = false;
@@ -1743,6 +1743,12 @@ static int block_tiles(const bp_graph *g, unsigned *grid, uint32_t *ntiles, bool
         const int fu = block_unroll<MS>();
         st = fu == 1 ? resident_blocks<MS, UNI, 1>(&bps)
                      : (fu == 2 ? resident_blocks<MS, UNI, 2>(&bps) : resident_blocks<MS, UNI, 4>(&bps));
+    } else if (serial) {
+        // a form of its own with fewer blocks per SM: a grid of the f64 form's
+        // residency ran as one full wave and a partial one (3 states, 600,000
+        // nodes and 2.4M edges 267 us an iteration, 238 with its own)
+        constexpr int FU = flood_unroll<MS>();
+        st = resident_blocks_mb<MS, UNI, FU, flood_min_blocks_serial<MS, FU>(), true>(&bps);
     } else {
         st = resident_blocks<MS, UNI, flood_unroll<MS>()>(&bps);
     }
@@ -1950,7 +1956,7 @@ static int enqueue_node_iterations(bp_graph *g, uint32_t k, bool serial, int var
     uint32_t ntiles = 0;
     bool overlap = false;
     if (!warp_tiled) {
-        int st = block_tiles<MS, UNI>(g, &grid, &ntiles, &overlap);
+        int st = block_tiles<MS, UNI>(g, &grid, &ntiles, &overlap, serial);
         if (st) return st;
     }
     const FloodArgs a = flood_args(g);
@@ -2036,7 +2042,7 @@ static int flood_grid(bp_graph *g, int variant, uint32_t *grid, bool serial) {
     if (variant == BP_KERNEL_BLOCK_TILE) {
         uint32_t ntiles = 0;
         bool overlap = false;
-        auto tiles = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, block_tiles, g, grid, &ntiles, &overlap); };
+        auto tiles = [&]() -> int { BP_DISPATCH_MS(g->ms, g->uniform != 0, block_tiles, g, grid, &ntiles, &overlap, serial); };
         return tiles();
     }
     *grid = grid_for(g->V, 256);

@@ -30,3 +30,12 @@ def test_cluster_kernel_meets_before_it_touches_its_peers_shared_memory():
     body = _body(_code("batch_cluster.cuh"), r"k_batch_cluster\(")
     assert "map_shared_rank" in body
     assert "cluster.sync()" in body[:body.index("map_shared_rank")]
+
+
+def test_serial_launches_take_their_own_residency():
+    """A persistent grid larger than the kernel's own resident blocks runs as a
+    full wave and a partial one: the serial-delta form's grid is asked of the
+    serial-delta form."""
+    body = _body(_code("loopy.cu"), r"static int block_tiles\(")
+    serial = body[body.index("else if (serial)"):]
+    assert re.search(r"resident_blocks_mb<MS, UNI, FU, flood_min_blocks_serial<MS, FU>\(\), true>", serial)
