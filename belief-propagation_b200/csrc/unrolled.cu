@@ -1766,64 +1766,41 @@ int bp_unrolled_create(bp_unrolled **out, uint32_t V, uint32_t E, uint32_t S, ui
         u->own_stream = true;
     }
     // destination-sorted (stable) and source-sorted edge orders, on the host
-    std::vector<uint32_t> in_ptr(V + 1, 0), out_ptr(V + 1, 0), in_src(E), pos_out(E);
+    // one or two tables and up to 8 states: the adjoint in pull form (BP_UBWD_PULL=0: the scatter form)
+    u->pull = K <= (uint32_t)kPull2Tables && S <= 8 && ubwd_env("BP_UBWD_PULL", 1, 0) == 1;
+    // the pull form with two tables takes each node's out-edges by kind (table,
+    // then orientation)
+    const uint32_t nk = u->pull && K > 1 ? 2 * K : 1;
+    auto kind = [&](uint32_t e) { return nk == 1 ? 0u : 2u * (tab[e] & 0x7fu) + (tab[e] >> 7); };
+    std::vector<uint32_t> in_ptr(V + 1, 0), out_ptr(V + 1, 0), ofill((size_t)V * nk, 0), in_src(E);
     std::vector<uint8_t> ptab(E);
     for (uint32_t e = 0; e < E; ++e) {
         in_ptr[dst[e] + 1]++;
-        out_ptr[src[e] + 1]++;
+        ofill[(size_t)src[e] * nk + kind(e)]++;
     }
-    for (uint32_t v = 0; v < V; ++v) {
+    for (uint32_t v = 0, n = 0; v < V; ++v) {
         in_ptr[v + 1] += in_ptr[v];
-        out_ptr[v + 1] += out_ptr[v];
+        for (uint32_t k = 0; k < nk; ++k) {   // counts to first slots
+            const uint32_t c = ofill[(size_t)v * nk + k];
+            ofill[(size_t)v * nk + k] = n;
+            n += c;
+        }
+        out_ptr[v + 1] = n;
     }
-    std::vector<uint32_t> fill(in_ptr.begin(), in_ptr.end() - 1), pos_of(E);
+    std::vector<uint32_t> fill(in_ptr.begin(), in_ptr.end() - 1);
+    // pull form: destination and table of each source-sorted slot; scatter
+    // form: the slot of each position
+    std::vector<uint32_t> odst(u->pull ? E : 0), pos_out(u->pull ? 0 : E);
+    std::vector<uint8_t> otab(u->pull ? E : 0);
     for (uint32_t e = 0; e < E; ++e) {
-        const uint32_t p = fill[dst[e]]++;
-        pos_of[e] = p;
+        const uint32_t p = fill[dst[e]]++, q = ofill[(size_t)src[e] * nk + kind(e)]++;
         in_src[p] = src[e];
         ptab[p] = tab[e];
-    }
-    std::vector<uint32_t> ofill(out_ptr.begin(), out_ptr.end() - 1);
-    for (uint32_t e = 0; e < E; ++e) pos_out[pos_of[e]] = ofill[src[e]]++;
-    // one or two tables and up to 8 states: the adjoint in pull form (BP_UBWD_PULL=0: the scatter form)
-    u->pull = K <= (uint32_t)kPull2Tables && S <= 8 && ubwd_env("BP_UBWD_PULL", 1, 0) == 1;
-    std::vector<uint32_t> odst;
-    std::vector<uint8_t> otab;
-    if (u->pull) {
-        odst.resize(E);
-        otab.resize(E);
-        for (uint32_t e = 0; e < E; ++e) {
-            const uint32_t q = pos_out[pos_of[e]];
+        if (u->pull) {
             odst[q] = dst[e];
             otab[q] = tab[e];
-        }
-        // two tables: each node's out-edges by kind (table, then orientation)
-        auto kind = [](uint8_t t) { return 2u * (t & 0x7fu) + (t >> 7); };
-        std::vector<std::pair<uint8_t, uint32_t>> many;
-        for (uint32_t v = 0; K > 1 && v < V; ++v) {
-            const uint32_t a = out_ptr[v], b = out_ptr[v + 1];
-            if (b - a <= 32) {   // in place, by insertion
-                for (uint32_t q = a + 1; q < b; ++q) {
-                    const uint8_t t = otab[q];
-                    const uint32_t w = odst[q];
-                    uint32_t p = q;
-                    for (; p > a && kind(otab[p - 1]) > kind(t); --p) {
-                        otab[p] = otab[p - 1];
-                        odst[p] = odst[p - 1];
-                    }
-                    otab[p] = t;
-                    odst[p] = w;
-                }
-                continue;
-            }
-            many.clear();
-            for (uint32_t q = a; q < b; ++q) many.push_back({otab[q], odst[q]});
-            std::stable_sort(many.begin(), many.end(),
-                             [&](const auto &x, const auto &y) { return kind(x.first) < kind(y.first); });
-            for (uint32_t q = a; q < b; ++q) {
-                otab[q] = many[q - a].first;
-                odst[q] = many[q - a].second;
-            }
+        } else {
+            pos_out[p] = q;
         }
     }
     // stored messages (see UMsgs): one per node and table orientation in use,
