@@ -1054,9 +1054,13 @@ __global__ void __launch_bounds__(kPullThreads, MB) k_u_bwd_pull(
 // The scatter form it replaces takes a launch per table to recompute every
 // edge's sums for the table adjoint, on top of the step's own, and holds two
 // E x S slot arrays: 201 x 201 grid, 5 states, T = 10, forward and backward
-// 555 us with it, 270 us here.  Bound by each node's chain of loads (its
-// out-edges' Pbar, kind after kind) at 4 to 8 blocks of 4 warps per SM, as many
-// as the registers of S states leave without large spills.
+// 559 us with it, 208 us here.  5-8 states: the table adjoint's products and the
+// sums of eight of them are fp32, the rest f64, as in the scatter form.  Split
+// TF32 products on the tensor cores, as k_u_bwd_pull's, lost half a digit: error
+// of the table gradient against 64 bits 3.0e-7 (5 states, 40 x 40 grid, T = 1;
+// scatter form and now 1.5e-7), for 0-6 % of a step.  Bound by each node's chain
+// of loads (its out-edges' Pbar, kind after kind) at 4 to 8 blocks of 4 warps
+// per SM, as many as the registers of S states leave without large spills.
 constexpr int kPull2Tables = 2;
 template <int S> constexpr int pull2_min_blocks() { return S <= 2 ? 8 : (S <= 4 ? 6 : (S <= 6 ? 5 : 4)); }
 
@@ -1066,26 +1070,30 @@ __global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_p
     const float *__restrict__ x_next, const float *__restrict__ pbar_next, const float *__restrict__ lb_t,
     const float *__restrict__ gin, float *__restrict__ gout, float *__restrict__ pbar_out, double *__restrict__ epart) {
     static_assert(S >= 1 && S <= 8, "pull form: up to 8 states");
-    constexpr bool MMA = S >= 5;
+    // 5-8 states: lane l sums the entries l and l + 32 of the table adjoint over
+    // the warp's 32 nodes, staged a row of nodes per state
+    constexpr bool STAGE = S >= 5;
+    constexpr int EL = (S * S + 31) / 32, LD = 36;   // entries per lane; floats per row, 16-byte rows in different banks
     constexpr int KT = kPull2Tables, NT = kPullThreads, NW = NT / 32;
     __shared__ __align__(16) float sm[2 * KT * S * S];
-    __shared__ __align__(16) float st_n[MMA ? NW : 1][32][8];
-    __shared__ __align__(16) float st_t[MMA ? NW : 1][32][8];
-    __shared__ __align__(16) float st_e[MMA ? NW : 1][32][8];
-    __shared__ float dred[MMA ? NW : 1][16][8];
-    __shared__ float wred[NW][MMA ? 1 : S * S];
+    __shared__ __align__(16) float st_n[STAGE ? NW : 1][S][LD];
+    __shared__ __align__(16) float st_t[STAGE ? NW : 1][S][LD];
+    __shared__ __align__(16) float st_e[STAGE ? NW : 1][S][LD];
+    __shared__ double dred[STAGE ? NW : 1][S * S];
+    __shared__ float wred[NW][STAGE ? 1 : S * S];
     griddep_launch_dependents();
     load_tables_smem<S>(g, sm);
     griddep_wait();
     const bool edges = x_next != nullptr;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
-    float acc[KT][MMA ? 1 : S * S], d[KT][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float acc[KT][STAGE ? 1 : S * S];
+    double d[KT][EL];
 #pragma unroll
     for (int k = 0; k < KT; ++k) {
 #pragma unroll
-        for (int i = 0; i < (MMA ? 1 : S * S); ++i) acc[k][i] = 0.0f;
+        for (int i = 0; i < (STAGE ? 1 : S * S); ++i) acc[k][i] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) d[k][i] = 0.0f;
+        for (int i = 0; i < EL; ++i) d[k][i] = 0.0;
     }
     for (uint32_t base = (blockIdx.x * NW + warp) * 32u;; base += gridDim.x * (uint32_t)NT) {
         const uint32_t u = base + lane;
@@ -1144,42 +1152,36 @@ __global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_p
                     }
                 }
                 // table k's adjoint from cN and cT (zero on idle lanes)
-                if constexpr (!MMA) {
+                if constexpr (!STAGE) {
 #pragma unroll
                     for (int i = 0; i < S; ++i)
 #pragma unroll
                         for (int j = 0; j < S; ++j) acc[k][i * S + j] += cc[0][i] * e[j] + cc[1][j] * e[i];
                 } else {
-                    float pn[8], pt[8], pe[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        pn[i] = i < S ? cc[0][i < S ? i : 0] : 0.0f;
-                        pt[i] = i < S ? cc[1][i < S ? i : 0] : 0.0f;
-                        pe[i] = i < S ? e[i < S ? i : 0] : 0.0f;
-                    }
-                    reinterpret_cast<float4 *>(st_n[warp][lane])[0] = make_float4(pn[0], pn[1], pn[2], pn[3]);
-                    reinterpret_cast<float4 *>(st_n[warp][lane])[1] = make_float4(pn[4], pn[5], pn[6], pn[7]);
-                    reinterpret_cast<float4 *>(st_t[warp][lane])[0] = make_float4(pt[0], pt[1], pt[2], pt[3]);
-                    reinterpret_cast<float4 *>(st_t[warp][lane])[1] = make_float4(pt[4], pt[5], pt[6], pt[7]);
-                    if (k == 0) {
-                        reinterpret_cast<float4 *>(st_e[warp][lane])[0] = make_float4(pe[0], pe[1], pe[2], pe[3]);
-                        reinterpret_cast<float4 *>(st_e[warp][lane])[1] = make_float4(pe[4], pe[5], pe[6], pe[7]);
+                    for (int i = 0; i < S; ++i) {
+                        st_n[warp][i][lane] = cc[0][i];
+                        st_t[warp][i][lane] = cc[1][i];
+                        if (k == 0) st_e[warp][i][lane] = e[i];
                     }
                     __syncwarp();
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        const int k0 = h * 8 + tq, k1 = k0 + 4;
-                        const float af[4] = {st_n[warp][k0][gq], st_t[warp][k0][gq], st_n[warp][k1][gq],
-                                             st_t[warp][k1][gq]};
-                        const float bf[2] = {st_e[warp][k0][gq], st_e[warp][k1][gq]};
-                        uint32_t ah[4], al[4], bh[2], bl[2];
+                    for (int q2 = 0; q2 < EL; ++q2) {
+                        const int at = lane + 32 * q2;
+                        if (at >= S * S) break;
+                        const int i = at / S, j = at % S;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) split_tf32(af[i], ah[i], al[i]);
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) split_tf32(bf[i], bh[i], bl[i]);
-                        mma_tf32_16x8x8(d[k], ah, bh);
-                        mma_tf32_16x8x8(d[k], ah, bl);
-                        mma_tf32_16x8x8(d[k], al, bh);
+                        for (int n = 0; n < 32; n += 4) {
+                            const float4 cn = *reinterpret_cast<const float4 *>(&st_n[warp][i][n]);
+                            const float4 ct = *reinterpret_cast<const float4 *>(&st_t[warp][j][n]);
+                            const float4 ej = *reinterpret_cast<const float4 *>(&st_e[warp][j][n]);
+                            const float4 ei = *reinterpret_cast<const float4 *>(&st_e[warp][i][n]);
+                            float t = cn.x * ej.x + ct.x * ei.x;
+                            t += cn.y * ej.y + ct.y * ei.y;
+                            t += cn.z * ej.z + ct.z * ei.z;
+                            t += cn.w * ej.w + ct.w * ei.w;
+                            d[k][q2] += (double)t;
+                        }
                     }
                     __syncwarp();
                 }
@@ -1218,18 +1220,15 @@ __global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_p
     for (int k = 0; k < KT; ++k) {
         double *row = epart + ((size_t)k * gridDim.x + blockIdx.x) * S * S;
         const float *J = sm + 2 * k * S * S;
-        if constexpr (MMA) {
-            dred[warp][gq][2 * tq] = d[k][0];
-            dred[warp][gq][2 * tq + 1] = d[k][1];
-            dred[warp][gq + 8][2 * tq] = d[k][2];
-            dred[warp][gq + 8][2 * tq + 1] = d[k][3];
+        if constexpr (STAGE) {
+#pragma unroll
+            for (int q2 = 0; q2 < EL; ++q2)
+                if (lane + 32 * q2 < S * S) dred[warp][lane + 32 * q2] = d[k][q2];
             __syncthreads();
-            // logJbar[a][b] += J[a][b] * (N[a][b] + T[b][a])
             for (int i = threadIdx.x; i < S * S; i += NT) {
-                const int ra = i / S, cb = i % S;
                 double t = 0.0;
-                for (int w = 0; w < NW; ++w) t += (double)dred[w][ra][cb] + (double)dred[w][8 + cb][ra];
-                row[i] += (double)J[ra * S + cb] * t;
+                for (int w = 0; w < NW; ++w) t += dred[w][i];
+                row[i] += (double)J[i] * t;
             }
         } else {
             block_partial_add<S, NT, true>(acc[k], nullptr, wred, row, J);

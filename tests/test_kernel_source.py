@@ -39,3 +39,10 @@ def test_serial_launches_take_their_own_residency():
     body = _body(_code("loopy.cu"), r"static int block_tiles\(")
     serial = body[body.index("else if (serial)"):]
     assert re.search(r"resident_blocks_mb<MS, UNI, FU, flood_min_blocks_serial<MS, FU>\(\), true>", serial)
+
+
+def test_two_table_adjoint_multiplies_in_fp32():
+    """Its scatter form multiplies fp32 operands; split into two TF32 parts
+    without their low product they carry up to seven times the error."""
+    body = _body(_code("unrolled.cu"), r"k_u_bwd_pull2\(")
+    assert "tf32" not in body and "mma" not in body.lower()
