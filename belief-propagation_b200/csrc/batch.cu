@@ -401,6 +401,9 @@ struct bp_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     std::vector<bpx::NetInfo> info;
+    // the launch of the last solve or tuning (of the default options until
+    // then) gives large networks a cluster: the f64 delta without block_threads
+    bool clusters = true;
     uint64_t totV = 0, totE = 0, totNodeF = 0, totMsgF = 0, totJointF = 0, totPtr = 0;
     bpx::NetInfo *d_info = nullptr;
     uint32_t *in_ptr = nullptr, *in_src = nullptr, *pos_edge = nullptr, *net_of_edge = nullptr;
@@ -427,15 +430,21 @@ namespace bpx {
 constexpr uint32_t kClusterEdges = 1024;
 constexpr uint32_t kDefaultBlock = 256;   // threads per network block, until tuned
 
-// the cluster launch of the group's large networks, and a block each for the
-// rest (every network with the serial delta)
+// the group's networks that the launch solves by a cluster each, the first of
+// `order`; the rest get a block each
+static uint32_t cluster_networks(const bp_batch *bt, const Group &gr) { return bt->clusters ? gr.large : 0u; }
+
+// clusters in flight for the group: as many as the resident blocks make
+static uint32_t cluster_count(const bp_batch *bt, const Group &gr) {
+    return std::min<uint32_t>(cluster_networks(bt, gr),
+                              (uint32_t)std::max(1, kClusterPerSm * bt->sm_count / kBatchCluster));
+}
+
+// the cluster launch of the group's large networks
 template <int S>
 static int launch_large(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, cudaStream_t s) {
     BP_CUDA(cudaFuncSetAttribute(k_batch_cluster<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem));
-    // as many clusters as the resident blocks make
-    const uint32_t clusters =
-        std::min<uint32_t>(gr.large, (uint32_t)std::max(1, kClusterPerSm * bt->sm_count / kBatchCluster));
-    k_batch_cluster<S><<<clusters * kBatchCluster, kClusterThreads, kClusterSmem, s>>>(a, gr.d_order, gr.large,
+    k_batch_cluster<S><<<cluster_count(bt, gr) * kBatchCluster, kClusterThreads, kClusterSmem, s>>>(a, gr.d_order, gr.large,
                                                                                      bt->queues + bt->groups.size() + gi);
     BP_CUDA(cudaGetLastError());
     return BP_OK;
@@ -444,7 +453,7 @@ static int launch_large(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi
 template <int S>
 static int launch_group(bp_batch *bt, Group &gr, const BatchArgs &a, uint32_t gi, uint32_t block, uint32_t grid,
                         cudaStream_t s) {
-    const uint32_t skip = a.serial ? 0u : gr.large, rest = (uint32_t)gr.order.size() - skip;
+    const uint32_t skip = cluster_networks(bt, gr), rest = (uint32_t)gr.order.size() - skip;
     if (!rest) return BP_OK;
     if (a.serial)
         k_batch_solve<S, true><<<grid, block, sizeof(float) * 2 * a.sum_ch, s>>>(a, gr.d_order, rest, bt->queues + gi);
@@ -561,7 +570,8 @@ static int enqueue_batch(bp_batch *bt, const BatchArgs &a) {
         const bool large = k < ng;
         const size_t gi = large ? k : k - ng;
         Group &gr = bt->groups[gi];
-        if (large ? (a.serial || !gr.large) : (!a.serial && gr.large == gr.order.size())) continue;
+        const uint32_t by_cluster = cluster_networks(bt, gr);
+        if (large ? !by_cluster : by_cluster == gr.order.size()) continue;
         cudaStream_t s = bt->side[k];
         BP_CUDA(cudaStreamWaitEvent(s, bt->fork_ev, 0));
         int st;
@@ -780,7 +790,7 @@ constexpr int kTuneRevision = 6;
 static std::string tune_key(bp_batch *bt, const Group &gr, int serial) {
     // the networks that run a block each
     uint64_t V = 0, E = 0;
-    const size_t skip = serial ? 0 : gr.large;
+    const size_t skip = cluster_networks(bt, gr);
     for (size_t k = skip; k < gr.order.size(); ++k) {
         V += bt->info[gr.order[k]].V;
         E += bt->info[gr.order[k]].E;
@@ -888,7 +898,7 @@ static int time_trial(bp_batch *bt, const TuneState &keep, F launch, float *ms) 
 static int tune_blocks(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
     for (size_t gi = 0; gi < bt->groups.size(); ++gi) {
         Group &gr = bt->groups[gi];
-        if (!a.serial && gr.large == gr.order.size()) continue;   // clusters only: nothing to tune
+        if (cluster_networks(bt, gr) == gr.order.size()) continue;   // clusters only: nothing to tune
         const std::string key = tune_key(bt, gr, a.serial);
         uint32_t best_grid = 0;
         uint32_t best = cache_lookup(key, &best_grid);
@@ -1085,6 +1095,7 @@ int bp_batch_autotune(bp_batch *bt, const bp_batch_options *o) {
     if (!bt || !o) return set_error(BP_ERR_INVALID, "null argument");
     const int serial = o->delta_mode == BP_DELTA_SERIAL_F32;
     if (serial && !bt->absdiff) BP_CUDA(cudaMalloc((void **)&bt->absdiff, sizeof(float) * 2 * (bt->totMsgF + 4)));
+    bt->clusters = !serial;
     TuneState keep;
     int st = keep.save(bt);
     if (!st) {
@@ -1105,24 +1116,19 @@ int bp_batch_get_groups(const bp_batch *bt, uint32_t *states, uint32_t *max_node
     if (!bt || !count) return set_error(BP_ERR_INVALID, "null argument");
     const uint32_t n = (uint32_t)bt->groups.size();
     for (uint32_t i = 0; i < n && i < *count; ++i) {
-        if (states) states[i] = (uint32_t)bt->groups[i].S;
-        if (max_nodes) max_nodes[i] = bt->groups[i].vmax;
-        if (block) block[i] = bt->groups[i].block;
-        if (grid) grid[i] = bt->groups[i].grid;
+        const Group &gr = bt->groups[i];
+        const uint32_t rest = (uint32_t)gr.order.size() - cluster_networks(bt, gr);
+        if (states) states[i] = (uint32_t)gr.S;
+        if (max_nodes) max_nodes[i] = gr.vmax;
+        if (block) block[i] = rest ? gr.block : (uint32_t)kClusterThreads;
+        if (grid) grid[i] = cluster_count(bt, gr) * kBatchCluster + std::min(gr.grid, rest);
     }
     *count = n;
     return BP_OK;
 }
 
 int bp_batch_get_block_threads(const bp_batch *bt, uint32_t *states, uint32_t *block, uint32_t *count) {
-    if (!bt || !count) return set_error(BP_ERR_INVALID, "null argument");
-    const uint32_t n = (uint32_t)bt->groups.size();
-    for (uint32_t i = 0; i < n && i < *count; ++i) {
-        if (states) states[i] = (uint32_t)bt->groups[i].S;
-        if (block) block[i] = bt->groups[i].block;
-    }
-    *count = n;
-    return BP_OK;
+    return bp_batch_get_groups(bt, states, nullptr, block, nullptr, count);
 }
 
 int bp_batch_loopy(bp_batch *bt, const bp_batch_options *o, bp_batch_result *r) {
@@ -1152,12 +1158,14 @@ int bp_batch_loopy(bp_batch *bt, const bp_batch_options *o, bp_batch_result *r) 
             }
     }
     if (o->max_iterations == 0) return set_error(BP_ERR_INVALID, "max_iterations must be at least 1");
+    bt->clusters = !serial && !o->block_threads;
     // one CUDA graph per (options, tiling): the queue reset and every group's launch
     uint64_t key = (uint64_t)o->max_iterations | ((uint64_t)serial << 32) | ((uint64_t)(o->init_messages != 0) << 33);
     uint32_t tb;
     memcpy(&tb, &o->tolerance, 4);
     key ^= (uint64_t)tb << 34;
     for (auto &gr : bt->groups) key = key * 1000003ull + gr.block;
+    key = key * 1000003ull + (bt->clusters ? 1u : 0u);
     if (!bt->exec || bt->exec_key != key) {
         if (bt->exec) {
             cudaGraphExecDestroy(bt->exec);

@@ -192,8 +192,9 @@ class BPGraph:
 
 
 class BPBatch:
-    """Many independent networks solved together (bp_batch): one persistent
-    launch per state count, each network with its own stopping rule."""
+    """Many independent networks solved together (bp_batch): persistent
+    launches per state count, a thread block or (large networks, f64 delta) a
+    cluster of eight per network, each with its own stopping rule."""
 
     def __init__(self, nets, stream=None):
         self.lib = N.load()
@@ -267,6 +268,8 @@ class BPBatch:
         return flat[a:a + net.E * S].reshape(net.E, S)
 
     def options(self, tol=1e-4, max_iterations=200, delta="f64", block_threads=0, init=True):
+        """block_threads: a block of so many threads for every network, none
+        by a cluster; 0 leaves both as created or tuned."""
         o = N.BatchOptions()
         self.lib.bp_batch_default_options(C.byref(o))
         o.tolerance, o.max_iterations = float(tol), int(max_iterations)
@@ -280,7 +283,8 @@ class BPBatch:
 
     def groups(self):
         """The launch groups: state count, size bound (0 = the larger
-        networks), threads per block and blocks in flight, launch order."""
+        networks), threads per block and blocks in flight, launch order; of
+        the last solve or tuning."""
         n = C.c_uint32(64)
         st, vm, bl, gr = (np.zeros(64, np.uint32) for _ in range(4))
         N.check(self.lib.bp_batch_get_groups(self.h, st.ctypes.data, vm.ctypes.data, bl.ctypes.data, gr.ctypes.data,

@@ -301,10 +301,12 @@ int bp_get_visited(bp_graph *g, char *visited);       /* host [V] */
 
 /* ---- batched loopy BP -------------------------------------------------- */
 /* Many independent networks, each with its own stopping rule
- * (loopy_propagate_until per network), solved in one persistent launch per
- * state count: a thread block takes the next network from a work queue
- * (largest first) and iterates it to convergence.  Each network's result is
- * what bp_loopy gives for it alone.  Every node of one network has the same
+ * (loopy_propagate_until per network), solved in persistent launches per
+ * state count: a thread block, or with the f64 delta a cluster of 8 blocks for
+ * a network of at least 1024 edges (BP_BATCH_CLUSTER_EDGES, read at create; 0:
+ * none), takes the next network from a work queue (largest first) and iterates
+ * it to convergence.  Each network's result is what bp_loopy gives for it
+ * alone.  Every node of one network has the same
  * state count; networks may differ.
  *
  * Layout of the batch-wide arrays (bp_batch_layout): network n's beliefs are
@@ -317,7 +319,8 @@ typedef struct {
     float tolerance;          /* per network, the reference's `convergence` */
     uint32_t max_iterations;  /* per network */
     int32_t delta_mode;       /* BP_DELTA_F64 (default) or BP_DELTA_SERIAL_F32 */
-    uint32_t block_threads;   /* threads per network block; 0 = as tuned (bp_batch_autotune) */
+    uint32_t block_threads;   /* a block of so many threads for every network, no clusters;
+                               * 0 = as tuned (bp_batch_autotune) */
     int32_t init_messages;    /* 1: init_previous_edge first */
     int32_t reserved;
 } bp_batch_options;
@@ -349,12 +352,15 @@ void bp_batch_default_options(bp_batch_options *o);
  * per network, and keeps the fastest (results cached in $BP_AUTOTUNE_CACHE,
  * default ~/.cache/bp_b200_autotune.txt); beliefs and messages are restored */
 int bp_batch_autotune(bp_batch *b, const bp_batch_options *o);
-/* per group (at most *count entries; *count returns the number of groups):
- * its state count and threads per block (a state count appears once per size
+/* per group (at most *count entries; *count returns the number of groups) the
+ * launch of the last solve or tuning, before these of the default options: its
+ * state count and threads per block -- of the networks solved by a block each,
+ * or of the clusters' blocks where none is (a state count appears once per size
  * class) */
 int bp_batch_get_block_threads(const bp_batch *b, uint32_t *states, uint32_t *block, uint32_t *count);
 /* per group as above, plus max_nodes: the group's size bound (0 = none, the
- * group of larger networks) and grid: its blocks in flight */
+ * group of larger networks) and grid: its blocks in flight, those of its
+ * clusters among them */
 int bp_batch_get_groups(const bp_batch *b, uint32_t *states, uint32_t *max_nodes, uint32_t *block, uint32_t *grid,
                         uint32_t *count);
 /* the whole batch: one CUDA graph launch */
