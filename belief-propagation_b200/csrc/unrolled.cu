@@ -1117,6 +1117,7 @@ __global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_p
 #pragma unroll
             for (int k = 0; k < KT; ++k) {
                 float cc[2][S];
+                const uint32_t qk = q;
 #pragma unroll
                 for (int o = 0; o < 2; ++o) {
                     float *c = cc[o];
@@ -1151,18 +1152,22 @@ __global__ void __launch_bounds__(kPullThreads, pull2_min_blocks<S>()) k_u_bwd_p
                         }
                     }
                 }
-                // table k's adjoint from cN and cT (zero on idle lanes)
+                // table k's adjoint from cN and cT; a node without out-edges of
+                // the table adds nothing, also where its state is NaN
+                float ek[S];
+#pragma unroll
+                for (int i = 0; i < S; ++i) ek[i] = q > qk ? e[i] : 0.0f;
                 if constexpr (!STAGE) {
 #pragma unroll
                     for (int i = 0; i < S; ++i)
 #pragma unroll
-                        for (int j = 0; j < S; ++j) acc[k][i * S + j] += cc[0][i] * e[j] + cc[1][j] * e[i];
+                        for (int j = 0; j < S; ++j) acc[k][i * S + j] += cc[0][i] * ek[j] + cc[1][j] * ek[i];
                 } else {
 #pragma unroll
                     for (int i = 0; i < S; ++i) {
                         st_n[warp][i][lane] = cc[0][i];
                         st_t[warp][i][lane] = cc[1][i];
-                        if (k == 0) st_e[warp][i][lane] = e[i];
+                        st_e[warp][i][lane] = ek[i];
                     }
                     __syncwarp();
 #pragma unroll
