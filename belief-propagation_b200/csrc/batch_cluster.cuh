@@ -23,9 +23,6 @@
 // of 24 warps per SM and a cluster barrier per iteration.
 #pragma once
 
-#ifndef XU
-#define XU 4
-#endif
 constexpr int kBatchCluster = 8;           // the largest portable cluster
 constexpr int kClusterThreads = 256;
 constexpr int kClusterPerSm = 3;           // resident blocks per SM

@@ -64,8 +64,7 @@ struct LoopyCtl {
     // set by a block of a one-launch loop whose bounded barrier wait ran out
     uint32_t bar_fail;
     // test hook of that bounded wait (BP_DEBUG_BARRIER_SKIP): block
-    // bar_skip - 1 does not arrive at the first barrier, so the others' waits
-    // run out; 0 = off
+    // bar_skip - 1 arrives at no barrier, so the others' waits run out; 0 = off
     uint32_t bar_skip;
     // serial mode: the reference's fp32 sum of a check's |diff| terms lies
     // in [dlo, dhi] (f64 sum of the terms +- the serial sum's rounding bound),
@@ -76,9 +75,7 @@ struct LoopyCtl {
     double dlo, dhi, plo, phi;
     uint32_t delta_exact, prev_exact, cur_buf, prev_buf;
     uint32_t serial_sums;  // serial sums formed because the bound could not decide
-    // the one-launch loop: block 0's serial sums for the other blocks
-    uint32_t fb_pform;     // the previous delta was formed too
-    float fb_s, fb_p;
+    float fb_s, fb_p;      // the one-launch loops: block 0's serial sums for the other blocks
     // [dlo, dhi] / [plo, phi] narrowed from the terms' own rounding errors
     uint32_t delta_ref, prev_ref;
     uint32_t serial_refines;   // checks that needed the narrowed interval

@@ -1301,7 +1301,7 @@ struct bp_unrolled {
     float *bT = nullptr;
     float *bbar[2] = {nullptr, nullptr};
     float *xc[2] = {nullptr, nullptr};       // [E][S] x adjoint terms, source-sorted slots (scatter form)
-    bool pull = false;                       // the adjoint in pull form (one table, S <= 8)
+    bool pull = false;                       // the adjoint in pull form (at most two tables, S <= 8)
     uint32_t *out_dst = nullptr;             // [E] destination of source-sorted slot q (pull form)
     uint8_t *out_tab = nullptr;              // [E] its table id (pull form)
     float *pbv[2] = {nullptr, nullptr};      // [V][S] Pbar of steps t and t+1 (pull form)
@@ -1453,7 +1453,7 @@ static int u_recompute(bp_unrolled *u, const UGraph &g, uint32_t s) {
 
 // the backward on the engine's own buffers (bbar[0] holds d loss / d lb_T on
 // entry; gtheta_buf, glogp_buf receive the gradients)
-// the backward in pull form (one table, S <= 8; see k_u_bwd_pull): kernel t
+// the backward in pull form (at most two tables, S <= 8; see k_u_bwd_pull and k_u_bwd_pull2): kernel t
 // finishes step t+1's edges and runs step t's node step; then the initial
 // gather (mode 1) and the priors (mode 2).  Recompute and segment buffers as
 // in the scatter form below.
