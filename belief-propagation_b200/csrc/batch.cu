@@ -424,10 +424,70 @@ struct bp_batch {
 
 namespace bpx {
 
-// networks of at least this many edges are solved by a cluster each (f64
-// delta; below, a block's own latency is about the cluster barrier's and more
-// networks run side by side); BP_BATCH_CLUSTER_EDGES overrides (0: none)
+// networks of at least this many edges can be solved by a cluster each (f64
+// delta; below, a block's own latency is about the cluster barrier's);
+// BP_BATCH_CLUSTER_EDGES=n gives one to every network of n edges or more (0:
+// none), without it clusters_pay decides for the batch
 constexpr uint32_t kClusterEdges = 1024;
+
+// clusters in flight, and an iteration's cost by state count: of a network by
+// a block, in a full GPU (ps an edge) and alone (ns an edge), and of one by a
+// cluster in a full GPU (ps an edge, tables in shared memory or from L2, beside
+// kClusterBase)
+static uint32_t cluster_slots(const bp_batch *bt) {
+    return (uint32_t)std::max(1, kClusterPerSm * bt->sm_count / kBatchCluster);
+}
+struct SolveCost {
+    float block, block_alone, cluster, cluster_l2;
+};
+constexpr SolveCost kSolveCost[BP_MAX_STATES + 1] = {
+    {}, {7, 2.0f, 6, 8}, {10, 2.4f, 10, 14}, {17, 3.5f, 20, 33}, {22, 3.9f, 10, 30}, {60, 8.0f, 37, 110},
+    {68, 7.7f, 30, 140}, {165, 17, 65, 325}, {120, 13.7f, 27, 70}, {280, 27, 90, 730}, {330, 29, 58, 600}};
+constexpr double kClusterBase = 65e3;   // ps
+
+// Whether the batch's large networks get clusters.  A cluster shortens one
+// network's iterations three to eight times, but 55 of them fill the GPU that
+// holds a thousand blocks: us per iteration of equal networks by blocks /
+// clusters, 1200 edges of 2 states 3.9 / 3.2 (30 networks), 4.2 / 11.9 (150),
+// 12.5 / 76.7 (1200); of 8 states 17 / 4.0, 30 / 16, 134 / 108; 9600 edges of 2
+// states 27 / 6.7, 42 / 27, 136 / 183.  So: while every large network has a
+// cluster at once, yes; else by the two estimated times, each the longer of all
+// the work at a full GPU's rate and the longest network (which others on its SM
+// hold up once there are more networks than SMs).  On the 392 batches that the
+// costs were fitted to (1 to 1200 equal networks of 1200-19,200 edges by state
+// count; 16 to 3000 networks of log-uniform sizes and mixed states) the choice
+// loses more than 10 % to the other in 15; the geometric mean over the better one
+// is 1.012, with clusters always 1.23 and blocks always 1.67.  On 56 others:
+// 1.018, and 1.10 with clusters always.
+static bool clusters_pay(const bp_batch *bt, uint32_t least) {
+    double work_b = 0.0, longest_b = 0.0, work_c = 0.0, longest_small = 0.0, largest_c = 0.0;   // ps
+    uint32_t large = 0;
+    for (const auto &gr : bt->groups)
+        for (const uint32_t x : gr.order) {
+            const double E = bt->info[x].E;
+            const SolveCost &k = kSolveCost[gr.S];
+            const double work = E * k.block, alone = 1.2e6 + E * k.block_alone * 1e3;
+            work_b += work;
+            longest_b = std::max(longest_b, alone);
+            if (bt->info[x].E < least) {
+                work_c += work;
+                longest_small = std::max(longest_small, alone);
+                continue;
+            }
+            ++large;
+            const bool fit = cluster_tables_fit((uint32_t)gr.S, bt->info[x].E);
+            const double c = kClusterBase + E * (fit ? k.cluster : k.cluster_l2);
+            work_c += c;
+            largest_c = std::max(largest_c, c);
+        }
+    const uint32_t slots = cluster_slots(bt);
+    if (large <= slots) return true;
+    const bool shared = bt->N > (uint32_t)bt->sm_count;
+    const double blocks = std::max(work_b, longest_b + (shared ? std::min(work_b, longest_b) : 0.0));
+    // the last clusters run a quarter of their time without the others
+    const double clusters = std::max(work_c + 0.25 * slots * largest_c, longest_small);
+    return clusters < 1.15 * blocks;
+}
 constexpr uint32_t kDefaultBlock = 256;   // threads per network block, until tuned
 
 // the group's networks that the launch solves by a cluster each, the first of
@@ -436,8 +496,7 @@ static uint32_t cluster_networks(const bp_batch *bt, const Group &gr) { return b
 
 // clusters in flight for the group: as many as the resident blocks make
 static uint32_t cluster_count(const bp_batch *bt, const Group &gr) {
-    return std::min<uint32_t>(cluster_networks(bt, gr),
-                              (uint32_t)std::max(1, kClusterPerSm * bt->sm_count / kBatchCluster));
+    return std::min<uint32_t>(cluster_networks(bt, gr), cluster_slots(bt));
 }
 
 // the cluster launch of the group's large networks
@@ -751,6 +810,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
     }
     const char *env = getenv("BP_BATCH_CLUSTER_EDGES");
     const uint32_t least = env ? (uint32_t)strtoul(env, nullptr, 10) : kClusterEdges;
+    const bool pay = env || clusters_pay(bt, least);
     for (auto &gr : bt->groups) {
         std::stable_sort(gr.order.begin(), gr.order.end(), [&](uint32_t x, uint32_t y) { return work(x) > work(y); });
         gr.block = kDefaultBlock;
@@ -760,7 +820,8 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
             // by edges up to the nodes' share)
             auto mid = std::stable_partition(gr.order.begin(), gr.order.end(),
                                              [&](uint32_t x) { return bt->info[x].E >= least; });
-            gr.large = gr.large_n = (uint32_t)(mid - gr.order.begin());
+            gr.large_n = (uint32_t)(mid - gr.order.begin());
+            gr.large = pay ? gr.large_n : 0;
         }
         BP_CUDA(cudaMalloc((void **)&gr.d_order, sizeof(uint32_t) * gr.order.size()));
         BP_CUDA(cudaMemcpyAsync(gr.d_order, gr.order.data(), sizeof(uint32_t) * gr.order.size(),
@@ -785,7 +846,7 @@ static int batch_create_impl(bp_batch *bt, uint32_t N, const bp_graph_desc *desc
 // ---- autotuning of threads per block, cached on disk ---------------------
 // kernel revision in the autotune key: a cached block size belongs to the
 // kernel it was timed on
-constexpr int kTuneRevision = 6;
+constexpr int kTuneRevision = 7;
 
 static std::string tune_key(bp_batch *bt, const Group &gr, int serial) {
     // the networks that run a block each
@@ -936,7 +997,7 @@ static int tune_blocks(bp_batch *bt, const BatchArgs &a, const TuneState &keep) 
 }
 
 // how a batch with networks large enough for clusters is launched
-enum BatchPlan : uint32_t { kPlanClusters = 1, kPlanClustersTuned = 2, kPlanBlocksTuned = 3 };
+enum BatchPlan : uint32_t { kPlanClusters = 1, kPlanClustersTuned = 2, kPlanBlocksTuned = 3, kPlanBlocks = 4 };
 
 // the launch of a plan: clusters for the large networks or a block for every
 // one, with the launch shape that batch_create_impl gives
@@ -951,8 +1012,9 @@ static void set_plan(bp_batch *bt, bool clusters) {
 // One group's best launch alone need not be the batch's, whose groups run side
 // by side, and clusters shorten the longest networks while blocks with a tuned
 // number in flight keep more of each network on its SM.  So whole batches are
-// timed: as created, clusters with the rest tuned, and tuned blocks for all,
-// the last only where untuned blocks come within twice the clusters' time
+// timed: clusters, clusters with the rest tuned, blocks for all, and tuned
+// blocks for all, the last only where the untuned come within twice the
+// clusters' time
 // (tuning has gained them 1.6x: 4096 networks 178 -> 112 ms, clusters 116;
 // 1024 networks 104, clusters 29).
 static int tune_batch(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
@@ -970,10 +1032,10 @@ static int tune_batch(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
     uint32_t unused = 0, plan = cache_lookup(key, &unused);
     if (!plan) {
         auto whole = [&](float *ms) { return time_trial(bt, keep, [&] { return enqueue_batch(bt, a); }, ms); };
-        float created = 0.0f, blocks = 0.0f, ms = 0.0f, best = 0.0f;
-        if ((st = whole(&created))) return st;
+        float clusters = 0.0f, blocks = 0.0f, ms = 0.0f, best = 0.0f;
+        if ((st = whole(&clusters))) return st;
         plan = kPlanClusters;
-        best = created;
+        best = clusters;
         if ((st = tune_blocks(bt, a, keep)) || (st = whole(&ms))) return st;
         if (ms < best) {
             plan = kPlanClustersTuned;
@@ -981,14 +1043,18 @@ static int tune_batch(bp_batch *bt, const BatchArgs &a, const TuneState &keep) {
         }
         set_plan(bt, false);
         if ((st = whole(&blocks))) return st;
-        if (blocks < 2.0f * created) {
+        if (blocks < best) {
+            plan = kPlanBlocks;
+            best = blocks;
+        }
+        if (blocks < 2.0f * clusters) {
             if ((st = tune_blocks(bt, a, keep)) || (st = whole(&ms))) return st;
             if (ms < best) plan = kPlanBlocksTuned;
         }
         cache_store(key, plan, 0);
     }
-    set_plan(bt, plan != kPlanBlocksTuned);
-    return plan == kPlanClusters ? BP_OK : tune_blocks(bt, a, keep);
+    set_plan(bt, plan == kPlanClusters || plan == kPlanClustersTuned);
+    return plan == kPlanClusters || plan == kPlanBlocks ? BP_OK : tune_blocks(bt, a, keep);
 }
 
 }  // namespace bpx

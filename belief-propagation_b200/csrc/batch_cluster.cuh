@@ -13,6 +13,8 @@
 // iteration orders both, and every block takes the same stopping decision
 // from the same partials in rank order.
 //
+// Which batches take clusters: clusters_pay (batch.cu).
+//
 // 1024 networks of 32-4096 nodes, 2-8 states, 200 iterations at most: 103 ms
 // with a block per network, 26.7 ms with clusters from 1024 edges on (28.4 from
 // 512, 30.2 from 2048, 51 from 4096).  Blocks per SM, their threads and shared
@@ -30,8 +32,15 @@ constexpr uint32_t kClusterSmem = 70u << 10;
 
 // floats between tables in shared memory: 16-byte rows whose starts fall in
 // different banks for eight consecutive edges
-template <int S> constexpr uint32_t cluster_table_stride() {
+constexpr uint32_t cluster_table_stride(uint32_t S) {
     return (S * S) % 4 ? S * S : ((S * S) % 8 ? S * S : (S == 2 ? 4 : S * S + 4));
+}
+
+// whether the tables of a network's block fit its shared memory beside the
+// messages and source ids (a block of ne edges, an eighth of the network's)
+inline bool cluster_tables_fit(uint32_t S, uint32_t E) {
+    const uint64_t ne = E / kBatchCluster + 1;
+    return 4 * ne * (2 * S + 1 + cluster_table_stride(S)) + 64 <= kClusterSmem;
 }
 
 template <int S>
@@ -91,7 +100,7 @@ __device__ __forceinline__ void cluster_send(const float *__restrict__ J, const 
 template <int S>
 __device__ void cluster_solve(const BatchArgs &a, uint32_t n, cooperative_groups::cluster_group &cluster, float *dyn,
                               double (*part)[kBatchCluster], double *red, uint32_t *bound) {
-    constexpr uint32_t T = kClusterThreads, C = kBatchCluster, TS = cluster_table_stride<S>();
+    constexpr uint32_t T = kClusterThreads, C = kBatchCluster, TS = cluster_table_stride(S);
     const NetInfo ni = a.info[n];
     const uint32_t V = ni.V, E = ni.E, tid = threadIdx.x, rank = cluster.block_rank();
     const uint32_t *ptr = a.in_ptr + ni.ptr_off;

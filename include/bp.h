@@ -303,9 +303,10 @@ int bp_get_visited(bp_graph *g, char *visited);       /* host [V] */
 /* Many independent networks, each with its own stopping rule
  * (loopy_propagate_until per network), solved in persistent launches per
  * state count: a thread block, or with the f64 delta a cluster of 8 blocks for
- * a network of at least 1024 edges (BP_BATCH_CLUSTER_EDGES, read at create; 0:
- * none), takes the next network from a work queue (largest first) and iterates
- * it to convergence.  Each network's result is what bp_loopy gives for it
+ * a network of at least 1024 edges in a batch that is estimated faster so
+ * (BP_BATCH_CLUSTER_EDGES=n, read at create: every network of n edges or more;
+ * 0: none), takes the next network from a work queue (largest first) and
+ * iterates it to convergence.  Each network's result is what bp_loopy gives for it
  * alone.  Every node of one network has the same
  * state count; networks may differ.
  *
