@@ -55,6 +55,18 @@ template <int MS, int FU> constexpr int flood_min_blocks() { return MS <= 2 ? (F
 // the serial-delta form carries the serial sum's code: a cap would spill
 template <int MS, int FU> constexpr int flood_min_blocks_serial() { return MS <= 2 ? flood_min_blocks<MS, FU>() : 1; }
 
+// the one-launch form of the same tiles (k_flood_fused): a graph takes it while
+// all its tiles are resident, so from 5 states on the registers are capped for
+// one more block per SM where that spills nothing.  Without the cap a graph of 45,000
+// nodes of 8 states (352 tiles, 2 blocks per SM) fell back to a launch per
+// iteration, whose CUDA graph its first solve captures: new graph and five
+// iterations 553 -> 690 us.
+template <int MS, bool UNI> constexpr int fused_min_blocks() {
+    if (MS <= 4) return flood_min_blocks<MS, flood_unroll<MS>()>();
+    if (!UNI) return MS == 5 ? 5 : 4;
+    return MS <= 6 ? 4 : (MS <= 8 ? 3 : 2);
+}
+
 struct FloodArgs {
     uint32_t V;          // tiles cover nodes [v_base, V)
     uint32_t v_base;     // first node of tile 0 (a node range of a sharded run; else 0)
@@ -898,7 +910,7 @@ __device__ __forceinline__ void publish_ctl(LoopyCtl *ctl, const LoopyCtl &sc) {
 // Every iteration of a run with the f64 delta in one cooperative launch, the
 // tile's data read from memory as k_flood reads it: see loop_plan for where it
 // is taken instead of k_flood_loop and of a launch per iteration.
-template <int MS, bool UNI, int FU, int MB = flood_min_blocks<MS, FU>()>
+template <int MS, bool UNI, int FU, int MB = fused_min_blocks<MS, UNI>()>
 __global__ void __launch_bounds__(flood_nt<MS>(), MB) k_flood_fused(const FloodArgs a, uint32_t *bar) {
     constexpr int NT = flood_nt<MS>();
     constexpr uint32_t EMAX = flood_smem_floats<MS>() / MS;
