@@ -255,10 +255,10 @@ __device__ __forceinline__ void divide_by_sum(float *m, float sum, int n) {
     }
 }
 
-// a message's quotients
-template <int MS, bool UNI>
+// a message's quotients; F32: by the fp32 divide
+template <int MS, bool UNI, bool F32 = MS <= 2>
 __device__ __forceinline__ void divide_message(float *m, float sum, int n) {
-    if constexpr (MS <= 2) {
+    if constexpr (F32) {
         if (sum <= 0.0f) sum = 1.0f;
 #pragma unroll
         for (int i = 0; i < MS; ++i) m[i] = (UNI || i < n) ? __fdiv_rn(m[i], sum) : 0.0f;
@@ -311,7 +311,7 @@ __device__ __forceinline__ void send_msg_rows(const float *J, const float *buf, 
     divide_message<MS, UNI>(m, sum, x);
 }
 
-template <int MS, bool UNI>
+template <int MS, bool UNI, bool F32 = MS <= 2>
 __device__ __forceinline__ void send_msg(const float *__restrict__ J, const float *buf, int x, int y,
                                          float *m) {
     float sum = 0.0f;
@@ -344,7 +344,7 @@ __device__ __forceinline__ void send_msg(const float *__restrict__ J, const floa
             m[i] = partial;
         }
     }
-    divide_message<MS, UNI>(m, sum, x);
+    divide_message<MS, UNI, F32>(m, sum, x);
 }
 
 // the same send step on a dense x-by-y table (row stride y; for uniform

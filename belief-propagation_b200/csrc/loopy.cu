@@ -55,6 +55,17 @@ template <int MS, int FU> constexpr int flood_min_blocks() { return MS <= 2 ? (F
 // the serial-delta form carries the serial sum's code: a cap would spill
 template <int MS, int FU> constexpr int flood_min_blocks_serial() { return MS <= 2 ? flood_min_blocks<MS, FU>() : 1; }
 
+// Whether a tile's messages are divided in fp32 (divide_message).  Mixed graphs of
+// up to 7, 9 and 10 states: the f64 quotients, all MS of them whatever the
+// message's own count, take 109, 194, 207 us an iteration of 250,000 nodes and
+// 750,000 edges (half of the nodes of 2 states, 24 iterations), fp32 divides,
+// which a message's count cuts short, 89, 141, 146; with beliefs that head
+// through the subnormals (divide_by_sum) 94, 156, 163.  Up to 3, 4, 5, 6 and 8
+// states f64 is level or faster.
+template <int MS, bool UNI> constexpr bool tile_divides_f32() {
+    return MS <= 2 || (!UNI && (MS == 7 || MS >= 9));
+}
+
 // the one-launch form of the same tiles (k_flood_fused): a graph takes it while
 // all its tiles are resident, so from 5 states on the registers are capped for
 // one more block per SM where that spills nothing.  Without the cap a graph of 45,000
@@ -637,7 +648,7 @@ __device__ __forceinline__ void flood_tile(const FloodArgs &a, uint32_t tile, bo
                     send_msg_regs<MS, UNI>(jt, q, x, y, m);
                 } else {
                     if (want) ldv<MS, kStream>(m_old + (size_t)p * MS, o);
-                    send_msg<MS, UNI>(a.joint + (size_t)p * (MS * MS), q, x, y, m);
+                    send_msg<MS, UNI, tile_divides_f32<MS, UNI>()>(a.joint + (size_t)p * (MS * MS), q, x, y, m);
                 }
                 if (want) {
                     float ad[MS];
@@ -692,7 +703,7 @@ __device__ __forceinline__ void flood_tile(const FloodArgs &a, uint32_t tile, bo
                 if (p >= c1) break;
                 float m[MS];
                 if constexpr (FU > 1) send_msg_regs<MS, UNI>(jt[u], q[u], x[u], y[u], m);
-                else send_msg<MS, UNI>(a.joint + (size_t)p * (MS * MS), q[u], x[u], y[u], m);
+                else send_msg<MS, UNI, tile_divides_f32<MS, UNI>()>(a.joint + (size_t)p * (MS * MS), q[u], x[u], y[u], m);
                 if (want) {
                     float ad[MS];
 #pragma unroll
