@@ -41,6 +41,13 @@ def test_serial_launches_take_their_own_residency():
     assert re.search(r"resident_blocks_mb<MS, UNI, FU, flood_min_blocks_serial<MS, FU>\(\), true>", serial)
 
 
+def test_network_blocks_of_ten_states_divide_in_fp32():
+    """The f64 quotients cost a twentieth of a batch's time there."""
+    code = _code("batch.cu")
+    assert "S == 10" in _body(code, r"constexpr bool block_divides_f32\(")
+    assert code.count("send_msg<S, true, block_divides_f32<S>()>(") == 2
+
+
 def test_two_table_adjoint_multiplies_in_fp32():
     """Its scatter form multiplies fp32 operands; split into two TF32 parts
     without their low product they carry up to seven times the error."""
