@@ -29,8 +29,11 @@
 // 50,001 nodes x 3 states.  The orbit is now followed only until its period
 // is known (Brent's method), and the rest taken modulo the period.
 // 50,001 nodes, 200,003 edges, 3 states, serial delta, 50 iterations:
-// 105.4 -> 3.8 ms per solve (0.9 ms of it the iterations; the rest forms the
-// serial sum in the 38 checks that need it, serial_grid.cuh); f64 delta 0.75 ms.
+// 105.4 -> 3.6 ms per solve (the rest of it forms the serial sum in the 38 checks
+// that need it, serial_grid.cuh); f64 delta 0.75 ms.  Mixed state counts: the
+// map changes with every run of equal counts, and in no order there are about
+// as many runs as nodes, each applied by that one thread: 3000 nodes of 2 and 8
+// states 337 us an iteration (540 before), of 8 alone 11.5.
 #pragma once
 
 struct EdgeArgs {

@@ -29,8 +29,9 @@
 // summed in k_flood's order, so results and the f64 delta equal the
 // one-launch-per-iteration loop's bit for bit.
 //
-// What bounds it: the instruction stream of the few warps of a tile -- 1,400
-// instructions an iteration at 8 to 10 cycles each -- more than the memory:
+// What bounds it: the instruction stream of the few warps of a tile more than the
+// memory, and with the serial delta its spills (20-110 bytes in the wide form of
+// 1-4 states at 128 registers, 330-690 in the narrow one):
 // 10,000 nodes, 40,000 edges, 2 states take 6.0 us an iteration with the f64
 // delta (8.2 before) and 7.5 with the serial one (11.7), 61 nodes of 2-4
 // states (one tile) 2.3 and 3.3 (5.7 and 6.8).
