@@ -41,6 +41,14 @@ def test_serial_launches_take_their_own_residency():
     assert re.search(r"resident_blocks_mb<MS, UNI, FU, flood_min_blocks_serial<MS, FU>\(\), true>", serial)
 
 
+def test_split_passes_of_small_graphs_do_not_overlap():
+    """Two kernels of less than a wave each then wait for each other's blocks: a
+    quarter of an iteration of 50,000 nodes."""
+    body = _body(_code("loopy.cu"), r"static int split_run_nv\(")
+    assert re.search(r"overlap = grid_for\(g->V, kNodeThreads\) >= 4u \* gb", body)
+    assert len(re.findall(r"Threads, overlap, g->stream", body)) == 2
+
+
 def test_network_blocks_of_ten_states_divide_in_fp32():
     """The f64 quotients cost a twentieth of a batch's time there."""
     code = _code("batch.cu")
