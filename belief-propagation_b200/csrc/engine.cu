@@ -219,8 +219,8 @@ __global__ void k_gather_joint(const float *__restrict__ jin, uint32_t rs, uint6
 // the same from dense 16-byte aligned tables (row stride MS, edge stride MS^2)
 // of an even state count: a thread per float4 (MS = 2: a table), so a table
 // is whole 16-byte loads and stores instead of a thread, two index loads and a
-// division per float.  400,000 tables of 8 x 8 with 2-8 states (a new tree of
-// 200,000 nodes): 137 -> 38 us; 4M tables of 2 x 2: 81 -> 49 us (ncu).
+// division per float.  The stage of a graph's build, 180,000 tables of 8 x 8: 57 ->
+// 28 us.
 template <int MS>
 __global__ void k_gather_joint_dense(const float4 *__restrict__ jin, const uint32_t *__restrict__ pos_edge,
                                      const uint8_t *__restrict__ pos_dims, uint32_t E,
