@@ -1358,6 +1358,12 @@ static int u_launch(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaS
 // the larger launch.
 constexpr uint32_t kUSmallNodes = 150000;
 static unsigned u_threads(uint32_t V) { return V < kUSmallNodes ? 128u : (unsigned)kUThreads; }
+// the forward without stored messages keeps the larger block from 5 states on (two
+// tables, T = 10: 256 x 256 grid of 5 states 122 us, 132 with 128 threads; of 3
+// states 96 and 94)
+template <int S> static unsigned u_fwd_threads(uint32_t V, bool stored) {
+    return stored || S <= 4 ? u_threads(V) : (unsigned)kUThreads;
+}
 static unsigned pull_nodes(uint32_t V) { return V < kUSmallNodes ? 1u : 2u; }
 
 // in-edges per batch of the adjoint kernel (BP_UBWD_BATCH=2|4, 1-4 states)
@@ -1373,7 +1379,7 @@ template <int S>
 static int u_forward(bp_unrolled *u) {
     const UGraph g{u->V, u->K, u->in_ptr, u->in_src, u->out_ptr, u->pos_out, u->pos_tab, u->tables};
     const size_t VS = (size_t)u->V * S;
-    const unsigned ut = u_threads(u->V), gv = grid_for(u->V, ut);
+    const unsigned ut = u_fwd_threads<S>(u->V, u->ms.n != 0), gv = grid_for(u->V, ut);
     cudaStream_t st = u->stream;
     int rc, mc = 0;   // mc: the message buffer read next
     if (u->ms.n) {

@@ -49,6 +49,13 @@ def test_split_passes_of_small_graphs_do_not_overlap():
     assert len(re.findall(r"Threads, overlap, g->stream", body)) == 2
 
 
+def test_forward_without_stored_messages_keeps_large_blocks():
+    """From 5 states on 128 threads cost it a twelfth of its time."""
+    code = _code("unrolled.cu")
+    assert re.search(r"stored \|\| S <= 4 \? u_threads\(V\) : \(unsigned\)kUThreads", code)
+    assert "u_fwd_threads<S>(u->V, u->ms.n != 0)" in _body(code, r"static int u_forward\(")
+
+
 def test_network_blocks_of_ten_states_divide_in_fp32():
     """The f64 quotients cost a twentieth of a batch's time there."""
     code = _code("batch.cu")
